@@ -14,6 +14,7 @@
 #include <cstring>
 #include <mutex>
 #include <string>
+#include <type_traits>
 #include <vector>
 
 #include "fcw_b200.h"
@@ -122,6 +123,7 @@ struct Workspace {
     double* out = nullptr;
     int32_t out_stride = 0;
     double* U = nullptr;        // forward update rows, (sum nr) x K doubles (reused as floats)
+    double* W = nullptr;        // assembled right-hand sides of the wide fronts (reused as floats)
     double* partials = nullptr; // per (vertex tile, source) health/MSD partial sums
     double* csum = nullptr;     // per (vertex tile, source) component sums, then the levels (several components)
     int32_t* near_list = nullptr;
@@ -129,8 +131,8 @@ struct Workspace {
     cudaStream_t stream = nullptr;  // this workspace's stream in the pipelined device path
     cudaEvent_t done = nullptr;
     std::vector<std::pair<int, cudaEvent_t>> marks;  // stage timeline on this workspace
-    double* part = nullptr;     // backward split-K partial sums
-    int* counters = nullptr;    // split-K arrival tickets, zero at rest
+    double* part = nullptr;     // tensor-core sweeps: backward split-K partial sums
+    int* counters = nullptr;    // and arrival tickets, zero at rest
     fcw::BlockDesc* desc = nullptr;     // the current block's inputs (device)
     // the block's launch chain captured as CUDA graphs, one per set of arguments (a few)
     struct Graph {
@@ -192,18 +194,25 @@ struct fcw_engine {
     int64_t bytes = 0;
     fcw::DevPlan plan;
     std::vector<int32_t> level_tiles;
-    // solve schedule: per level, task ranges of the forward / backward task lists
-    std::vector<int32_t> fwd_ptr, bwd_ptr;
-    std::vector<int32_t> level_rows;  // backward tile rows per level: 32 if all its supernodes are <= 32 wide
-    std::vector<uint8_t> level_gathers;  // some supernode of the level has children
-    int2 *fwd_tasks = nullptr, *bwd_tasks = nullptr;
+    // the sweeps' fronts and task lists (fronts.h) and their panels: forward and backward, of the
+    // heat, Poisson and (FP32) grounded Poisson factors
+    fcw::Fronts fr;
+    fcw::FrontPlan frp;
+    std::vector<int32_t> bwd_depth;  // per level: the most front rows a backward task multiplies
+    fcw::SweepTask *fwd_tasks = nullptr, *bwd_tasks = nullptr;
+    fcw::GatherRec* rec_d = nullptr;
+    int32_t *rec_child_d = nullptr, *more_d = nullptr, *front_rows_d = nullptr, *asm_rows_d = nullptr;
+    double *pan_hf = nullptr, *pan_hb = nullptr, *pan_pf = nullptr, *pan_pb = nullptr;
+    float *pan_gf = nullptr, *pan_gb = nullptr;
+    // tensor-core sweeps: per level of supernodes, task ranges of the backward task list
+    std::vector<int32_t> tc_bwd_ptr;
+    int2* tc_bwd_tasks = nullptr;
     int64_t* uoff_d = nullptr;
     int64_t* poff_d = nullptr;
     int32_t* nsplit_d = nullptr;
     int32_t *gm_ptr_d = nullptr, *gm_src_d = nullptr, *gm_child_d = nullptr;
     int64_t n_urows = 0, n_parts = 0;
     double *val_h = nullptr, *inv_h = nullptr, *val_p = nullptr, *inv_p = nullptr;
-    float *val_g = nullptr, *inv_g = nullptr;
     fcw::CsrOperator lg;  // the grounded Poisson operator in FP64, elimination order (refinement residuals)
     // tensor-core FP32 sweeps: core arrays of the grounded factor and the forward task list
     float *core_hi = nullptr, *core_lo = nullptr, *coreT_hi = nullptr, *coreT_lo = nullptr;
@@ -471,6 +480,7 @@ int build_engine(fcw_engine* e, const double* V, int64_t nv, const int32_t* F, i
     FCW_CUDA(cudaSetDevice(e->device));
     FCW_CUDA(cudaDeviceGetAttribute(&e->num_sms, cudaDevAttrMultiProcessorCount, e->device));
     FCW_CUDA(fcw::configure_kernels());
+    FCW_CUDA(fcw::configure_front_kernels());
     FCW_CUDA(fcw::configure_solve_kernels());
     FCW_CUDA(fcw::configure_tc_kernels());
     FCW_CUDA(cudaStreamCreateWithFlags(&e->stream, cudaStreamNonBlocking));
@@ -524,8 +534,54 @@ int build_engine(fcw_engine* e, const double* V, int64_t nv, const int32_t* F, i
         e->level_tiles[l] = (int32_t)std::min<int64_t>(mx, 512);
     }
 
-    // solve schedule (see solve.cu): forward row-chunk tasks, backward split-K tasks,
-    // update-row offsets and the per-front-row gather lists of children's update rows
+    // the batched sweeps' fronts and tasks
+    if (fcw::build_fronts(S, e->fr, err)) return fail(FCW_E_INVALID, err);
+    {
+        fcw::Fronts& f = e->fr;
+        fcw::FrontPlan& q = e->frp;
+        std::vector<int64_t> ptr((size_t)f.nf + 1, 0);
+        std::vector<int32_t> sn_front((size_t)S.nsuper), merged;
+        for (int32_t t = 0; t < f.nf; ++t) {
+            const int32_t ns = f.c0[t + 1] - f.c0[t];
+            ptr[t + 1] = ptr[t] + (int64_t)f.m[t] * ns;
+            for (int32_t k = f.sn0[t]; k < f.sn0[t + 1]; ++k) sn_front[k] = t;
+            if (f.sn0[t + 1] - f.sn0[t] > 1) {
+                merged.push_back(t);
+                q.max_m = std::max(q.max_m, f.m[t]);
+                q.max_ns = std::max(q.max_ns, ns);
+            }
+            if (f.m[t] > fcw::max_front_rows())
+                return fail(FCW_E_INVALID, "front too large for the sweeps (" + std::to_string(f.m[t]) + " rows)");
+        }
+        e->bwd_depth.assign(f.nlevels, 0);
+        for (int32_t l = 0; l < f.nlevels; ++l)
+            for (int32_t k = f.bwd_ptr[l]; k < f.bwd_ptr[l + 1]; ++k)
+                e->bwd_depth[l] = std::max(e->bwd_depth[l], f.bwd[k].depth);
+        int32_t *c0, *m, *parent, *sn0, *snf, *colf, *pos, *mg;
+        int64_t* pd;
+        FCW_TRY(e->upload(&c0, f.c0));
+        FCW_TRY(e->upload(&m, f.m));
+        FCW_TRY(e->upload(&parent, f.parent));
+        FCW_TRY(e->upload(&sn0, f.sn0));
+        FCW_TRY(e->upload(&snf, sn_front));
+        FCW_TRY(e->upload(&colf, f.col_front));
+        FCW_TRY(e->upload(&pos, f.pos));
+        FCW_TRY(e->upload(&mg, merged));
+        FCW_TRY(e->upload(&pd, ptr));
+        q.nf = f.nf; q.n_merged = (int32_t)merged.size(); q.entries = ptr[f.nf];
+        q.c0 = c0; q.m = m; q.parent = parent; q.sn0 = sn0; q.sn_front = snf; q.col_front = colf; q.pos = pos;
+        q.merged = mg; q.ptr = pd;
+        FCW_TRY(e->upload(&e->fwd_tasks, f.fwd));
+        FCW_TRY(e->upload(&e->bwd_tasks, f.bwd));
+        FCW_TRY(e->upload(&e->rec_d, f.rec));
+        FCW_TRY(e->upload(&e->rec_child_d, f.rec_child));
+        FCW_TRY(e->upload(&e->more_d, f.more));
+        FCW_TRY(e->upload(&e->front_rows_d, f.rows));
+        FCW_TRY(e->upload(&e->asm_rows_d, f.asm_rows));
+    }
+
+    // the supernodes' update rows and the per-front-row gather lists of the single-source and
+    // tensor-core sweeps, and the latter's tasks (see solve_tc.cu)
     {
         const int32_t NS = S.nsuper;
         std::vector<int64_t> uoff(NS + 1, 0), poff(NS, 0);
@@ -539,41 +595,28 @@ int build_engine(fcw_engine* e, const double* V, int64_t nv, const int32_t* F, i
             if (nsplit[s] > 1) parts += nsplit[s];
         }
         e->n_urows = uoff[NS];
-        e->n_parts = parts;
-        std::vector<int2> ft, bt, tft;
-        e->tc_fwd_ptr.assign(S.nlevels + 1, 0);
-        e->fwd_ptr.assign(S.nlevels + 1, 0);
-        e->bwd_ptr.assign(S.nlevels + 1, 0);
-        e->level_rows.assign(S.nlevels, fcw::kMaxWidth);
-        e->level_gathers.assign(S.nlevels, 0);
-        for (int32_t l = 0; l < S.nlevels; ++l) {
-            int32_t widest = 0;
-            for (int32_t q = S.level_ptr[l]; q < S.level_ptr[l + 1]; ++q) {
-                const int32_t s = S.level_nodes[q];
-                widest = std::max(widest, S.sn_c0[s + 1] - S.sn_c0[s]);
-                if (S.child_ptr[s + 1] > S.child_ptr[s]) e->level_gathers[l] = 1;
+        e->n_parts = e->prm.tc_sweeps ? parts : 0;
+        if (e->prm.tc_sweeps) {
+            std::vector<int2> bt, tft;
+            e->tc_fwd_ptr.assign(S.nlevels + 1, 0);
+            e->tc_bwd_ptr.assign(S.nlevels + 1, 0);
+            for (int32_t l = 0; l < S.nlevels; ++l) {
+                // forward: per supernode the inverse block with the first 64 update rows, then
+                // 128-row update chunks
+                for (int32_t q = S.level_ptr[l]; q < S.level_ptr[l + 1]; ++q) {
+                    const int32_t s = S.level_nodes[q];
+                    const int32_t ns = S.sn_c0[s + 1] - S.sn_c0[s], nr = S.sn_m[s] - ns;
+                    const int32_t nchunk = 1 + std::max(0, (nr - 64 + 127) / 128);
+                    for (int32_t c = 0; c < nchunk; ++c) tft.push_back(make_int2(s, c));
+                    for (int32_t c = 0; c < nsplit[s]; ++c) bt.push_back(make_int2(s, c));
+                }
+                e->tc_fwd_ptr[l + 1] = (int32_t)tft.size();
+                e->tc_bwd_ptr[l + 1] = (int32_t)bt.size();
             }
-            // narrow backward tiles on the leaf levels; the forward sweep keeps 64-row
-            // tasks everywhere (32-row tasks would recompute X_s for twice as many chunks)
-            e->level_rows[l] = widest <= 32 ? 32 : fcw::kMaxWidth;
-            for (int32_t q = S.level_ptr[l]; q < S.level_ptr[l + 1]; ++q) {
-                const int32_t s = S.level_nodes[q];
-                const int32_t ns = S.sn_c0[s + 1] - S.sn_c0[s], nr = S.sn_m[s] - ns;
-                const int32_t nch = std::max(1, (nr + fcw::kMaxWidth - 1) / fcw::kMaxWidth);
-                for (int32_t c = 0; c < nch; ++c) ft.push_back(make_int2(s, c));
-                for (int32_t c = 0; c < nsplit[s]; ++c) bt.push_back(make_int2(s, c));
-            }
-            e->fwd_ptr[l + 1] = (int32_t)ft.size();
-            e->bwd_ptr[l + 1] = (int32_t)bt.size();
-            // tensor-core forward: per supernode the inverse block with the first 64 update rows,
-            // then 128-row update chunks
-            for (int32_t q = S.level_ptr[l]; q < S.level_ptr[l + 1]; ++q) {
-                const int32_t s = S.level_nodes[q];
-                const int32_t ns = S.sn_c0[s + 1] - S.sn_c0[s], nr = S.sn_m[s] - ns;
-                const int32_t nchunk = 1 + std::max(0, (nr - 64 + 127) / 128);
-                for (int32_t c = 0; c < nchunk; ++c) tft.push_back(make_int2(s, c));
-            }
-            e->tc_fwd_ptr[l + 1] = (int32_t)tft.size();
+            FCW_TRY(e->upload(&e->tc_fwd_tasks, tft));
+            FCW_TRY(e->upload(&e->tc_bwd_tasks, bt));
+            FCW_TRY(e->upload(&e->poff_d, poff));
+            FCW_TRY(e->upload(&e->nsplit_d, nsplit));
         }
         const int64_t nfront = S.sn_rowptr[NS];
         std::vector<int32_t> gptr(nfront + 1, 0), gsrc(e->n_urows), gchild(e->n_urows);
@@ -597,12 +640,7 @@ int build_engine(fcw_engine* e, const double* V, int64_t nv, const int32_t* F, i
             }
         }
         if (e->n_urows > INT32_MAX || nfront > INT32_MAX) return fail(FCW_E_INVALID, "mesh too large for 32-bit update indices");
-        FCW_TRY(e->upload(&e->fwd_tasks, ft));
-        FCW_TRY(e->upload(&e->bwd_tasks, bt));
-        FCW_TRY(e->upload(&e->tc_fwd_tasks, tft));
         FCW_TRY(e->upload(&e->uoff_d, uoff));
-        FCW_TRY(e->upload(&e->poff_d, poff));
-        FCW_TRY(e->upload(&e->nsplit_d, nsplit));
         FCW_TRY(e->upload(&e->gm_ptr_d, gptr));
         FCW_TRY(e->upload(&e->gm_src_d, gsrc));
         FCW_TRY(e->upload(&e->gm_child_d, gchild));
@@ -724,6 +762,22 @@ int build_engine(fcw_engine* e, const double* V, int64_t nv, const int32_t* F, i
     FCW_TRY(e->dalloc(&e->inv_h, S.n_inv));
     FCW_TRY(e->dalloc(&e->val_p, S.nnz_factor));
     FCW_TRY(e->dalloc(&e->inv_p, S.n_inv));
+    double* front_rows;
+    FCW_TRY(e->dalloc(&front_rows, e->frp.entries));
+    // the sweeps' panels of one factor; a chunk's copy may run up to three depth rows past a panel
+    constexpr int64_t kPanelSlack = 1024;
+    auto pack = [&](const double* val, const double* inv, auto** fwd, auto** bwd, int64_t nfwd, int64_t nbwd) -> int {
+        using T = std::remove_reference_t<decltype(**fwd)>;
+        FCW_TRY(e->dalloc(fwd, (size_t)(nfwd + kPanelSlack)));
+        FCW_TRY(e->dalloc(bwd, (size_t)(nbwd + kPanelSlack)));
+        FCW_CUDA(cudaMemsetAsync(*fwd + nfwd, 0, kPanelSlack * sizeof(T), e->stream));
+        FCW_CUDA(cudaMemsetAsync(*bwd + nbwd, 0, kPanelSlack * sizeof(T), e->stream));
+        fcw::launch_front_rows(e->plan, e->frp, val, inv, front_rows, e->stream);
+        fcw::launch_pack<T>(e->frp, true, e->fwd_tasks, (int32_t)e->fr.fwd.size(), front_rows, *fwd, e->stream);
+        fcw::launch_pack<T>(e->frp, false, e->bwd_tasks, (int32_t)e->fr.bwd.size(), front_rows, *bwd, e->stream);
+        FCW_CUDA(cudaGetLastError());
+        return FCW_OK;
+    };
     auto run_factor = [&](Op op, double* val, double* inv, const char* what) -> int {
         std::vector<double> av = operator_values(e, op);
         FCW_CUDA(cudaMemcpyAsync(aval_d, av.data(), av.size() * sizeof(double), cudaMemcpyHostToDevice, e->stream));
@@ -741,6 +795,8 @@ int build_engine(fcw_engine* e, const double* V, int64_t nv, const int32_t* F, i
     };
     FCW_TRY(run_factor(Op::Heat, e->val_h, e->inv_h, "heat factorisation"));
     FCW_TRY(run_factor(Op::Poisson, e->val_p, e->inv_p, "Poisson factorisation"));
+    FCW_TRY(pack(e->val_h, e->inv_h, &e->pan_hf, &e->pan_hb, e->fr.fwd64, e->fr.bwd64));
+    FCW_TRY(pack(e->val_p, e->inv_p, &e->pan_pf, &e->pan_pb, e->fr.fwd64, e->fr.bwd64));
     if (e->prm.build_mixed && e->prm.refine > 0) {
         // L_g in CSR, elimination order: the entries the FP32 factor came from
         std::vector<int64_t> rp(S.n + 1, 0);
@@ -776,10 +832,7 @@ int build_engine(fcw_engine* e, const double* V, int64_t nv, const int32_t* F, i
         FCW_TRY(e->dalloc(&val_tmp, S.nnz_factor));
         FCW_TRY(e->dalloc(&inv_tmp, S.n_inv));
         FCW_TRY(run_factor(Op::Grounded, val_tmp, inv_tmp, "grounded Poisson factorisation"));
-        FCW_TRY(e->dalloc(&e->val_g, S.nnz_factor));
-        FCW_TRY(e->dalloc(&e->inv_g, S.n_inv));
-        fcw::launch_to_float(S.nnz_factor, val_tmp, e->val_g, e->stream);
-        fcw::launch_to_float(S.n_inv, inv_tmp, e->inv_g, e->stream);
+        FCW_TRY(pack(val_tmp, inv_tmp, &e->pan_gf, &e->pan_gb, e->fr.fwd32, e->fr.bwd32));
         if (e->prm.tc_sweeps) {
             std::vector<int64_t> cptr(S.nsuper + 1, 0);
             for (int32_t s = 0; s < S.nsuper; ++s) {
@@ -801,6 +854,7 @@ int build_engine(fcw_engine* e, const double* V, int64_t nv, const int32_t* F, i
         e->release(inv_tmp);
     }
     FCW_CUDA(cudaStreamSynchronize(e->stream));
+    e->release(front_rows);
     e->release(upd);
     e->release(aval_d);
     e->factor_ms = now_ms() - t0;
@@ -811,7 +865,7 @@ int ensure_one(fcw_engine* e, Workspace& w, int32_t K, int32_t stride) {
     if (w.K >= K && w.out_stride >= stride) return FCW_OK;
     const int32_t Kn = std::max(K, w.K);
     const int32_t sn = std::max(stride, w.out_stride);
-    void* old[] = {w.Bh, w.Bp64, w.Y, w.dT64, w.src, w.reach, w.band, w.longf, w.out, w.U, w.part,
+    void* old[] = {w.Bh, w.Bp64, w.Y, w.dT64, w.src, w.reach, w.band, w.longf, w.out, w.U, w.W, w.part,
                    w.counters, w.partials, w.near_list, w.near_count, w.desc, w.csum};
     for (void* p : old)
         if (p) e->release(p);
@@ -829,7 +883,7 @@ int ensure_one(fcw_engine* e, Workspace& w, int32_t K, int32_t stride) {
     FCW_TRY(e->dalloc(&w.dT64, (size_t)n * Kn));
     w.dT32 = reinterpret_cast<float*>(w.dT64);
     FCW_TRY(e->dalloc(&w.src, (size_t)Kn));
-    FCW_TRY(e->dalloc(&w.reach, (size_t)std::max<int64_t>(e->sym.nsuper, 1) * (Kn / fcw::kReachCols)));
+    FCW_TRY(e->dalloc(&w.reach, (size_t)std::max<int64_t>(e->fr.nf, 1) * (Kn / fcw::kReachCols)));
     FCW_TRY(e->dalloc(&w.band, (size_t)nf * Kn));
     FCW_TRY(e->dalloc(&w.longf, (size_t)nf * Kn));
     FCW_TRY(e->dalloc(&w.out, (size_t)sn * Kn));
@@ -837,11 +891,15 @@ int ensure_one(fcw_engine* e, Workspace& w, int32_t K, int32_t stride) {
     FCW_TRY(e->dalloc(&w.partials, (size_t)ntiles * Kn * 8));
     FCW_TRY(e->dalloc(&w.near_list, (size_t)n * Kn));
     FCW_TRY(e->dalloc(&w.near_count, (size_t)Kn));
-    FCW_TRY(e->dalloc(&w.U, (size_t)std::max<int64_t>(e->n_urows, 1) * Kn));
-    FCW_TRY(e->dalloc(&w.part, (size_t)std::max<int64_t>(e->n_parts, 1) * fcw::kMaxWidth * Kn));
-    const int64_t nctr = (int64_t)std::max<int32_t>(e->sym.nsuper, 1) * (Kn / fcw::kRhsTile);
-    FCW_TRY(e->dalloc(&w.counters, (size_t)nctr));
-    FCW_CUDA(cudaMemset(w.counters, 0, nctr * sizeof(int)));
+    const int64_t urows = e->prm.tc_sweeps ? std::max(e->fr.n_urows, e->n_urows) : e->fr.n_urows;
+    FCW_TRY(e->dalloc(&w.U, (size_t)std::max<int64_t>(urows, 1) * Kn));
+    FCW_TRY(e->dalloc(&w.W, (size_t)std::max<int64_t>(e->fr.n_wrows, 1) * Kn));
+    if (e->prm.tc_sweeps) {
+        FCW_TRY(e->dalloc(&w.part, (size_t)std::max<int64_t>(e->n_parts, 1) * fcw::kMaxWidth * Kn));
+        const int64_t nctr = (int64_t)std::max<int32_t>(e->sym.nsuper, 1) * (Kn / fcw::kRhsTile);
+        FCW_TRY(e->dalloc(&w.counters, (size_t)nctr));
+        FCW_CUDA(cudaMemset(w.counters, 0, nctr * sizeof(int)));
+    }
     FCW_TRY(e->dalloc(&w.desc, 1));
     if (e->ncomp > 1) FCW_TRY(e->dalloc(&w.csum, (size_t)(fcw::component_tiles(n) + 1) * Kn));
     w.K = Kn;
@@ -860,7 +918,7 @@ int ensure_workspace(fcw_engine* e, int32_t K, int32_t stride) {
         e->sync_streams();
         for (size_t j = i; j < e->pool.size(); ++j) {
             Workspace& w = e->pool[j];
-            void* bufs[] = {w.Bh, w.Bp64, w.Y, w.dT64, w.src, w.reach, w.band, w.longf, w.out, w.U, w.part,
+            void* bufs[] = {w.Bh, w.Bp64, w.Y, w.dT64, w.src, w.reach, w.band, w.longf, w.out, w.U, w.W, w.part,
                             w.counters, w.partials, w.near_list, w.near_count, w.desc, w.csum};
             for (void* p : bufs)
                 if (p) e->release(p);
@@ -876,22 +934,70 @@ int ensure_workspace(fcw_engine* e, int32_t K, int32_t stride) {
     return FCW_OK;
 }
 
+// Both sweeps on the front panels: right-hand sides R (or the identity columns and reach flags in
+// `a`), forward result into Y, solution into X (n x K, three different arrays).
 template <typename T>
-fcw::SolveArgs<T> solve_args(fcw_engine* e, const T* val, const T* inv, T* B, int32_t K) {
-    fcw::SolveArgs<T> a;
-    a.p = e->plan;
-    a.val = val;
-    a.inv = inv;
-    a.B = B;
-    a.K = K;
+void sweep(fcw_engine* e, fcw::SweepArgs<T> a, const T* fwd, const T* bwd, const T* R, T* Y, T* X, int32_t K,
+           cudaStream_t st, int stage_fwd, int stage_bwd) {
+    const fcw::Fronts& f = e->fr;
+    a.R = R;
+    a.Y = Y;
+    a.X = X;
     a.U = reinterpret_cast<T*>(e->cw().U);
+    a.W = reinterpret_cast<T*>(e->cw().W);
+    a.K = K;
+    a.rec = reinterpret_cast<const int4*>(e->rec_d);
+    a.rec_child = e->rec_child_d;
+    a.more = e->more_d;
+    a.rows = e->front_rows_d;
+    a.asm_rows = reinterpret_cast<const int4*>(e->asm_rows_d);
+    a.err = e->err_d;
+    mark(e, st, stage_fwd);
+    a.tasks = e->fwd_tasks;
+    a.panel = fwd;
+    for (int32_t l = 0; l < f.nlevels; ++l) {
+        const bool wide = l >= f.first_wide;
+        a.gathers = l > 0;
+        if (wide) fcw::launch_assemble<T>(a, f.asm_ptr[l], f.asm_ptr[l + 1] - f.asm_ptr[l], st);
+        fcw::launch_fwd_level<T>(a, f.fwd_ptr[l], f.fwd_ptr[l + 1] - f.fwd_ptr[l], f.fwd_rows[l], wide, st);
+    }
+    a.delta_src = nullptr;
+    mark(e, st, stage_bwd);
+    a.tasks = e->bwd_tasks;
+    a.panel = bwd;
+    for (int32_t l = f.nlevels - 1; l >= 0; --l)
+        fcw::launch_bwd_level<T>(a, f.bwd_ptr[l], f.bwd_ptr[l + 1] - f.bwd_ptr[l], f.bwd_rows[l], e->bwd_depth[l], st);
+    e->launches += 2 * (int64_t)f.nlevels + (f.nlevels - f.first_wide);
+}
+
+// Heat solve for the K sources in ws.src: u (elimination order, n x K) in ws.Bh.
+void heat_solve(fcw_engine* e, int32_t K, cudaStream_t st) {
+    Workspace& w = e->cw();
+    mark(e, st, FCW_STAGE_HEAT_FWD);
+    fcw::launch_reach(e->frp.col_front, e->frp.parent, e->fr.nf, e->fr.nlevels, w.src, K, w.reach, st);
+    e->launches += 2;
+    fcw::SweepArgs<double> a;
+    a.delta_src = w.src;
+    a.reach = w.reach;
+    a.reach_tiles = K / fcw::kReachCols;
+    sweep<double>(e, a, e->pan_hf, e->pan_hb, nullptr, w.Y, w.Bh, K, st, FCW_STAGE_HEAT_FWD, FCW_STAGE_HEAT_BWD);
+}
+
+// FP32 sweeps on the tensor cores, over the supernodes' levels: R -> Y (in place after the forward).
+int sweep_tc(fcw_engine* e, const float* R, float* Y, int32_t K, cudaStream_t st) {
+    const auto& S = e->sym;
+    fcw::SolveArgs<float> a;
+    a.p = e->plan;
+    a.R = R;
+    a.B = Y;
+    a.K = K;
+    a.U = reinterpret_cast<float*>(e->cw().U);
     a.uoff = e->uoff_d;
     a.gm_ptr = e->gm_ptr_d;
     a.gm_src = e->gm_src_d;
-    a.gm_child = e->gm_child_d;
     a.nsplit = e->nsplit_d;
     a.poff = e->poff_d;
-    a.part = reinterpret_cast<T*>(e->cw().part);
+    a.part = reinterpret_cast<float*>(e->cw().part);
     a.counters = e->cw().counters;
     a.ktiles = e->cw().K / fcw::kRhsTile;
     a.core_hi = e->core_hi;
@@ -900,42 +1006,6 @@ fcw::SolveArgs<T> solve_args(fcw_engine* e, const T* val, const T* inv, T* B, in
     a.coreT_lo = e->coreT_lo;
     a.core_ptr = e->core_ptr_d;
     a.err = e->err_d;
-    return a;
-}
-
-template <typename T>
-void sweep(fcw_engine* e, fcw::SolveArgs<T> a, cudaStream_t st, int stage_fwd, int stage_bwd) {
-    const auto& S = e->sym;
-    mark(e, st, stage_fwd);
-    for (int32_t l = 0; l < S.nlevels; ++l) {
-        a.tasks = e->fwd_tasks;
-        fcw::launch_fwd_level<T>(a, e->fwd_ptr[l], e->fwd_ptr[l + 1] - e->fwd_ptr[l], e->level_gathers[l] != 0, st);
-    }
-    a.delta_src = nullptr;
-    mark(e, st, stage_bwd);
-    for (int32_t l = S.nlevels - 1; l >= 0; --l) {
-        a.tasks = e->bwd_tasks;
-        fcw::launch_bwd_level<T>(a, e->bwd_ptr[l], e->bwd_ptr[l + 1] - e->bwd_ptr[l], e->level_rows[l], st);
-    }
-    e->launches += 2 * (int64_t)S.nlevels;
-}
-
-// Heat solve for the K sources in ws.src: u (elimination order, n x K) in ws.Bh.
-void heat_solve(fcw_engine* e, int32_t K, cudaStream_t st) {
-    Workspace& w = e->cw();
-    mark(e, st, FCW_STAGE_HEAT_FWD);
-    fcw::launch_reach(e->plan, w.src, K, w.reach, st);
-    e->launches += 2;
-    fcw::SolveArgs<double> a = solve_args<double>(e, e->val_h, e->inv_h, w.Bh, K);
-    a.delta_src = w.src;
-    a.reach = w.reach;
-    a.reach_tiles = K / fcw::kReachCols;
-    sweep<double>(e, a, st, FCW_STAGE_HEAT_FWD, FCW_STAGE_HEAT_BWD);
-}
-
-// FP32 sweeps on the tensor cores: the same level schedule, the forward with its own task list.
-int sweep_tc(fcw_engine* e, fcw::SolveArgs<float> a, cudaStream_t st) {
-    const auto& S = e->sym;
     CUtensorMap rmap, bmap;
     if (fcw::make_rows_map(&rmap, a.R, S.n, a.K) || fcw::make_rows_map(&bmap, a.B, S.n, a.K))
         return fail(FCW_E_CUDA, "cuTensorMapEncodeTiled failed for the Poisson right-hand sides");
@@ -944,22 +1014,22 @@ int sweep_tc(fcw_engine* e, fcw::SolveArgs<float> a, cudaStream_t st) {
     for (int32_t l = 0; l < S.nlevels; ++l)
         fcw::launch_fwd_level_tc(a, e->tc_fwd_ptr[l], e->tc_fwd_ptr[l + 1] - e->tc_fwd_ptr[l], rmap, st);
     mark(e, st, FCW_STAGE_POISSON_BWD);
-    a.tasks = e->bwd_tasks;
+    a.tasks = e->tc_bwd_tasks;
     for (int32_t l = S.nlevels - 1; l >= 0; --l)
-        fcw::launch_bwd_level_tc(a, e->bwd_ptr[l], e->bwd_ptr[l + 1] - e->bwd_ptr[l], bmap, st);
+        fcw::launch_bwd_level_tc(a, e->tc_bwd_ptr[l], e->tc_bwd_ptr[l + 1] - e->tc_bwd_ptr[l], bmap, st);
     e->launches += 2 * (int64_t)S.nlevels;
     return FCW_OK;
 }
 
-// Poisson solve: right-hand sides R, solution into Y (both n x K, elimination order).
+// Poisson solve: right-hand sides R, solution into Y (both n x K, elimination order). The forward
+// result goes to the heat solution's buffer, which the divergence has read by now.
 template <typename T>
-int poisson_solve(fcw_engine* e, const T* val, const T* inv, const T* R, T* Y, int32_t K, cudaStream_t st) {
-    fcw::SolveArgs<T> a = solve_args<T>(e, val, inv, Y, K);
-    a.R = R;
+int poisson_solve(fcw_engine* e, const T* fwd, const T* bwd, const T* R, T* Y, int32_t K, cudaStream_t st) {
     if constexpr (sizeof(T) == 4) {
-        if (e->core_hi && K % fcw::kTcCols == 0) return sweep_tc(e, a, st);
+        if (e->core_hi && K % fcw::kTcCols == 0) return sweep_tc(e, R, Y, K, st);
     }
-    sweep<T>(e, a, st, FCW_STAGE_POISSON_FWD, FCW_STAGE_POISSON_BWD);
+    sweep<T>(e, fcw::SweepArgs<T>{}, fwd, bwd, R, reinterpret_cast<T*>(e->cw().Bh), Y, K, st, FCW_STAGE_POISSON_FWD,
+             FCW_STAGE_POISSON_BWD);
     return FCW_OK;
 }
 
@@ -973,14 +1043,14 @@ int distances_block(fcw_engine* e, int32_t K, int precision, cudaStream_t st, co
     if (precision == FCW_PREC_MIXED) {
         float* Y = reinterpret_cast<float*>(w.Y);
         fcw::launch_divergence_mixed(e->fd, w.Bh, w.Bp32, K, e->grounded_d, st);
-        FCW_TRY(poisson_solve<float>(e, e->val_g, e->inv_g, w.Bp32, Y, K, st));
+        FCW_TRY(poisson_solve<float>(e, e->pan_gf, e->pan_gb, w.Bp32, Y, K, st));
         // refinement: residual in FP64 and its FP32 solution, in the shift's output buffer
         // (two n x K float halves of dT64) before the shift writes it
         for (int32_t it = 0; it < e->prm.refine && e->lg.rp; ++it) {
             float* r = w.dT32;
             float* d = w.dT32 + (int64_t)n * K;
             fcw::launch_residual(e->lg, K, w.Bp32, Y, r, st);
-            FCW_TRY(poisson_solve<float>(e, e->val_g, e->inv_g, r, d, K, st));
+            FCW_TRY(poisson_solve<float>(e, e->pan_gf, e->pan_gb, r, d, K, st));
             fcw::launch_add((int64_t)n * K, Y, d, e->num_sms, st);
             e->launches += 2;
         }
@@ -993,7 +1063,7 @@ int distances_block(fcw_engine* e, int32_t K, int precision, cudaStream_t st, co
         else fcw::launch_shift_transpose<float, float>(n, K, Y, w.src, w.dT32, st);
     } else {
         fcw::launch_divergence_fp64(e->fd, w.Bh, w.Bp64, K, st);
-        FCW_TRY(poisson_solve<double>(e, e->val_p, e->inv_p, w.Bp64, w.Y, K, st));
+        FCW_TRY(poisson_solve<double>(e, e->pan_pf, e->pan_pb, w.Bp64, w.Y, K, st));
         mark(e, st, FCW_STAGE_SHIFT);
         if (ma) fcw::launch_shift_stats<double, double>(*ma, K, w.Y, w.dT64, st);
         else fcw::launch_shift_transpose<double, double>(n, K, w.Y, w.src, w.dT64, st);
@@ -1332,7 +1402,7 @@ int fcw_engine_destroy(fcw_engine* e) {
 int fcw_compute_distances(fcw_engine* e, const int32_t* sources, int64_t n, int32_t precision, double* out_host) {
     FCW_TRY(check_engine(e));
     if (n < 0 || (n > 0 && (!sources || !out_host))) return fail(FCW_E_INVALID, "NULL argument");
-    if (precision == FCW_PREC_MIXED && !e->val_g) return fail(FCW_E_INVALID, "engine was built without the mixed form");
+    if (precision == FCW_PREC_MIXED && !e->pan_gf) return fail(FCW_E_INVALID, "engine was built without the mixed form");
     const int32_t Kmax = e->prm.block_k;
     const int64_t nv = e->sym.n;
     std::vector<int32_t> buf;
@@ -1593,7 +1663,7 @@ int fcw_compute_metrics_device(fcw_engine* e, const int32_t* sources_dev, int64_
                                void* stream) {
     FCW_TRY(check_engine(e));
     if (n < 0 || (n > 0 && (!sources_dev || !out_dev))) return fail(FCW_E_INVALID, "NULL argument");
-    if (precision == FCW_PREC_MIXED && !e->val_g) return fail(FCW_E_INVALID, "engine was built without the mixed form");
+    if (precision == FCW_PREC_MIXED && !e->pan_gf) return fail(FCW_E_INVALID, "engine was built without the mixed form");
     if (n == 0) return FCW_OK;
     cudaStream_t user = static_cast<cudaStream_t>(stream);
     const int32_t stride = fcw_metrics_stride(nt, nb);
@@ -1816,7 +1886,7 @@ int fcw_poisson_solve_device(fcw_engine* e, const double* div_dev, const int32_t
                                                    e->err_d);
     FCW_CUDA(cudaMemsetAsync(e->cw().Bp64, 0, (size_t)e->sym.n * K * sizeof(double), st));
     fcw::launch_permute_rows((int32_t)e->sym.n, k, div_dev, k, nullptr, e->cw().Bp64, K, e->iperm_d, st);
-    FCW_TRY(poisson_solve<double>(e, e->val_p, e->inv_p, e->cw().Bp64, e->cw().Y, K, st));
+    FCW_TRY(poisson_solve<double>(e, e->pan_pf, e->pan_pb, e->cw().Bp64, e->cw().Y, K, st));
     fcw::launch_shift_transpose<double, double>((int32_t)e->sym.n, K, e->cw().Y, e->cw().src, e->cw().dT64, st);
     // phi_dev[old][c] = dT[c][iperm[old]]: transpose back through the permute kernel, column by column
     for (int32_t c = 0; c < k; ++c)

@@ -7,6 +7,8 @@
 
 #include <vector>
 
+#include "fronts.h"
+
 namespace fcw {
 
 // Error bits a kernel may raise (OR-ed into a device word read by the host).
@@ -59,28 +61,83 @@ void launch_to_float(int64_t n, const double* src, float* dst, cudaStream_t st);
 // after every level: each panel's L21 becomes Q = L21 L11^{-1} (what the solves read)
 void launch_panel_inverse(const DevPlan& p, double* val, const double* inv, cudaStream_t st);
 
-// ---- multi-RHS supernodal triangular solves (solve.cu) ----
-constexpr int kRhsTile = 64;     // right-hand sides per solve CTA; K is a multiple of this
+// ---- fronts: the solve's panels (fronts.cu; planned in fronts.h) ----
+struct FrontPlan {  // device memory
+    int32_t nf = 0, n_merged = 0, max_m = 0, max_ns = 0;
+    const int32_t* c0 = nullptr;        // nf + 1
+    const int32_t* m = nullptr;
+    const int32_t* parent = nullptr;
+    const int32_t* sn0 = nullptr;       // nf + 1
+    const int32_t* sn_front = nullptr;  // per supernode
+    const int32_t* col_front = nullptr; // per column
+    const int32_t* pos = nullptr;       // aligned with the supernodes' rows: the row in its front
+    const int64_t* ptr = nullptr;       // offset of the front's m x ns rows in the FP64 work array
+    const int32_t* merged = nullptr;    // fronts of several supernodes
+    int64_t entries = 0;                // of the work array
+};
+cudaError_t configure_front_kernels();
+// rows = every front's [inv(L_ss); Q_s], m x ns row-major, from one factor's blocks
+void launch_front_rows(const DevPlan& p, const FrontPlan& f, const double* val, const double* inv, double* rows,
+                       cudaStream_t st);
+template <typename T>
+void launch_pack(const FrontPlan& f, bool fwd, const SweepTask* tasks, int32_t ntasks, const double* rows, T* out,
+                 cudaStream_t st);
+
+// ---- multi-RHS triangular solves over fronts (solve.cu) ----
+constexpr int kRhsTile = 64;     // K is a multiple of this
 constexpr int kReachCols = 64;   // columns per tile of the heat solve's reach flags (its FP64 tile width)
+
+template <typename T>
+struct SweepArgs {
+    const SweepTask* tasks = nullptr;
+    const T* panel = nullptr;        // the sweep's task panels
+    const T* R = nullptr;            // forward: n x K right-hand sides (unused with delta_src)
+    T* Y = nullptr;                  // n x K: forward result
+    T* X = nullptr;                  // n x K: solution (not Y)
+    T* U = nullptr;                  // update rows
+    T* W = nullptr;                  // the wide levels' assembled right-hand sides
+    int32_t K = 0;
+    const int4* rec = nullptr;       // GatherRec per front row
+    const int32_t* rec_child = nullptr;
+    const int32_t* more = nullptr;
+    const int32_t* rows = nullptr;   // elimination row of each front row
+    const int4* asm_rows = nullptr;
+    int32_t gathers = 0;             // forward: some front of the level has children
+    const int32_t* delta_src = nullptr;  // forward: identity columns for these sources (elimination order)
+    const uint8_t* reach = nullptr;      // heat solve: reach[f * reach_tiles + t], front f on the path to the root
+                                         // of some source of column tile t (kReachCols columns)
+    int32_t reach_tiles = 0;
+    int* err = nullptr;              // error bits (bounded waits that expired)
+};
+
+cudaError_t configure_solve_kernels();
+int32_t max_front_rows();  // the backward sweep holds a front's row list in shared memory
+// One level of the forward sweep: tasks [t0, t0 + ntasks) of `rows` rows; wide: the level's
+// right-hand sides have been assembled (launch_assemble, rows [r0, r0 + nrows) of asm_rows).
+template <typename T>
+void launch_fwd_level(const SweepArgs<T>& a, int32_t t0, int32_t ntasks, int32_t rows, bool wide, cudaStream_t st);
+template <typename T>
+void launch_assemble(const SweepArgs<T>& a, int32_t r0, int32_t nrows, cudaStream_t st);
+// One level of the backward sweep; max_depth: the most front rows a task multiplies.
+template <typename T>
+void launch_bwd_level(const SweepArgs<T>& a, int32_t t0, int32_t ntasks, int32_t rows, int32_t max_depth,
+                      cudaStream_t st);
+void launch_reach(const int32_t* col_front, const int32_t* parent, int32_t nfronts, int32_t nlevels,
+                  const int32_t* src, int32_t K, uint8_t* reach, cudaStream_t st);
+
+// ---- FP32 sweeps on the tensor cores, over supernodes (solve_tc.cu, fcw_params.tc_sweeps) ----
 constexpr int kSplitRows = 128;  // structure rows per backward split-K task
 
 template <typename T>
 struct SolveArgs {
     DevPlan p;
-    const T* val = nullptr;          // panels: below the diagonal block, Q = L21 L11^{-1}
-    const T* inv = nullptr;          // inverse diagonal blocks
-    const T* R = nullptr;            // n x K right-hand sides (read only; unused with delta_src)
+    const T* R = nullptr;            // n x K right-hand sides (read only)
     T* B = nullptr;                  // n x K forward result, then solution (elimination order)
     int32_t K = 0;
     T* U = nullptr;                  // forward update rows, (sum nr) x K
     const int64_t* uoff = nullptr;   // first update row of each supernode
     const int32_t* gm_ptr = nullptr; // per front row (sn_rowptr-based index): update rows that land on it
     const int32_t* gm_src = nullptr;
-    const int32_t* gm_child = nullptr;
-    const int32_t* delta_src = nullptr;  // forward: identity columns for these sources (elimination order)
-    const uint8_t* reach = nullptr;      // heat solve: reach[s * reach_tiles + t], supernode s on the path to the
-                                         // root of some source of column tile t (kReachCols columns)
-    int32_t reach_tiles = 0;
     const int2* tasks = nullptr;         // (supernode, row chunk | split)
     const int32_t* nsplit = nullptr;     // backward splits per supernode
     const int64_t* poff = nullptr;       // partial-sum slot of the first split (units of 64 x K)
@@ -88,9 +145,8 @@ struct SolveArgs {
     int* counters = nullptr;             // per (supernode, column tile) arrival tickets, zero at rest
     int32_t ktiles = 0;                  // column tiles the counters were sized for
     int32_t stage = 0;                   // forward: children's update rows staged per chunk (set by the launcher)
-    // FP32 tensor-core sweeps: per supernode the stacked [inv(L_ss); Q_s] split into TF32 hi and
-    // lo terms, in core-matrix order (tc.cuh), ns8 = round_up(ns, 8) columns and ns8 +
-    // round_up(nr, 32) rows (padding zero)
+    // per supernode the stacked [inv(L_ss); Q_s] split into TF32 hi and lo terms, in core-matrix
+    // order (tc.cuh), ns8 = round_up(ns, 8) columns and ns8 + round_up(nr, 32) rows (padding zero)
     const float* core_hi = nullptr;
     const float* core_lo = nullptr;
     const float* coreT_hi = nullptr;     // the transposes (backward products), 32-row chunks
@@ -99,22 +155,10 @@ struct SolveArgs {
     int* err = nullptr;                  // error bits (bounded waits that expired)
 };
 
-cudaError_t configure_solve_kernels();
-// Forward sweep of one level (tasks [t0, t0+ntasks) of the level's list);
-// gathers: some supernode of the level has children (leaf levels have none and
-// launch without a staging buffer, so more CTAs share an SM).
-template <typename T>
-void launch_fwd_level(const SolveArgs<T>& a, int32_t t0, int32_t ntasks, bool gathers, cudaStream_t st);
-// Backward sweep of one level; tile_rows is 32 when every supernode of the
-// level is at most 32 wide, else 64.
-template <typename T>
-void launch_bwd_level(const SolveArgs<T>& a, int32_t t0, int32_t ntasks, int32_t tile_rows, cudaStream_t st);
-void launch_reach(const DevPlan& p, const int32_t* src, int32_t K, uint8_t* reach, cudaStream_t st);
-
 // FP32 sweeps on the tensor cores (tcgen05.mma kind::tf32, each operand split into two TF32
 // terms, three products accumulated in tensor memory); K a multiple of 64, 64 columns per CTA.
 // Forward tasks are (supernode, c): c = 0 forms X_s = inv(L_ss) W and update rows [0, 64),
-// c >= 1 update rows [64 + 128 (c - 1), 64 + 128 c). Backward tasks are those of launch_bwd_level. rows_map is a tiled tensor
+// c >= 1 update rows [64 + 128 (c - 1), 64 + 128 c). Backward tasks are (supernode, split). rows_map is a tiled tensor
 // map of the sweep's own-row input (forward: R, backward: B) made by make_rows_map.
 constexpr int kTcCols = 64;
 void launch_fwd_level_tc(const SolveArgs<float>& a, int32_t t0, int32_t ntasks, const CUtensorMap& rows_map,

@@ -1,620 +1,548 @@
-// Multi-right-hand-side supernodal triangular solves, one etree level per launch.
+// Multi-right-hand-side triangular solves over fronts, one tree level per launch.
 //
-// Right-hand sides R and results B are n x K row-major (a vertex row holds K
-// contiguous right-hand sides). The forward sweep reads R and writes the
-// forward result into B; the backward sweep turns B into the solution in
-// place. R is never written, because several CTAs of one supernode (its row
-// chunks) each rebuild that supernode's right-hand side.
+// Right-hand sides and results are n x K row-major (a vertex row holds K contiguous right-hand
+// sides). A CTA owns one task of one front and one column tile of the right-hand sides (64 columns
+// in FP64, 128 in FP32: a tile row is 512 bytes either way), so all row traffic is contiguous
+// 512-byte segments.
 //
-// A CTA owns one task of one supernode and one column tile of the right-hand
-// sides (64 columns in FP64, 128 in FP32: a tile row is 512 bytes either way).
-// Every row of a tile is a contiguous 512-byte segment of an n x K array, so
-// all row traffic (right-hand sides, children's update rows, the ancestors'
-// solution rows, results) moves as 16-byte cp.async copies or vector stores,
-// and a CTA issues all the copies of a stage before it waits for any of them.
+// With A_s = [inv(L_ss); Q_s], Q_s = L_rs inv(L_ss) (fronts.cu):
 //
-// Dense products run on shared-memory tiles. FP64 uses the FP64 tensor path
-// (mma.sync m8n8k4: one instruction per 256 multiply-adds; each of the 8 warps
-// owns 8 columns and walks the 8-row tiles the supernode needs). FP32 uses
-// register tiles on the FMA pipes (a thread owns 4 rows x KT/16 columns in
-// 16-byte column groups).
-//
-// The panels below the diagonal blocks hold Q_s = L_rs inv(L_ss) (formed once
-// after the factorisation), so nothing waits for X_s:
-//
-// Forward (leaves -> root), multifrontal: supernode s forms
+// Forward (leaves -> root), multifrontal: front s forms
 //   W   = b_s - the children's update rows that land on s's columns
-//   X_s = inv(L_ss) W                                   (written to B)
+//   X_s = inv(L_ss) W                                   (written to Y)
 //   U_s = Q_s W + the children's update rows that land on s's structure
-// and leaves U_s (nr x K) for its parent. Children's rows are listed per front
-// row in ascending child order and added in that order, so results are
-// deterministic. A supernode with a long structure is split into 64-row tasks;
-// each forms W and its own rows of U_s, and the first also X_s.
+// and leaves U_s for its parent. A task is up to 128 stacked rows of A_s. On the levels whose fronts
+// are at most 64 columns wide each task gathers W itself, into shared memory; a leaf's A_s has 88
+// rows on average, so one task mostly does the whole front. The wider fronts near the root have many
+// tasks, so there W is assembled once (k_assemble) and the products read it in 32-row chunks.
+// Children's rows are added in ascending child order, so results are deterministic.
 //
-// Backward (root -> leaves): X_s = inv(L_ss)^T y_s - Q_s^T X_r, where X_r are
-// the structure rows (ancestors, final; gathered two chunks in flight). Long
-// structures are split over several CTAs (split-K); each writes a partial sum
-// of Q_s^T X_r, and the CTA that arrives last (atomic ticket, no waiting) adds
-// the partials in split order and finishes the supernode.
+// Backward (root -> leaves): X_s = A_s^T [y_s; -X_r], X_r the structure rows (ancestors, final). A
+// task is up to 64 of the front's columns over all rows below them, gathered in 32-row chunks, three
+// chunks in flight. The solution goes to an array of its own, so tasks of one front need no order.
 //
-// Heat right-hand sides are columns of the identity: the forward sweep builds
-// them from the source list, and only supernodes on a source's path to the
-// root (`reach`, per supernode and 64-column tile) are solved; the others' forward results
-// are zero.
+// Each task's part of A_s is stored as it is used: k-major (for each depth row, the task's rows or
+// columns side by side), one bulk copy (cp.async.bulk) per 32-row chunk, requested before anything
+// else. FP64 products run on the FP64 tensor path (mma.sync m8n8k4; tcgen05 has no FP64 kind), FP32
+// products on packed FMAs (fma.rn.f32x2: two columns per instruction, which leaves issue slots for
+// the shared-memory reads). A warp owns 16 rows, so a task computes its rows rounded up to 16, and
+// the triangles of inv(L_ss) are cut at 16.
+//
+// Launches overlap: a level's CTAs read their task, request their panels and load their gather lists
+// while the previous level finishes (programmatic dependent launch), then wait for it.
+//
+// Heat right-hand sides are columns of the identity: the forward sweep builds them from the source
+// list, and only fronts on a source's path to the root (`reach`, per front and 64-column tile) are
+// solved; the others' forward results are zero and are not read.
+#include <algorithm>
 #include <type_traits>
 
 #include "kernels.cuh"
-#include "sweep_rows.cuh"
+#include "tc.cuh"
 
 namespace fcw {
 
 namespace {
 
-constexpr int PT = kMaxWidth;   // rows of a backward partial-sum slot (= widest supernode)
-constexpr int RC = 32;          // structure rows per backward chunk
-// Tiles are TR = 64 rows (any supernode); the backward sweep also has TR = 32
-// for the levels whose supernodes are all at most 32 wide (the leaves), where
-// smaller tiles and accumulators let three CTAs share an SM.
+constexpr int NT = 256;  // threads per CTA
+constexpr int DC = 32;   // depth rows per chunk
+constexpr int kNarrowCols = 64;  // columns of a front whose right-hand side one task gathers
 
-// Column tile of each precision when K allows it (512-byte rows).
+template <typename T>
+constexpr int vec() { return 16 / (int)sizeof(T); }  // elements per 16-byte vector
 template <typename T>
 constexpr int wide_tile() { return sizeof(T) == 4 ? 128 : 64; }
-// Most children's update rows a forward CTA stages per gather chunk. The
-// launcher picks the count per level (SolveArgs::stage): none on levels without
-// children, else what keeps two CTAs on an SM (three for FP32 with KT = 64).
-template <typename T, int TR>
-constexpr int stage_rows() { return sizeof(T) == 4 ? 112 : 80; }
+// Right-hand-side rows in shared memory. FP64 tensor fragments read 4 depths x 8 columns: a row
+// stride of 8 banks more than a multiple of 32 keeps them apart (as the panels' row stride does).
 template <typename T, int KT>
-constexpr int stage_used() { return sizeof(T) == 8 ? 80 : (KT == 128 ? 88 : 96); }
-// FP32 forward CTAs hold the inverse and the chunk's Q rows in two tiles (both
-// products start as soon as W is formed); FP64 tiles are twice the size, so
-// there the Q rows replace the inverse after X_s.
+constexpr int ld_rhs() { return sizeof(T) == 8 ? KT + 4 : KT; }
+template <typename T, int M>
+constexpr int panel_stage() { return DC * (sizeof(T) == 8 ? M + 4 : M); }  // elements of a chunk's panel rows
 template <typename T>
-constexpr bool separate_q() { return sizeof(T) == 4; }
+__device__ __forceinline__ int panel_stride(int h) { return (h + 7) / 8 * 8 + (sizeof(T) == 8 ? 4 : 0); }
 
-// Shared-tile leading dimensions, chosen so that the product's operand reads
-// are free of bank conflicts: FP64 tensor fragments read 8 rows x 4 depths
-// (row stride TR + 4 doubles = 8 banks apart), FP32 register tiles read rows ty and
-// ty+1 of a row-major A (odd stride) or adjacent columns of a transposed one.
-template <typename T, int TR>
-constexpr int ld_fwd_a() { return sizeof(T) == 8 ? TR + 4 : TR + 1; }  // forward inverse / panel, row-major
-template <typename T, int TR>
-constexpr int ld_bwd_a() { return sizeof(T) == 8 ? TR + 4 : TR; }      // backward panel / inverse, transposed
-template <typename T, int KT>
-constexpr int ld_rows() { return sizeof(T) == 8 ? KT + 4 : KT; }    // right-hand-side rows (W, X, C, gathers)
-template <typename T>
-constexpr int depth_pad() { return sizeof(T) == 8 ? 4 : 1; }        // product depth granularity
+__device__ __forceinline__ void allow_dependents() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+__device__ __forceinline__ void wait_predecessor() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void copy16_async(void* smem, const void* gmem) {
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(tc::smem_u32(smem)), "l"(gmem) : "memory");
+}
+__device__ __forceinline__ void copy_async_commit() { asm volatile("cp.async.commit_group;\n" ::: "memory"); }
+template <int N>
+__device__ __forceinline__ void copy_async_wait() { asm volatile("cp.async.wait_group %0;\n" ::"n"(N) : "memory"); }
 
+// A panel copy that does not land in time raises KERR_TIMEOUT; the second bounded wait lets a late
+// copy finish before the CTA goes on.
+__device__ __forceinline__ void wait_panel(uint64_t* bar, uint32_t parity, int* err) {
+    if (!tc::mbar_wait(bar, parity)) {
+        atomicOr(err, KERR_TIMEOUT);
+        tc::mbar_wait(bar, parity);
+    }
+}
 
-// ---------------------------------------------------------------------------
-// Accumulators. C (rows < nrows, KT columns) += A B, with A either row-major
-// (rows(): A[i*lda + k]) or transposed (cols(): A[k*lda + i]) and B row-major
-// (Bm[k*ldb + c]). visit(nrows, f) hands each thread's results to
-// f(row, col, T* v), v holding V adjacent columns.
-// ---------------------------------------------------------------------------
-
-// V adjacent elements (8 or 16 bytes, aligned) through L2 only: values other CTAs wrote.
+// V adjacent elements (4 to 16 bytes, aligned); values other launches wrote.
 template <typename T, int V>
-__device__ __forceinline__ void ld_cg(const T* p, T* w) {
+__device__ __forceinline__ void ld_n(const T* p, T* w) {
     if constexpr (V * sizeof(T) == 16 && sizeof(T) == 4) {
-        const float4 x = __ldcg(reinterpret_cast<const float4*>(p));
+        const float4 x = *reinterpret_cast<const float4*>(p);
         w[0] = x.x; w[1] = x.y; w[2] = x.z; w[3] = x.w;
     } else if constexpr (V * sizeof(T) == 16) {
-        const double2 x = __ldcg(reinterpret_cast<const double2*>(p));
+        const double2 x = *reinterpret_cast<const double2*>(p);
+        w[0] = x.x; w[1] = x.y;
+    } else if constexpr (V == 2) {
+        const float2 x = *reinterpret_cast<const float2*>(p);
         w[0] = x.x; w[1] = x.y;
     } else {
-        static_assert(V == 2 && sizeof(T) == 4, "8-byte groups are float pairs");
-        const float2 x = __ldcg(reinterpret_cast<const float2*>(p));
-        w[0] = x.x; w[1] = x.y;
+        w[0] = *p;
     }
 }
-
-// Calls f(std::integral_constant<int, m>) with m = min(n, N), for n >= 1: the row
-// blocks a product needs, as a compile-time count.
-template <int N, class F>
-__device__ __forceinline__ void upto(int n, F&& f) {
-    if constexpr (N > 1) {
-        if (n < N) {
-            upto<N - 1>(n, f);
-            return;
-        }
-    }
-    f(std::integral_constant<int, N>{});
+template <typename T, int V>
+__device__ __forceinline__ void st_n(T* p, const T* w) {
+    if constexpr (V * sizeof(T) == 16 && sizeof(T) == 4) *reinterpret_cast<float4*>(p) = make_float4(w[0], w[1], w[2], w[3]);
+    else if constexpr (V * sizeof(T) == 16) *reinterpret_cast<double2*>(p) = make_double2(w[0], w[1]);
+    else if constexpr (V == 2) *reinterpret_cast<float2*>(p) = make_float2(w[0], w[1]);
+    else *p = w[0];
 }
 
-// FP32 register tiles: thread (ty, tx) owns rows ty + 16a (a < NA) and 16-byte
-// column groups at vec*tx + 16*vec*h.
-template <typename T, int KT, int NA>
-struct AccScalar {
-    static constexpr int NB = KT / 16, G = vec<T>(), V = G;
-    T c[NA][NB];
+// ---------------------------------------------------------------------------
+// Products C (M x KT) += P V on shared-memory tiles, P k-major (P[d * ld + row]), V[d * ldv + col].
+// Eight warps: warp group g = 16 rows, and with fewer than 8 groups the column tile is split
+// between the warps of a group. run(): depths [d0, nd); rows and cols of a thread's accumulators
+// are visited in vectors of V adjacent columns.
+// ---------------------------------------------------------------------------
+__device__ __forceinline__ int logical_warp() {
+    // tasks shorter than M leave the last groups idle: other CTAs of the SM get other idle warps
+    return ((threadIdx.x >> 5) + 2 * (blockIdx.x & 3)) & 7;
+}
+
+template <int KT, int M>
+struct AccF32 {
+    using T = float;
+    static constexpr int CS = 128 / M, WN = KT / CS, CN = WN / 16;  // column split, warp and thread columns
+    static constexpr int V = CN >= 4 ? 4 : CN, NV = CN / V;
+    float c[8][CN];
+
+    __device__ __forceinline__ int group() const { return logical_warp() / CS; }
+    __device__ __forceinline__ int row0() const { return 16 * group() + 8 * ((threadIdx.x >> 4) & 1); }
+    __device__ __forceinline__ int col0() const { return (logical_warp() % CS) * WN + V * (threadIdx.x & 15); }
+    static constexpr int vstep() { return 16 * V; }
 
     __device__ __forceinline__ void zero() {
 #pragma unroll
-        for (int a = 0; a < NA; ++a)
+        for (int i = 0; i < 8; ++i)
 #pragma unroll
-            for (int b = 0; b < NB; ++b) c[a][b] = T(0);
+            for (int q = 0; q < CN; ++q) c[i][q] = 0.0f;
     }
-    __device__ __forceinline__ void negate() {
+    __device__ __forceinline__ void run(const float* P, int ld, const float* Vm, int ldv, int d0, int nd, int) {
+        const float* pp = P + row0();
+        const float* vp = Vm + col0();
+#pragma unroll 4
+        for (int d = d0; d < nd; ++d) {
+            float p[8], w[CN];
+            ld_n<float, 4>(pp + d * ld, p);
+            ld_n<float, 4>(pp + d * ld + 4, p + 4);
 #pragma unroll
-        for (int a = 0; a < NA; ++a)
+            for (int v = 0; v < NV; ++v) ld_n<float, V>(vp + d * ldv + vstep() * v, w + V * v);
+            if constexpr (CN == 1) {
 #pragma unroll
-            for (int b = 0; b < NB; ++b) c[a][b] = -c[a][b];
-    }
-
-    template <int MA>
-    __device__ __forceinline__ void rows_n(const T* A, int lda, const T* Bm, int ldb, int depth) {
-        const int ty = threadIdx.x >> 4, tx = threadIdx.x & 15;
-        const T* ap = A + ty * lda;
-        const T* bp = Bm + G * tx;
-        for (int j = 0; j < depth; ++j) {
-            T w[NB];
+                for (int i = 0; i < 8; ++i) c[i][0] = fmaf(p[i], w[0], c[i][0]);
+            } else {
+                unsigned long long w2[CN / 2];
 #pragma unroll
-            for (int h = 0; h < NB / G; ++h) ldv(bp + j * ldb + 16 * G * h, &w[G * h]);
+                for (int q = 0; q < CN / 2; ++q)
+                    asm("mov.b64 %0, {%1, %2};" : "=l"(w2[q]) : "f"(w[2 * q]), "f"(w[2 * q + 1]));
 #pragma unroll
-            for (int a = 0; a < MA; ++a) {
-                const T l = ap[16 * a * lda + j];
+                for (int i = 0; i < 8; ++i) {
+                    unsigned long long p2;
+                    asm("mov.b64 %0, {%1, %1};" : "=l"(p2) : "f"(p[i]));
 #pragma unroll
-                for (int b = 0; b < NB; ++b) c[a][b] += l * w[b];
-            }
-        }
-    }
-
-    template <int MA>
-    __device__ __forceinline__ void cols_n(const T* A, int lda, const T* Bm, int ldb, int depth) {
-        const int ty = threadIdx.x >> 4, tx = threadIdx.x & 15;
-        const T* bp = Bm + G * tx;
-        for (int j = 0; j < depth; ++j) {
-            T w[NB], l[MA];
-#pragma unroll
-            for (int h = 0; h < NB / G; ++h) ldv(bp + j * ldb + 16 * G * h, &w[G * h]);
-#pragma unroll
-            for (int a = 0; a < MA; ++a) l[a] = A[j * lda + ty + 16 * a];
-#pragma unroll
-            for (int a = 0; a < MA; ++a)
-#pragma unroll
-                for (int b = 0; b < NB; ++b) c[a][b] += l[a] * w[b];
-        }
-    }
-
-    // A lower triangular (row-major, zeros above the diagonal): depth block q of 16 reaches
-    // only the row blocks a >= q; the skipped products are exact zeros.
-    template <int MA>
-    __device__ __forceinline__ void rows_lower_n(const T* A, int lda, const T* Bm, int ldb, int depth) {
-        const int ty = threadIdx.x >> 4, tx = threadIdx.x & 15;
-        const T* ap = A + ty * lda;
-        const T* bp = Bm + G * tx;
-#pragma unroll
-        for (int q = 0; q < MA; ++q) {
-            const int j1 = min(depth, 16 * q + 16);
-            for (int j = 16 * q; j < j1; ++j) {
-                T w[NB];
-#pragma unroll
-                for (int h = 0; h < NB / G; ++h) ldv(bp + j * ldb + 16 * G * h, &w[G * h]);
-#pragma unroll
-                for (int a = q; a < MA; ++a) {
-                    const T l = ap[16 * a * lda + j];
-#pragma unroll
-                    for (int b = 0; b < NB; ++b) c[a][b] += l * w[b];
+                    for (int q = 0; q < CN / 2; ++q) {
+                        unsigned long long x;
+                        asm("mov.b64 %0, {%1, %2};" : "=l"(x) : "f"(c[i][2 * q]), "f"(c[i][2 * q + 1]));
+                        asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(x) : "l"(p2), "l"(w2[q]));
+                        asm("mov.b64 {%0, %1}, %2;" : "=f"(c[i][2 * q]), "=f"(c[i][2 * q + 1]) : "l"(x));
+                    }
                 }
             }
         }
     }
-
-    // A read transposed (A[k*lda + i]) from a lower-triangular block: row i needs depth
-    // k >= i, so depth block q reaches only the row blocks a <= q.
-    template <int MA>
-    __device__ __forceinline__ void cols_upper_n(const T* A, int lda, const T* Bm, int ldb, int depth) {
-        const int ty = threadIdx.x >> 4, tx = threadIdx.x & 15;
-        const T* bp = Bm + G * tx;
-#pragma unroll
-        for (int q = 0; q < MA; ++q) {
-            const int j1 = min(depth, 16 * q + 16);
-            for (int j = 16 * q; j < j1; ++j) {
-                T w[NB], l[MA];
-#pragma unroll
-                for (int h = 0; h < NB / G; ++h) ldv(bp + j * ldb + 16 * G * h, &w[G * h]);
-#pragma unroll
-                for (int a = 0; a <= q; ++a) l[a] = A[j * lda + ty + 16 * a];
-#pragma unroll
-                for (int a = 0; a <= q; ++a)
-#pragma unroll
-                    for (int b = 0; b < NB; ++b) c[a][b] += l[a] * w[b];
-            }
-        }
-    }
-
-    // only the 16-row blocks holding one of the first nrows rows are computed
-    __device__ __forceinline__ void rows(const T* A, int lda, const T* Bm, int ldb, int depth, int nrows) {
-        const int na = (nrows + 15) >> 4;
-        if (na > 0) upto<NA>(na, [&](auto m) { rows_n<decltype(m)::value>(A, lda, Bm, ldb, depth); });
-    }
-    __device__ __forceinline__ void cols(const T* A, int lda, const T* Bm, int ldb, int depth, int nrows) {
-        const int na = (nrows + 15) >> 4;
-        if (na > 0) upto<NA>(na, [&](auto m) { cols_n<decltype(m)::value>(A, lda, Bm, ldb, depth); });
-    }
-    // square triangular products (depth <= 16 * row blocks)
-    __device__ __forceinline__ void rows_lower(const T* A, int lda, const T* Bm, int ldb, int depth, int nrows) {
-        const int na = (nrows + 15) >> 4;
-        if (na > 0) upto<NA>(na, [&](auto m) { rows_lower_n<decltype(m)::value>(A, lda, Bm, ldb, depth); });
-    }
-    __device__ __forceinline__ void cols_upper(const T* A, int lda, const T* Bm, int ldb, int depth, int nrows) {
-        const int na = (nrows + 15) >> 4;
-        if (na > 0) upto<NA>(na, [&](auto m) { cols_upper_n<decltype(m)::value>(A, lda, Bm, ldb, depth); });
-    }
-
+    // f(row, col, float* v): V adjacent columns
     template <class F>
     __device__ __forceinline__ void visit(int nrows, F&& f) {
-        const int ty = threadIdx.x >> 4, tx = threadIdx.x & 15;
+        const int r0 = row0(), k0 = col0();
 #pragma unroll
-        for (int a = 0; a < NA; ++a) {
-            const int t = ty + 16 * a;
-            if (t < nrows)
+        for (int i = 0; i < 8; ++i)
+            if (r0 + i < nrows)
 #pragma unroll
-                for (int h = 0; h < NB / G; ++h) f(t, G * tx + 16 * G * h, &c[a][G * h]);
-        }
+                for (int v = 0; v < NV; ++v) f(r0 + i, k0 + vstep() * v, &c[i][V * v]);
     }
 };
 
-// FP64 tensor tiles (KT = 64): warp w owns columns [8w, 8w+8) and the 8-row
-// m8n8k4 tiles down to row 8*MT; lane (g = lane/4, t = lane%4) holds rows 8m+g,
-// columns 8w+2t and 8w+2t+1. The depth must be a multiple of 4 with the padded
-// depths zero in both operands.
-template <int MT>
-struct AccDmma {
-    static constexpr int V = 2;
-    double c[MT][2];
+// FP64 tensor tiles: lane (g = lane / 4, t = lane % 4) holds row 8m + g, columns 8n + 2t and + 1 of
+// the warp's 16 x WN tile. The depth runs in steps of 4; padded depths are zero in both operands.
+template <int KT, int M>
+struct AccF64 {
+    using T = double;
+    static constexpr int CS = 128 / M, WN = KT / CS, NN = WN / 8, V = 2;
+    double c[2][NN][2];
 
+    __device__ __forceinline__ int group() const { return logical_warp() / CS; }
+    __device__ __forceinline__ int colw() const { return (logical_warp() % CS) * WN; }
     __device__ __forceinline__ void zero() {
 #pragma unroll
-        for (int m = 0; m < MT; ++m) c[m][0] = c[m][1] = 0.0;
-    }
-    __device__ __forceinline__ void negate() {
+        for (int m = 0; m < 2; ++m)
 #pragma unroll
-        for (int m = 0; m < MT; ++m) {
-            c[m][0] = -c[m][0];
-            c[m][1] = -c[m][1];
+            for (int n = 0; n < NN; ++n) c[m][n][0] = c[m][n][1] = 0.0;
+    }
+    template <int MM>
+    __device__ __forceinline__ void steps(const double* P, int ld, const double* Vm, int ldv, int d0, int nd) {
+        const int lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
+        const double* pp = P + t * ld + 16 * group() + g;
+        const double* vp = Vm + t * ldv + colw() + g;
+        for (int d = d0; d < nd; d += 4) {
+            double a[MM], b[NN];
+#pragma unroll
+            for (int m = 0; m < MM; ++m) a[m] = pp[d * ld + 8 * m];
+#pragma unroll
+            for (int n = 0; n < NN; ++n) b[n] = vp[d * ldv + 8 * n];
+#pragma unroll
+            for (int m = 0; m < MM; ++m)
+#pragma unroll
+                for (int n = 0; n < NN; ++n)
+                    asm("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0, %1}, {%2}, {%3}, {%0, %1};\n"
+                        : "+d"(c[m][n][0]), "+d"(c[m][n][1])
+                        : "d"(a[m]), "d"(b[n]));
         }
     }
-
-    static __device__ __forceinline__ void mma(double (&d)[2], double a, double b) {
-        asm("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0, %1}, {%2}, {%3}, {%0, %1};\n"
-            : "+d"(d[0]), "+d"(d[1])
-            : "d"(a), "d"(b));
+    // rows: the task's rows (a group whose last 8 rows are past them runs one row tile)
+    __device__ __forceinline__ void run(const double* P, int ld, const double* Vm, int ldv, int d0, int nd, int rows) {
+        if (16 * group() + 8 < rows) steps<2>(P, ld, Vm, ldv, d0, nd);
+        else steps<1>(P, ld, Vm, ldv, d0, nd);
     }
-
-    template <int MM, bool TRANS>
-    __device__ __forceinline__ void run(const double* A, int lda, const double* Bm, int ldb, int depth) {
-        const int lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3, n0 = 8 * (threadIdx.x >> 5);
-        const double* bp = Bm + t * ldb + n0 + g;
-        for (int k = 0; k < depth; k += 4) {
-            const double b = bp[k * ldb];
-#pragma unroll
-            for (int m = 0; m < MM; ++m) {
-                const double a = TRANS ? A[(k + t) * lda + 8 * m + g] : A[(8 * m + g) * lda + k + t];
-                mma(c[m], a, b);
-            }
-        }
-    }
-
-    // Triangular A (lower, zeros above the diagonal): depth steps [8q, 8q+8) reach the row
-    // tiles m >= q (row-major: rows need k <= row) or m <= q (transposed: k >= row).
-    template <int MM, bool TRANS>
-    __device__ __forceinline__ void run_tri(const double* A, int lda, const double* Bm, int ldb, int depth) {
-        const int lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3, n0 = 8 * (threadIdx.x >> 5);
-        const double* bp = Bm + t * ldb + n0 + g;
-#pragma unroll
-        for (int q = 0; q < MM; ++q) {
-#pragma unroll
-            for (int h = 0; h < 2; ++h) {
-                const int k = 8 * q + 4 * h;
-                if (k >= depth) break;
-                const double b = bp[k * ldb];
-#pragma unroll
-                for (int m = TRANS ? 0 : q; m < (TRANS ? q + 1 : MM); ++m) {
-                    const double a = TRANS ? A[(k + t) * lda + 8 * m + g] : A[(8 * m + g) * lda + k + t];
-                    mma(c[m], a, b);
-                }
-            }
-        }
-    }
-    __device__ __forceinline__ void rows_lower(const double* A, int lda, const double* Bm, int ldb, int depth,
-                                               int nrows) {
-        const int nm = (nrows + 7) >> 3;
-        if (nm > 0) upto<MT>(nm, [&](auto m) { run_tri<decltype(m)::value, false>(A, lda, Bm, ldb, depth); });
-    }
-    __device__ __forceinline__ void cols_upper(const double* A, int lda, const double* Bm, int ldb, int depth,
-                                               int nrows) {
-        const int nm = (nrows + 7) >> 3;
-        if (nm > 0) upto<MT>(nm, [&](auto m) { run_tri<decltype(m)::value, true>(A, lda, Bm, ldb, depth); });
-    }
-
-    template <bool TRANS>
-    __device__ __forceinline__ void dispatch(const double* A, int lda, const double* Bm, int ldb, int depth,
-                                             int nrows) {
-        const int nm = (nrows + 7) >> 3;
-        if (nm > 0) upto<MT>(nm, [&](auto m) { run<decltype(m)::value, TRANS>(A, lda, Bm, ldb, depth); });
-    }
-    __device__ __forceinline__ void rows(const double* A, int lda, const double* Bm, int ldb, int depth,
-                                         int nrows) {
-        dispatch<false>(A, lda, Bm, ldb, depth, nrows);
-    }
-    __device__ __forceinline__ void cols(const double* A, int lda, const double* Bm, int ldb, int depth,
-                                         int nrows) {
-        dispatch<true>(A, lda, Bm, ldb, depth, nrows);
-    }
-
     template <class F>
     __device__ __forceinline__ void visit(int nrows, F&& f) {
-        const int lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3, n0 = 8 * (threadIdx.x >> 5);
+        const int lane = threadIdx.x & 31, r = 16 * group() + (lane >> 2), k0 = colw() + 2 * (lane & 3);
 #pragma unroll
-        for (int m = 0; m < MT; ++m)
-            if (8 * m + g < nrows) f(8 * m + g, n0 + 2 * t, c[m]);
+        for (int m = 0; m < 2; ++m)
+            if (r + 8 * m < nrows)
+#pragma unroll
+                for (int n = 0; n < NN; ++n) f(r + 8 * m, k0 + 8 * n, c[m][n]);
     }
 };
 
-template <typename T, int KT, int TR>
-struct AccSel {
-    using type = AccScalar<T, KT, TR / 16>;
-};
-template <int TR>
-struct AccSel<double, 64, TR> {
-    using type = AccDmma<TR / 8>;
-};
-template <typename T, int KT, int TR>
-using Acc = typename AccSel<T, KT, TR>::type;
+template <typename T, int KT, int M>
+using Acc = std::conditional_t<sizeof(T) == 8, AccF64<KT, M>, AccF32<KT, M>>;
 
-// Zero rows [r0, r1) x columns [0, ncols) of a shared tile (padding of a product's depth).
+// ---------------------------------------------------------------------------
+// Children's update rows
+// ---------------------------------------------------------------------------
 template <typename T>
-__device__ __forceinline__ void zero_rows(T* D, int ld, int r0, int r1, int ncols) {
-    for (int e = threadIdx.x; e < (r1 - r0) * ncols; e += NT) {
-        const int r = e / ncols, c = e - r * ncols;
-        D[(r0 + r) * ld + c] = T(0);
-    }
+__device__ __forceinline__ bool reached(const SweepArgs<T>& a, int front, int tile) {
+    return !a.reach || __ldcg(a.reach + (int64_t)front * a.reach_tiles + tile);
 }
-// Zero columns [c0, c1) of rows [0, nrows).
+// A front row's record, without the children that are off the sources' paths (their update rows
+// were never written).
 template <typename T>
-__device__ __forceinline__ void zero_cols(T* D, int ld, int nrows, int c0, int c1) {
-    const int w = c1 - c0;
-    for (int e = threadIdx.x; e < nrows * w; e += NT) {
-        const int r = e / w, c = e - r * w;
-        D[r * ld + c0 + c] = T(0);
+__device__ __forceinline__ int4 live_record(const SweepArgs<T>& a, int64_t q, int tile) {
+    int4 r = a.rec[q];
+    if (a.reach) {
+        const int32_t* ch = a.rec_child + 3 * q;
+        const int c0 = ch[0], c1 = ch[1], c2 = ch[2];
+        if (r.x >= 0 && !reached(a, c0, tile)) r.x = -1;
+        if (r.y >= 0 && !reached(a, c1, tile)) r.y = -1;
+        if (r.z >= 0 && !reached(a, c2, tile)) r.z = -1;
+    }
+    return r;
+}
+// w (+ or -)= the record's rows after the first three
+template <typename T, int V, bool SUB>
+__device__ __forceinline__ void add_more(const SweepArgs<T>& a, int more, int tile, const T* U, T* w) {
+    const int n = a.more[more];
+    for (int e = 0; e < n; ++e) {
+        if (!reached(a, a.more[more + 2 + 2 * e], tile)) continue;
+        T u[V];
+        ld_n<T, V>(U + (int64_t)a.more[more + 1 + 2 * e] * a.K, u);
+#pragma unroll
+        for (int q = 0; q < V; ++q) w[q] = SUB ? w[q] - u[q] : w[q] + u[q];
     }
 }
 
-
-template <typename T, int KT, int TR>
-__global__ void __launch_bounds__(NT, 3) k_fwd(SolveArgs<T> a, int32_t t0) {
-    constexpr int VPR = KT / vec<T>(), LW = ld_rows<T, KT>(), LA = ld_fwd_a<T, TR>(), DP = depth_pad<T>();
-    using AccT = Acc<T, KT, TR>;
-    constexpr bool kSepQ = separate_q<T>();
-    extern __shared__ __align__(16) unsigned char smraw[];
-    T* Wt = reinterpret_cast<T*>(smraw);   // TR x LW: W, then this chunk's update rows
-    T* Li = Wt + TR * LW;                   // TR x LA: inverse diagonal block (first chunk)
-    T* Pn = kSepQ ? Li + TR * LA : Li;      // TR x LA: this chunk's rows of Q_s
-    T* St = Pn + TR * LA;                   // a.stage x KT: children's update rows
-    __shared__ int grs[TR + 1];
-    __shared__ unsigned char live[stage_rows<T, TR>()];
-    static_assert(sizeof(T) == 4 || KT == kReachCols, "the heat solve's reach tiles are its column tiles");
-    const int2 task = a.tasks[t0 + blockIdx.x];
-    const int s = task.x, chunk = task.y;
-    if (a.reach && !a.reach[(int64_t)s * a.reach_tiles + blockIdx.y]) return;
-    const DevPlan& p = a.p;
-    const int tid = threadIdx.x;
-    const int K = a.K, k0 = blockIdx.y * KT;
-    const int c0 = p.sn_c0[s], ns = p.sn_c0[s + 1] - c0, m = p.sn_m[s], nr = m - ns;
-    const int nsp = (ns + DP - 1) / DP * DP;  // product depth
-    const int64_t fb = p.sn_rowptr[s];
-    const int q0 = chunk * TR;
-    const int nq = nr > 0 ? min(TR, nr - q0) : 0;
-    const bool want_x = chunk == 0;
-    const bool q_early = nq > 0 && (kSepQ || !want_x);  // Q rows come with the first copies
-    const T* Q = a.val + p.sn_valptr[s] + (int64_t)(ns + q0) * ns;
-
-    // the inverse block, this chunk's rows of Q_s, the right-hand side rows and
-    // the first children's rows are in flight together (identity right-hand
-    // sides are built in place)
-    if (want_x) {
-        const T* inv = a.inv + p.sn_invptr[s];
-        for (int e = tid; e < ns * ns; e += NT) {
-            const int i = e / ns, j = e - i * ns;
-            copy_async(&Li[i * LA + j], inv + e);
-        }
-    }
-    if (q_early)
-        for (int e = tid; e < nq * ns; e += NT) {
-            const int r = e / ns, j = e - r * ns;
-            copy_async(&Pn[r * LA + j], Q + e);
-        }
-    if (a.delta_src) {
-        for (int e = tid; e < ns * KT; e += NT) {
-            const int f = e / KT, c = e - f * KT;
-            Wt[f * LW + c] = (a.delta_src[k0 + c] == c0 + f) ? T(1) : T(0);
-        }
-    } else {
-        for (int i = tid; i < ns * VPR; i += NT) {
-            const int f = i / VPR, v = i - f * VPR;
-            copy16_async(Wt + f * LW + v * vec<T>(), a.R + (int64_t)(c0 + f) * K + k0 + v * vec<T>());
-        }
-    }
-    if (nsp > ns) {  // padded depth: zero in both operands
-        zero_rows(Wt, LW, ns, nsp, KT);
-        if (want_x) zero_cols(Li, LA, ns, ns, nsp);
-        if (q_early) zero_cols(Pn, LA, nq, ns, nsp);
-    }
-    const GatherRange g1 = gather_open(a, fb, 0, ns, grs);
-    if (g1.E > 0) gather_issue<T, KT, TR>(a, g1, 0, k0, St, live);
-    copy_async_commit();
-    gather_finish<T, KT, TR, true>(a, g1, k0, Wt, LW, ns, St, live, grs);
-
-    // the children's rows of this chunk's update rows arrive while X_s and U_s are formed
-    GatherRange g2{0, 0};
-    if (nq > 0) {
-        g2 = gather_open(a, fb, ns + q0, nq, grs);
-        if (g2.E > 0) gather_issue<T, KT, TR>(a, g2, 0, k0, St, live);
-        copy_async_commit();
-    }
-    AccT acc;
-    if (want_x) {  // X = inv(L_ss) W, straight from the registers to B
-        acc.zero();
-        acc.rows_lower(Li, LA, Wt, LW, nsp, ns);
-        T* xb = a.B + (int64_t)c0 * K + k0;
-        acc.visit(ns, [&](int r, int c, T* v) { st_n<T, AccT::V>(xb + (int64_t)r * K + c, v); });
-    }
-    if (nq <= 0) return;
-    if (!q_early) {  // one shared tile: the Q rows take the inverse's place now
-        __syncthreads();
-        for (int e = tid; e < nq * ns; e += NT) {
-            const int r = e / ns, j = e - r * ns;
-            copy_async(&Pn[r * LA + j], Q + e);
-        }
-        if (nsp > ns) zero_cols(Pn, LA, nq, ns, nsp);
-        copy_async_commit();
-        copy_async_wait();
-        __syncthreads();
-    }
-    // U_s rows of this chunk = Q_s W + the children's rows landing on them
-    acc.zero();
-    acc.rows(Pn, LA, Wt, LW, nsp, nq);
-    __syncthreads();  // every thread is done reading W
-    acc.visit(nq, [&](int r, int c, T* v) { st_n<T, AccT::V>(Wt + r * LW + c, v); });
-    gather_finish<T, KT, TR, false>(a, g2, k0, Wt, LW, nq, St, live, grs);
-    tile_rows_to_global<T, KT>(a.U + (a.uoff[s] + q0) * (int64_t)K + k0, K, Wt, LW, nq);
-}
-
-template <typename T, int KT, int TR>
-__global__ void __launch_bounds__(NT, 3) k_bwd(SolveArgs<T> a, int32_t t0) {
-    constexpr int VPR = KT / vec<T>(), LW = ld_rows<T, KT>(), LA = ld_bwd_a<T, TR>(), DP = depth_pad<T>();
-    constexpr int PS = RC * LA, XS = RC * LW;  // one chunk buffer: panel rows, gathered solution rows
-    static_assert(2 * (PS + XS) >= TR * LW + TR * LA, "the finishing tiles alias the chunk buffers");
-    static_assert(sizeof(T) == 4 || KT == kReachCols, "the heat solve's reach tiles are its column tiles");
-    using AccT = Acc<T, KT, TR>;
-    extern __shared__ __align__(16) unsigned char smraw[];
-    T* buf = reinterpret_cast<T*>(smraw);
-    T* Ys = buf;             // TR x LW: y_s, after the gather
-    T* Ms = buf + TR * LW;   // TR x LA inverse diagonal block, after the gather
-    __shared__ int last_arrival;
-    const int2 task = a.tasks[t0 + blockIdx.x];
-    const int s = task.x, split = task.y;
-    const DevPlan& p = a.p;
-    const int tid = threadIdx.x;
-    const int K = a.K, k0 = blockIdx.y * KT;
-    const int c0 = p.sn_c0[s], ns = p.sn_c0[s + 1] - c0, m = p.sn_m[s], nr = m - ns;
-    const int nsp = (ns + DP - 1) / DP * DP;
-    const int nspl = a.nsplit[s];
-    const int q0 = split * kSplitRows, q1 = min(nr, q0 + kSplitRows);
-    const T* P = a.val + p.sn_valptr[s];
-    const int32_t* rows = p.rows + p.sn_rowptr[s];
-
-    // chunk ci of the split's structure rows into buffer ci & 1
-    auto issue = [&](int ci) {
-        const int qq = q0 + ci * RC, nc = min(RC, q1 - qq), ncp = (nc + DP - 1) / DP * DP;
-        T* Ps = buf + (ci & 1) * (PS + XS);
-        T* Xg = Ps + PS;
-        for (int e = tid; e < nc * ns; e += NT) {
-            const int r = e / ns, j = e - r * ns;
-            copy_async(&Ps[r * LA + j], P + (int64_t)(ns + qq + r) * ns + j);
-        }
-        for (int i = tid; i < nc * VPR; i += NT) {
-            const int r = i / VPR, v = i - r * VPR;
-            copy16_async(Xg + r * LW + v * vec<T>(), a.B + (int64_t)rows[ns + qq + r] * K + k0 + v * vec<T>());
-        }
-        if (ncp > nc) {
-            zero_rows(Ps, LA, nc, ncp, TR);
-            zero_rows(Xg, LW, nc, ncp, KT);
-        }
-        copy_async_commit();
-    };
-    AccT acc;
-    acc.zero();
-    const int nchunks = q1 > q0 ? (q1 - q0 + RC - 1) / RC : 0;
-    if (nchunks > 0) issue(0);
-    for (int ci = 0; ci < nchunks; ++ci) {
-        if (ci + 1 < nchunks) {
-            issue(ci + 1);
-            copy_async_wait_prev();
+// R rows' vectors at column k (16 bytes each) minus their records' rows: base[] holds the
+// right-hand-side rows (negative: zero row). All loads of the R rows are in flight together.
+template <typename T, int R>
+__device__ __forceinline__ void gather_rows(const SweepArgs<T>& a, const int4* rec, const int64_t* base, int k, int tile,
+                                            const int* delta, T (*w)[vec<T>()]) {
+    constexpr int G = vec<T>();
+    const T* U = a.U + k;
+    T u[R][G];
+#pragma unroll
+    for (int i = 0; i < R; ++i) {
+        if (a.delta_src) {
+#pragma unroll
+            for (int q = 0; q < G; ++q) w[i][q] = (base[i] >= 0 && delta[q] == (int)base[i]) ? T(1) : T(0);
+        } else if (base[i] >= 0) {
+            ld_n<T, G>(a.R + base[i] * a.K + k, w[i]);
         } else {
-            copy_async_wait();
+#pragma unroll
+            for (int q = 0; q < G; ++q) w[i][q] = T(0);
         }
-        __syncthreads();
-        const T* Ps = buf + (ci & 1) * (PS + XS);
-        const int nc = min(RC, q1 - q0 - ci * RC);
-        acc.cols(Ps, LA, Ps + PS, LW, (nc + DP - 1) / DP * DP, ns);
-        __syncthreads();
     }
-
-    const bool zero_y = a.reach && !a.reach[(int64_t)s * a.reach_tiles + blockIdx.y];
-    if (nspl > 1) {
-        T* part = a.part + a.poff[s] * (int64_t)PT * K + k0;
-        T* mine = part + (int64_t)split * PT * K;
-        acc.visit(ns, [&](int r, int c, T* v) { st_n<T, AccT::V>(mine + (int64_t)r * K + c, v); });
-        __threadfence();
-        __syncthreads();
-        if (tid == 0) {
-            const int ticket = atomicAdd(&a.counters[(int64_t)s * a.ktiles + blockIdx.y], 1);
-            last_arrival = ticket == nspl - 1;
+#pragma unroll
+    for (int s = 0; s < 3; ++s) {
+#pragma unroll
+        for (int i = 0; i < R; ++i) {
+            const int src = s == 0 ? rec[i].x : (s == 1 ? rec[i].y : rec[i].z);
+            if (src >= 0) ld_n<T, G>(U + (int64_t)src * a.K, u[i]);
         }
-        __syncthreads();
-        if (!last_arrival) return;
-        __threadfence();
-        // the partial sums in split order; four splits' vectors are loaded before any is added,
-        // so the loads overlap instead of waiting on one another
-        acc.visit(ns, [&](int r, int c, T* v) {
-            constexpr int V = AccT::V;
-            const T* base = part + (int64_t)r * K + c;
-            const int64_t ss = (int64_t)PT * K;  // one split's slot
-            T sum[V];
 #pragma unroll
-            for (int q = 0; q < V; ++q) sum[q] = T(0);
-            int sp = 0;
-            for (; sp + 4 <= nspl; sp += 4) {
-                T w[4][V];
+        for (int i = 0; i < R; ++i) {
+            const int src = s == 0 ? rec[i].x : (s == 1 ? rec[i].y : rec[i].z);
+            if (src >= 0) {
 #pragma unroll
-                for (int u = 0; u < 4; ++u) ld_cg<T, V>(base + (sp + u) * ss, w[u]);
-#pragma unroll
-                for (int u = 0; u < 4; ++u)
-#pragma unroll
-                    for (int q = 0; q < V; ++q) sum[q] += w[u][q];
+                for (int q = 0; q < G; ++q) w[i][q] -= u[i][q];
             }
-            for (; sp < nspl; ++sp) {
-                T w[V];
-                ld_cg<T, V>(base + sp * ss, w);
-#pragma unroll
-                for (int q = 0; q < V; ++q) sum[q] += w[q];
-            }
-#pragma unroll
-            for (int q = 0; q < V; ++q) v[q] = sum[q];
-        });
-        if (tid == 0) a.counters[(int64_t)s * a.ktiles + blockIdx.y] = 0;
+        }
     }
-    // X_s = inv(L_ss)^T y_s - Q_s^T X_r (y_s = 0 off the sources' paths)
-    acc.negate();
-    if (!zero_y) {
-        const T* inv = a.inv + p.sn_invptr[s];
-        for (int e = tid; e < ns * ns; e += NT) {
-            const int i = e / ns, j = e - i * ns;
-            copy_async(&Ms[i * LA + j], inv + e);
-        }
-        for (int i = tid; i < ns * VPR; i += NT) {
-            const int r = i / VPR, v = i - r * VPR;
-            copy16_async(Ys + r * LW + v * vec<T>(), a.B + (int64_t)(c0 + r) * K + k0 + v * vec<T>());
-        }
-        copy_async_commit();
-        if (nsp > ns) {
-            zero_rows(Ms, LA, ns, nsp, TR);
-            zero_rows(Ys, LW, ns, nsp, KT);
-        }
-        copy_async_wait();
-        __syncthreads();
-        acc.cols_upper(Ms, LA, Ys, LW, nsp, ns);
-    }
-    T* out = a.B + (int64_t)c0 * K + k0;
-    acc.visit(ns, [&](int r, int c, T* v) { st_n<T, AccT::V>(out + (int64_t)r * K + c, v); });
+#pragma unroll
+    for (int i = 0; i < R; ++i)
+        if (rec[i].w >= 0) add_more<T, G, true>(a, rec[i].w, tile, U, w[i]);
 }
 
-// reach[s * tiles + t]: some source of column tile t (kReachCols columns) has supernode s on
-// its path to the root.
-__global__ void k_reach(const int32_t* __restrict__ col_sn, const int32_t* __restrict__ parent,
+// ---------------------------------------------------------------------------
+// Forward
+// ---------------------------------------------------------------------------
+template <typename T, int KT, int M, bool WIDE>
+__global__ void __launch_bounds__(NT, 2) k_fwd(SweepArgs<T> a, int32_t t0) {
+    constexpr int G = vec<T>(), VPR = KT / G, RPP = NT / VPR, LW = ld_rhs<T, KT>();
+    constexpr int S = WIDE ? 3 : kNarrowCols / DC;  // a narrow front's chunks are all resident
+    constexpr int PS = panel_stage<T, M>(), VS = DC * LW;
+    extern __shared__ __align__(128) unsigned char smraw[];
+    T* Ps = reinterpret_cast<T*>(smraw);
+    T* Vs = Ps + S * PS;
+    __shared__ __align__(8) uint64_t bar[S];
+    __shared__ int4 crec[WIDE ? 1 : kNarrowCols], urec[M];
+    allow_dependents();
+    const int tid = threadIdx.x, tile = blockIdx.y, k0 = tile * KT;
+    const SweepTask t = a.tasks[t0 + blockIdx.x];
+    if (a.reach) {
+        wait_predecessor();
+        if (!reached(a, t.front, tile)) return;
+    }
+    const int ld = panel_stride<T>(t.h);
+    const T* panel = a.panel + (sizeof(T) == 8 ? t.off64 : t.off32);
+    const int depth4 = (t.depth + 3) & ~3, nch = (t.depth + DC - 1) / DC;
+    auto chunk_rows = [&](int c) { return min(DC, depth4 - DC * c); };
+    auto request = [&](int c) {  // chunk c's panel rows, by one thread
+        const uint32_t bytes = (uint32_t)(chunk_rows(c) * ld * (int)sizeof(T));
+        tc::mbar_arrive_expect_tx(&bar[c % S], bytes);
+        tc::bulk_load(Ps + (c % S) * PS, panel + (int64_t)c * DC * ld, bytes, &bar[c % S]);
+    };
+    if (tid == 0) {
+        for (int s = 0; s < S; ++s) tc::mbar_init(&bar[s], 1);
+        tc::fence_mbar_init();
+        for (int c = 0; c < min(nch, WIDE ? S - 1 : S); ++c) request(c);
+    }
+    if (a.gathers) {
+        if (!WIDE)
+            for (int i = tid; i < t.ns; i += NT) crec[i] = live_record(a, t.row0 + i, tile);
+        for (int i = tid; i < t.h; i += NT)
+            urec[i] = t.r0 + i >= t.ns ? live_record(a, t.row0 + t.r0 + i, tile) : make_int4(-1, -1, -1, -1);
+    }
+    if (!a.reach) wait_predecessor();
+    __syncthreads();
+
+    if constexpr (!WIDE) {
+        // W, four rows per thread in flight
+        const int v = tid % VPR, rr = tid / VPR;
+        int delta[G];
+        if (a.delta_src) {
+#pragma unroll
+            for (int q = 0; q < G; ++q) delta[q] = a.delta_src[k0 + v * G + q];
+        }
+        constexpr int R = 4;
+        for (int f0 = rr; f0 < depth4; f0 += R * RPP) {
+            int4 rec[R];
+            int64_t base[R];
+            T w[R][G];
+#pragma unroll
+            for (int i = 0; i < R; ++i) {
+                const int f = f0 + i * RPP;
+                base[i] = f < t.depth ? t.c0 + f : -1;
+                rec[i] = (a.gathers && f < t.depth) ? crec[f] : make_int4(-1, -1, -1, -1);
+            }
+            gather_rows<T, R>(a, rec, base, k0 + v * G, tile, delta, w);
+#pragma unroll
+            for (int i = 0; i < R; ++i) {
+                const int f = f0 + i * RPP;
+                if (f < depth4) st_n<T, G>(Vs + f * LW + v * G, w[i]);
+            }
+        }
+    }
+    auto load_chunk = [&](int c) {  // wide: chunk c of the assembled right-hand sides
+        T* V = Vs + (c % S) * VS;
+        const int nd = min(DC, t.depth - DC * c), n4 = chunk_rows(c);
+        for (int e = tid; e < n4 * VPR; e += NT) {
+            const int f = e / VPR, v = e - f * VPR;
+            T* dst = V + f * LW + v * G;
+            if (f < nd) {
+                copy16_async(dst, a.W + (int64_t)(t.wrow + DC * c + f) * a.K + k0 + v * G);
+            } else {
+                T z[G] = {};
+                st_n<T, G>(dst, z);
+            }
+        }
+    };
+    if constexpr (WIDE) {
+        for (int c = 0; c < S - 1; ++c) {
+            if (c < nch) load_chunk(c);
+            copy_async_commit();
+        }
+    }
+    // the children's rows that land on this task's structure rows start the accumulators
+    Acc<T, KT, M> acc;
+    using A = Acc<T, KT, M>;
+    acc.zero();
+    if (a.gathers && t.r0 + t.h > t.ns) {
+        const T* U = a.U + k0;
+#pragma unroll
+        for (int s = 0; s < 3; ++s)
+            acc.visit(t.h, [&](int r, int c, T* v) {
+                const int src = s == 0 ? urec[r].x : (s == 1 ? urec[r].y : urec[r].z);
+                if (src < 0) return;
+                T u[A::V];
+                ld_n<T, A::V>(U + (int64_t)src * a.K + c, u);
+#pragma unroll
+                for (int q = 0; q < A::V; ++q) v[q] += u[q];
+            });
+        acc.visit(t.h, [&](int r, int c, T* v) {
+            if (urec[r].w >= 0) add_more<T, A::V, false>(a, urec[r].w, tile, U + c, v);
+        });
+    }
+    // rows of the inverse stop at the diagonal
+    const int g16 = 16 * acc.group(), last = t.r0 + g16 + 15;
+    const int limit = g16 < t.h ? (last < t.ns ? min(t.depth, last + 1) : t.depth) : 0;
+    for (int c = 0; c < nch; ++c) {
+        if constexpr (WIDE) copy_async_wait<S - 2>();
+        wait_panel(&bar[c % S], (c / S) & 1, a.err);
+        if (WIDE || c == 0) __syncthreads();
+        if constexpr (WIDE) {
+            if (c + S - 1 < nch) {
+                if (tid == 0) request(c + S - 1);
+                load_chunk(c + S - 1);
+            }
+            copy_async_commit();
+        }
+        const int nd = min(DC, limit - DC * c);
+        if (nd > 0) acc.run(Ps + (c % S) * PS, ld, Vs + (c % S) * VS, LW, 0, nd, t.h);
+    }
+    T* y = a.Y + (int64_t)t.c0 * a.K + k0;
+    T* u = a.U + (t.urow - t.ns) * (int64_t)a.K + k0;
+    acc.visit(t.h, [&](int r, int c, T* v) {
+        const int R = t.r0 + r;
+        st_n<T, A::V>((R < t.ns ? y : u) + (int64_t)R * a.K + c, v);
+    });
+}
+
+// Right-hand sides of the wide levels' fronts: W = b - the children's update rows.
+template <typename T, int KT>
+__global__ void __launch_bounds__(NT) k_assemble(SweepArgs<T> a, int32_t r0, int32_t nrows) {
+    constexpr int G = vec<T>(), VPR = KT / G, RPP = NT / VPR;
+    allow_dependents();
+    const int tile = blockIdx.y, v = threadIdx.x % VPR, i = blockIdx.x * RPP + threadIdx.x / VPR;
+    const int k = tile * KT + v * G;
+    const int4 row = i < nrows ? a.asm_rows[r0 + i] : make_int4(0, 0, -1, 0);
+    int4 rec[1] = {make_int4(-1, -1, -1, -1)};
+    wait_predecessor();
+    if (i >= nrows || !reached(a, row.z, tile)) return;
+    rec[0] = live_record(a, row.x, tile);
+    const int64_t base[1] = {row.y};
+    int delta[G];
+    if (a.delta_src) {
+#pragma unroll
+        for (int q = 0; q < G; ++q) delta[q] = a.delta_src[k + q];
+    }
+    T w[1][G];
+    gather_rows<T, 1>(a, rec, base, k, tile, delta, w);
+    st_n<T, G>(a.W + (int64_t)(r0 + i) * a.K + k, w[0]);
+}
+
+// ---------------------------------------------------------------------------
+// Backward
+// ---------------------------------------------------------------------------
+template <typename T, int KT, int M>
+__global__ void __launch_bounds__(NT, sizeof(T) == 8 ? 2 : 3) k_bwd(SweepArgs<T> a, int32_t t0) {
+    constexpr int G = vec<T>(), VPR = KT / G, LW = ld_rhs<T, KT>(), S = 3;
+    constexpr int PS = panel_stage<T, M>(), VS = DC * LW;
+    extern __shared__ __align__(128) unsigned char smraw[];
+    T* Ps = reinterpret_cast<T*>(smraw);
+    T* Vs = Ps + S * PS;
+    int32_t* idx = reinterpret_cast<int32_t*>(Vs + S * VS);  // the task's depth rows
+    __shared__ __align__(8) uint64_t bar[S];
+    allow_dependents();
+    const int tid = threadIdx.x, tile = blockIdx.y, k0 = tile * KT;
+    const SweepTask t = a.tasks[t0 + blockIdx.x];
+    const int own = t.ns - t.r0;  // depth rows [0, own): y_s; then the structure rows
+    // y_s = 0 off the sources' paths (reach was written launches ago: the forward sweep has read it)
+    const int d0 = (a.reach && !reached(a, t.front, tile)) ? own : 0;
+    const int ld = panel_stride<T>(t.h);
+    const T* panel = a.panel + (sizeof(T) == 8 ? t.off64 : t.off32);
+    const int nrow = t.depth - d0, nrow4 = (nrow + 3) & ~3, nch = (nrow + DC - 1) / DC;
+    auto chunk_rows = [&](int c) { return min(DC, nrow4 - DC * c); };
+    auto request = [&](int c) {
+        const uint32_t bytes = (uint32_t)(chunk_rows(c) * ld * (int)sizeof(T));
+        tc::mbar_arrive_expect_tx(&bar[c % S], bytes);
+        tc::bulk_load(Ps + (c % S) * PS, panel + (int64_t)(d0 + c * DC) * ld, bytes, &bar[c % S]);
+    };
+    if (tid == 0) {
+        for (int s = 0; s < S; ++s) tc::mbar_init(&bar[s], 1);
+        tc::fence_mbar_init();
+        for (int c = 0; c < min(nch, S - 1); ++c) request(c);
+    }
+    for (int i = tid; i < nrow; i += NT) idx[i] = a.rows[t.row0 + t.r0 + d0 + i];
+    wait_predecessor();
+    __syncthreads();
+    auto load_chunk = [&](int c) {
+        T* V = Vs + (c % S) * VS;
+        const int nd = min(DC, nrow - DC * c), n4 = chunk_rows(c);
+        for (int e = tid; e < n4 * VPR; e += NT) {
+            const int f = e / VPR, v = e - f * VPR, d = d0 + DC * c + f;
+            T* dst = V + f * LW + v * G;
+            if (f < nd) {
+                const T* src = d < own ? a.Y : a.X;
+                copy16_async(dst, src + (int64_t)idx[DC * c + f] * a.K + k0 + v * G);
+            } else {
+                T z[G] = {};
+                st_n<T, G>(dst, z);
+            }
+        }
+    };
+    for (int c = 0; c < S - 1; ++c) {
+        if (c < nch) load_chunk(c);
+        copy_async_commit();
+    }
+    Acc<T, KT, M> acc;
+    using A = Acc<T, KT, M>;
+    acc.zero();
+    const int g16 = 16 * acc.group();
+    for (int c = 0; c < nch; ++c) {
+        copy_async_wait<S - 2>();
+        wait_panel(&bar[c % S], (c / S) & 1, a.err);
+        __syncthreads();
+        if (c + S - 1 < nch) {
+            if (tid == 0) request(c + S - 1);
+            load_chunk(c + S - 1);
+        }
+        copy_async_commit();
+        // column j of the inverse starts at row j
+        const int nd = min(DC, nrow - DC * c), from = max(0, g16 - d0 - DC * c);
+        if (g16 < t.h && from < nd) acc.run(Ps + (c % S) * PS, ld, Vs + (c % S) * VS, LW, from, nd, t.h);
+    }
+    T* x = a.X + (int64_t)(t.c0 + t.r0) * a.K + k0;
+    acc.visit(t.h, [&](int r, int c, T* v) { st_n<T, A::V>(x + (int64_t)r * a.K + c, v); });
+}
+
+// reach[f * tiles + t]: some source of column tile t (kReachCols columns) has front f on its path
+// to the root.
+__global__ void k_reach(const int32_t* __restrict__ col_front, const int32_t* __restrict__ parent,
                         const int32_t* __restrict__ src, int32_t K, int32_t nlevels, int32_t tiles,
                         uint8_t* __restrict__ reach) {
     const int k = blockIdx.x * blockDim.x + threadIdx.x;
@@ -622,7 +550,7 @@ __global__ void k_reach(const int32_t* __restrict__ col_sn, const int32_t* __res
     const int s0 = src[k];
     if (s0 < 0) return;
     const int t = k / kReachCols;
-    int s = col_sn[s0];
+    int s = col_front[s0];
     // the parent chain is strictly increasing and at most nlevels long
     for (int it = 0; s >= 0 && it <= nlevels; ++it) {
         reach[(int64_t)s * tiles + t] = 1;
@@ -630,79 +558,121 @@ __global__ void k_reach(const int32_t* __restrict__ col_sn, const int32_t* __res
     }
 }
 
-template <typename T, int KT, int TR>
-constexpr size_t fwd_smem(int stage = stage_rows<T, TR>()) {
-    return (size_t)(TR * ld_rows<T, KT>() + (separate_q<T>() ? 2 : 1) * TR * ld_fwd_a<T, TR>() + stage * KT) *
-           sizeof(T);
+template <typename T, int KT, int M, bool WIDE>
+constexpr size_t fwd_smem() {
+    return (size_t)(WIDE ? 3 : kNarrowCols / DC) * (panel_stage<T, M>() + DC * ld_rhs<T, KT>()) * sizeof(T);
 }
-template <typename T, int KT, int TR>
-constexpr size_t bwd_smem() {
-    return (size_t)2 * (RC * ld_bwd_a<T, TR>() + RC * ld_rows<T, KT>()) * sizeof(T);
+template <typename T, int KT, int M>
+size_t bwd_smem(int max_depth) {
+    return (size_t)3 * (panel_stage<T, M>() + DC * ld_rhs<T, KT>()) * sizeof(T) + (size_t)max_depth * sizeof(int32_t);
+}
+constexpr size_t kSmemMax = 227 * 1024 - 4096;  // static shared memory is kept apart
+
+// A launch that may start while the stream's previous kernel finishes; its reads of that kernel's
+// results come after griddepcontrol.wait.
+template <typename Kern, typename... Args>
+void launch_overlapped(Kern kern, dim3 grid, size_t smem, cudaStream_t st, Args... args) {
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = grid;
+    cfg.blockDim = dim3(NT);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = st;
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = at;
+    cfg.numAttrs = 1;
+    cudaLaunchKernelEx(&cfg, kern, args...);
 }
 
-// forward sweeps run 64-row tiles; backward sweeps 64- or 32-row tiles
-template <typename T, int KT>
+template <typename T, int KT, int M>
 cudaError_t set_smem() {
-    cudaError_t e = cudaFuncSetAttribute(k_fwd<T, KT, 64>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                         (int)fwd_smem<T, KT, 64>());
-    if (e != cudaSuccess) return e;
-    e = cudaFuncSetAttribute(k_bwd<T, KT, 64>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             (int)bwd_smem<T, KT, 64>());
-    if (e != cudaSuccess) return e;
-    return cudaFuncSetAttribute(k_bwd<T, KT, 32>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                (int)bwd_smem<T, KT, 32>());
+    cudaError_t e = cudaFuncSetAttribute(k_fwd<T, KT, M, true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                         (int)fwd_smem<T, KT, M, true>());
+    if constexpr (M == 128)
+        if (e == cudaSuccess)
+            e = cudaFuncSetAttribute(k_fwd<T, KT, M, false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                     (int)fwd_smem<T, KT, M, false>());
+    if constexpr (M <= 64)
+        if (e == cudaSuccess)
+            e = cudaFuncSetAttribute(k_bwd<T, KT, M>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmemMax);
+    return e;
+}
+template <typename T, int KT>
+cudaError_t set_smem_tiles() {
+    cudaError_t e;
+    if ((e = set_smem<T, KT, 128>())) return e;
+    if ((e = set_smem<T, KT, 64>())) return e;
+    return set_smem<T, KT, 32>();
 }
 
-template <typename T, int KT, int TR>
-void fwd_launch(const SolveArgs<T>& args, int32_t t0, int32_t ntasks, bool gathers, cudaStream_t st) {
-    SolveArgs<T> a = args;
-    a.stage = gathers ? stage_used<T, KT>() : 0;
-    k_fwd<T, KT, TR><<<dim3(ntasks, a.K / KT), NT, fwd_smem<T, KT, TR>(a.stage), st>>>(a, t0);
+template <typename T, int KT>
+void fwd_tile(const SweepArgs<T>& a, int32_t t0, int32_t n, int32_t rows, bool wide, cudaStream_t st) {
+    const dim3 grid(n, a.K / KT);
+    if (!wide) launch_overlapped(k_fwd<T, KT, 128, false>, grid, fwd_smem<T, KT, 128, false>(), st, a, t0);
+    else if (rows == 128) launch_overlapped(k_fwd<T, KT, 128, true>, grid, fwd_smem<T, KT, 128, true>(), st, a, t0);
+    else if (rows == 64) launch_overlapped(k_fwd<T, KT, 64, true>, grid, fwd_smem<T, KT, 64, true>(), st, a, t0);
+    else launch_overlapped(k_fwd<T, KT, 32, true>, grid, fwd_smem<T, KT, 32, true>(), st, a, t0);
 }
-template <typename T, int KT, int TR>
-void bwd_launch(const SolveArgs<T>& a, int32_t t0, int32_t ntasks, cudaStream_t st) {
-    k_bwd<T, KT, TR><<<dim3(ntasks, a.K / KT), NT, bwd_smem<T, KT, TR>(), st>>>(a, t0);
+template <typename T, int KT>
+void bwd_tile(const SweepArgs<T>& a, int32_t t0, int32_t n, int32_t rows, int32_t max_depth, cudaStream_t st) {
+    const dim3 grid(n, a.K / KT);
+    if (rows == 64) launch_overlapped(k_bwd<T, KT, 64>, grid, bwd_smem<T, KT, 64>(max_depth), st, a, t0);
+    else launch_overlapped(k_bwd<T, KT, 32>, grid, bwd_smem<T, KT, 32>(max_depth), st, a, t0);
+}
+template <typename T, int KT>
+void asm_tile(const SweepArgs<T>& a, int32_t r0, int32_t n, cudaStream_t st) {
+    constexpr int RPP = NT / (KT / vec<T>());
+    launch_overlapped(k_assemble<T, KT>, dim3((n + RPP - 1) / RPP, a.K / KT), 0, st, a, r0, n);
 }
 
 }  // namespace
 
 cudaError_t configure_solve_kernels() {
     cudaError_t e;
-    if ((e = set_smem<double, 64>())) return e;
-    if ((e = set_smem<float, 64>())) return e;
-    return set_smem<float, 128>();
+    if ((e = set_smem_tiles<double, 64>())) return e;
+    if ((e = set_smem_tiles<float, 64>())) return e;
+    return set_smem_tiles<float, 128>();
 }
+
+int32_t max_front_rows() { return (int32_t)((kSmemMax - bwd_smem<double, 64, 64>(0)) / sizeof(int32_t)); }
 
 template <typename T>
-void launch_fwd_level(const SolveArgs<T>& a, int32_t t0, int32_t ntasks, bool gathers, cudaStream_t st) {
+void launch_fwd_level(const SweepArgs<T>& a, int32_t t0, int32_t ntasks, int32_t rows, bool wide, cudaStream_t st) {
     if (ntasks <= 0 || a.K <= 0) return;
     constexpr int W = wide_tile<T>();
-    if (W != 64 && a.K % W == 0)
-        fwd_launch<T, W, 64>(a, t0, ntasks, gathers, st);
-    else
-        fwd_launch<T, 64, 64>(a, t0, ntasks, gathers, st);
+    if (W != 64 && a.K % W == 0) fwd_tile<T, W>(a, t0, ntasks, rows, wide, st);
+    else fwd_tile<T, 64>(a, t0, ntasks, rows, wide, st);
 }
-
 template <typename T>
-void launch_bwd_level(const SolveArgs<T>& a, int32_t t0, int32_t ntasks, int32_t tile_rows, cudaStream_t st) {
+void launch_assemble(const SweepArgs<T>& a, int32_t r0, int32_t nrows, cudaStream_t st) {
+    if (nrows <= 0 || a.K <= 0) return;
+    constexpr int W = wide_tile<T>();
+    if (W != 64 && a.K % W == 0) asm_tile<T, W>(a, r0, nrows, st);
+    else asm_tile<T, 64>(a, r0, nrows, st);
+}
+template <typename T>
+void launch_bwd_level(const SweepArgs<T>& a, int32_t t0, int32_t ntasks, int32_t rows, int32_t max_depth,
+                      cudaStream_t st) {
     if (ntasks <= 0 || a.K <= 0) return;
     constexpr int W = wide_tile<T>();
-    const bool wide = W != 64 && a.K % W == 0;
-    if (tile_rows == 32)
-        wide ? bwd_launch<T, W, 32>(a, t0, ntasks, st) : bwd_launch<T, 64, 32>(a, t0, ntasks, st);
-    else
-        wide ? bwd_launch<T, W, 64>(a, t0, ntasks, st) : bwd_launch<T, 64, 64>(a, t0, ntasks, st);
+    if (W != 64 && a.K % W == 0) bwd_tile<T, W>(a, t0, ntasks, rows, max_depth, st);
+    else bwd_tile<T, 64>(a, t0, ntasks, rows, max_depth, st);
 }
 
-void launch_reach(const DevPlan& p, const int32_t* src, int32_t K, uint8_t* reach, cudaStream_t st) {
+void launch_reach(const int32_t* col_front, const int32_t* parent, int32_t nfronts, int32_t nlevels,
+                  const int32_t* src, int32_t K, uint8_t* reach, cudaStream_t st) {
     const int32_t tiles = K / kReachCols;
-    cudaMemsetAsync(reach, 0, (size_t)p.nsuper * tiles, st);
-    k_reach<<<(K + 127) / 128, 128, 0, st>>>(p.col_sn, p.sn_parent, src, K, p.nlevels, tiles, reach);
+    cudaMemsetAsync(reach, 0, (size_t)nfronts * tiles, st);
+    k_reach<<<(K + 127) / 128, 128, 0, st>>>(col_front, parent, src, K, nlevels, tiles, reach);
 }
 
-template void launch_fwd_level<double>(const SolveArgs<double>&, int32_t, int32_t, bool, cudaStream_t);
-template void launch_fwd_level<float>(const SolveArgs<float>&, int32_t, int32_t, bool, cudaStream_t);
-template void launch_bwd_level<double>(const SolveArgs<double>&, int32_t, int32_t, int32_t, cudaStream_t);
-template void launch_bwd_level<float>(const SolveArgs<float>&, int32_t, int32_t, int32_t, cudaStream_t);
+#define FCW_SWEEPS(T)                                                                                           \
+    template void launch_fwd_level<T>(const SweepArgs<T>&, int32_t, int32_t, int32_t, bool, cudaStream_t);      \
+    template void launch_assemble<T>(const SweepArgs<T>&, int32_t, int32_t, cudaStream_t);                      \
+    template void launch_bwd_level<T>(const SweepArgs<T>&, int32_t, int32_t, int32_t, int32_t, cudaStream_t);
+FCW_SWEEPS(double)
+FCW_SWEEPS(float)
+#undef FCW_SWEEPS
 
 }  // namespace fcw

@@ -56,7 +56,7 @@ __device__ __forceinline__ uint32_t swz(int r, int c) {
 }
 
 // Own-row tile rows [0, nrows) -= the staged children's rows [e0, e1) that land on them.
-__device__ __forceinline__ void gather_sub_swz(unsigned char* Tt, const float* St, const unsigned char* live,
+__device__ __forceinline__ void gather_sub_swz(unsigned char* Tt, const float* St,
                                                const int* grs, int nrows, int e0, int e1) {
     constexpr int TPR = TCN / 4, RG = NT / TPR;
     const int c = 4 * (threadIdx.x % TPR);
@@ -66,7 +66,6 @@ __device__ __forceinline__ void gather_sub_swz(unsigned char* Tt, const float* S
         float4* d = reinterpret_cast<float4*>(Tt + swz(r, c));
         float4 v = *d;
         for (int e = lo; e < hi; ++e) {
-            if (!live[e - e0]) continue;
             const float4 u = *reinterpret_cast<const float4*>(St + (e - e0) * TCN + c);
             v.x -= u.x;
             v.y -= u.y;
@@ -79,18 +78,18 @@ __device__ __forceinline__ void gather_sub_swz(unsigned char* Tt, const float* S
 
 // gather_finish of solve.cu on the swizzled own-row tile (subtracting).
 __device__ __forceinline__ void gather_finish_swz(const SolveArgs<float>& a, const GatherRange& g, int k0,
-                                                  unsigned char* Tt, int nrows, float* St, unsigned char* live,
+                                                  unsigned char* Tt, int nrows, float* St,
                                                   const int* grs) {
     const int SG = a.stage;
     int e0 = 0;
     do {
         if (e0 > 0) {
-            gather_issue<float, TCN, TCM>(a, g, e0, k0, St, live);
+            gather_issue<float, TCN, TCM>(a, g, e0, k0, St);
             copy_async_commit();
         }
         copy_async_wait();
         __syncthreads();
-        if (g.E > 0) gather_sub_swz(Tt, St, live, grs, nrows, e0, min(g.E, e0 + SG));
+        if (g.E > 0) gather_sub_swz(Tt, St, grs, nrows, e0, min(g.E, e0 + SG));
         __syncthreads();
         e0 += SG;
     } while (e0 < g.E);
@@ -237,7 +236,6 @@ __global__ void __launch_bounds__(NT, 2) k_fwd_tc(SolveArgs<float> a, int32_t t0
     float* Blo = reinterpret_cast<float*>(sm + 2 * TC_FTILE + TC_TILE);
     float* St = reinterpret_cast<float*>(sm + 2 * TC_FTILE + 2 * TC_TILE);
     __shared__ int grs[TCF + 1];
-    __shared__ unsigned char live[TC_STAGE];
     __shared__ uint64_t bar_ld, bar_mma;
     __shared__ uint32_t tbase;
     __shared__ int bail;
@@ -290,11 +288,11 @@ __global__ void __launch_bounds__(NT, 2) k_fwd_tc(SolveArgs<float> a, int32_t t0
     }
     // the children's rows that land on this supernode's columns, while the TMA copies fly
     const GatherRange g1 = gather_open(a, fb, 0, ns, grs);
-    if (g1.E > 0) gather_issue<float, TCN, TCF>(a, g1, 0, k0, St, live);
+    if (g1.E > 0) gather_issue<float, TCN, TCF>(a, g1, 0, k0, St);
     copy_async_commit();
     bool ok = wait_all(&bar_ld, 0, &bail, a.err);
     if (ok) {
-        gather_finish_swz(a, g1, k0, Tt, ns, St, live, grs);  // W = R - children's rows
+        gather_finish_swz(a, g1, k0, Tt, ns, St, grs);  // W = R - children's rows
         split_own_rows(Tt, ns, Bhi, Blo);
         tc::fence_async_smem();
         __syncthreads();
@@ -308,7 +306,7 @@ __global__ void __launch_bounds__(NT, 2) k_fwd_tc(SolveArgs<float> a, int32_t t0
         GatherRange g2{0, 0};
         if (nq > 0) {
             g2 = gather_open(a, fb, ns + q0, nq, grs);
-            if (g2.E > 0) gather_issue<float, TCN, TCF>(a, g2, 0, k0, St, live);
+            if (g2.E > 0) gather_issue<float, TCN, TCF>(a, g2, 0, k0, St);
             copy_async_commit();
         }
         ok = wait_all(&bar_mma, 0, &bail, a.err);
@@ -329,7 +327,7 @@ __global__ void __launch_bounds__(NT, 2) k_fwd_tc(SolveArgs<float> a, int32_t t0
             const int u0 = xtask ? 64 : 0;  // output-tile row of the first update row
             if (xtask) tile_rows_to_global<float, TCN>(a.B + (int64_t)c0 * K + k0, K, Ot, TC_LS, ns);
             if (nq > 0) {
-                gather_finish<float, TCN, TCF, false>(a, g2, k0, Ot + u0 * TC_LS, TC_LS, nq, St, live, grs);
+                gather_finish<float, TCN, TCF, false>(a, g2, k0, Ot + u0 * TC_LS, TC_LS, nq, St, grs);
                 tile_rows_to_global<float, TCN>(a.U + (a.uoff[s] + q0) * (int64_t)K + k0, K, Ot + u0 * TC_LS,
                                                 TC_LS, nq);
             }
