@@ -71,28 +71,62 @@ __global__ void k_set_block(fcw::BlockDesc* d, const int32_t* sources, int64_t n
     d->out = out;
 }
 
-// k_map_sources with the block's sources from the descriptor.
-__global__ void k_map_block_sources(const fcw::BlockDesc* __restrict__ d, const int32_t* __restrict__ iperm,
-                                    int32_t nv, int32_t K, int32_t* __restrict__ out, int* __restrict__ err) {
-    const int k = blockIdx.x * blockDim.x + threadIdx.x;
-    if (k >= K) return;
-    int v = -1;
-    if (k < d->n) {
-        const int s = d->sources[k];
-        if (s >= 0 && s < nv) v = iperm[s];
-        else atomicOr(err, fcw::KERR_ARGS);
+// A block's sources (the descriptor's, or n of `raw`) in elimination order: src[c] = column c's
+// source, dst[c] = its place in the caller's list; -1 for padding and invalid sources, which come
+// last. The heat forward sweep solves, per 64-column tile, the fronts on its sources' paths to the
+// root: neighbours in this order share theirs. One CTA, a bitonic sort of (elimination index,
+// place) keys in shared memory, N = K rounded up to a power of two. 1024 sources in random order
+// at 147k vertices: heat forward 0.86 to 0.45 ms, heat backward 1.37 to 1.32 ms.
+constexpr int kSortThreads = 1024;
+constexpr int kMaxSort = 4096;  // block_k's largest
+__global__ void __launch_bounds__(kSortThreads) k_sort_sources(const fcw::BlockDesc* __restrict__ d,
+                                                               const int32_t* __restrict__ raw, int64_t n,
+                                                               const int32_t* __restrict__ iperm, int32_t nv,
+                                                               int32_t K, int32_t N, int32_t* __restrict__ src,
+                                                               int32_t* __restrict__ dst, int* __restrict__ err) {
+    extern __shared__ unsigned long long key[];
+    const int32_t* from = d ? d->sources : raw;
+    const int64_t count = d ? d->n : n;
+    for (int k = threadIdx.x; k < N; k += blockDim.x) {
+        unsigned long long x = ~0ull;
+        if (k < count) {
+            const int s = from[k];
+            if (s >= 0 && s < nv) x = ((unsigned long long)iperm[s] << 32) | (unsigned)k;
+            else atomicOr(err, fcw::KERR_ARGS);
+        }
+        key[k] = x;
     }
-    out[k] = v;
+    for (int size = 2; size <= N; size <<= 1)
+        for (int step = size >> 1; step > 0; step >>= 1) {
+            __syncthreads();
+            for (int i = threadIdx.x; i < N / 2; i += blockDim.x) {
+                const int a = 2 * i - (i & (step - 1)), b = a + step;
+                const bool up = (a & size) == 0;
+                const unsigned long long x = key[a], y = key[b];
+                if ((x > y) == up) {
+                    key[a] = y;
+                    key[b] = x;
+                }
+            }
+        }
+    __syncthreads();
+    for (int k = threadIdx.x; k < K; k += blockDim.x) {
+        const unsigned long long x = key[k];
+        src[k] = x == ~0ull ? -1 : (int32_t)(x >> 32);
+        dst[k] = x == ~0ull ? -1 : (int32_t)(x & 0xffffffffu);
+    }
 }
 
-// Rows [0, k) of dT (K x n, one field per source, elimination order) -> out (k x n, caller order).
+// Rows [0, k) of dT (K x n, one field per source, elimination order) -> out (k x n, caller order;
+// row r is the caller's source dst[r]).
 template <typename T>
 __global__ void k_fields_out(int32_t n, int32_t k, const T* __restrict__ dT, const int32_t* __restrict__ iperm,
-                             double* __restrict__ out) {
+                             const int32_t* __restrict__ dst, double* __restrict__ out) {
     const int64_t total = (int64_t)k * n;
     for (int64_t e = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; e < total; e += (int64_t)gridDim.x * blockDim.x) {
         const int r = (int)(e / n), i = (int)(e - (int64_t)r * n);
-        out[e] = (double)dT[(int64_t)r * n + iperm[i]];
+        const int o = dst[r];
+        if (o >= 0) out[(int64_t)o * n + i] = (double)dT[(int64_t)r * n + iperm[i]];
     }
 }
 
@@ -117,6 +151,7 @@ struct Workspace {
     double* dT64 = nullptr;
     float* dT32 = nullptr;
     int32_t* src = nullptr;
+    int32_t* dst = nullptr;     // each column's place in the caller's list
     uint8_t* reach = nullptr;
     int4* band = nullptr;
     int32_t* longf = nullptr;
@@ -865,7 +900,7 @@ int ensure_one(fcw_engine* e, Workspace& w, int32_t K, int32_t stride) {
     if (w.K >= K && w.out_stride >= stride) return FCW_OK;
     const int32_t Kn = std::max(K, w.K);
     const int32_t sn = std::max(stride, w.out_stride);
-    void* old[] = {w.Bh, w.Bp64, w.Y, w.dT64, w.src, w.reach, w.band, w.longf, w.out, w.U, w.W, w.part,
+    void* old[] = {w.Bh, w.Bp64, w.Y, w.dT64, w.src, w.dst, w.reach, w.band, w.longf, w.out, w.U, w.W, w.part,
                    w.counters, w.partials, w.near_list, w.near_count, w.desc, w.csum};
     for (void* p : old)
         if (p) e->release(p);
@@ -883,6 +918,7 @@ int ensure_one(fcw_engine* e, Workspace& w, int32_t K, int32_t stride) {
     FCW_TRY(e->dalloc(&w.dT64, (size_t)n * Kn));
     w.dT32 = reinterpret_cast<float*>(w.dT64);
     FCW_TRY(e->dalloc(&w.src, (size_t)Kn));
+    FCW_TRY(e->dalloc(&w.dst, (size_t)Kn));
     FCW_TRY(e->dalloc(&w.reach, (size_t)std::max<int64_t>(e->fr.nf, 1) * (Kn / fcw::kReachCols)));
     FCW_TRY(e->dalloc(&w.band, (size_t)nf * Kn));
     FCW_TRY(e->dalloc(&w.longf, (size_t)nf * Kn));
@@ -918,7 +954,7 @@ int ensure_workspace(fcw_engine* e, int32_t K, int32_t stride) {
         e->sync_streams();
         for (size_t j = i; j < e->pool.size(); ++j) {
             Workspace& w = e->pool[j];
-            void* bufs[] = {w.Bh, w.Bp64, w.Y, w.dT64, w.src, w.reach, w.band, w.longf, w.out, w.U, w.W, w.part,
+            void* bufs[] = {w.Bh, w.Bp64, w.Y, w.dT64, w.src, w.dst, w.reach, w.band, w.longf, w.out, w.U, w.W, w.part,
                             w.counters, w.partials, w.near_list, w.near_count, w.desc, w.csum};
             for (void* p : bufs)
                 if (p) e->release(p);
@@ -1150,18 +1186,23 @@ int check_engine(fcw_engine* e) {
     return FCW_OK;
 }
 
-int map_sources_host(fcw_engine* e, const int32_t* sources, int64_t n, int32_t K, cudaStream_t st,
-                     std::vector<int32_t>& buf) {
-    buf.assign(K, -1);
-    for (int64_t k = 0; k < n; ++k) {
-        const int32_t s = sources[k];
-        if (s < 0 || s >= e->sym.n)
-            return fail(FCW_E_INVALID, "source_idx out of range: " + std::to_string(s) + " for mesh with " +
+int check_sources(fcw_engine* e, const int32_t* sources, int64_t n) {
+    for (int64_t k = 0; k < n; ++k)
+        if (sources[k] < 0 || sources[k] >= e->sym.n)
+            return fail(FCW_E_INVALID, "source_idx out of range: " + std::to_string(sources[k]) + " for mesh with " +
                                            std::to_string(e->sym.n) + " vertices");
-        buf[k] = e->sym.iperm[s];
-    }
-    FCW_CUDA(cudaMemcpyAsync(e->cw().src, buf.data(), K * sizeof(int32_t), cudaMemcpyHostToDevice, st));
     return FCW_OK;
+}
+
+// w.src and w.dst from the block's descriptor, or from n sources at `raw` (device; may be w.src).
+void sort_sources(fcw_engine* e, Workspace& w, const fcw::BlockDesc* d, const int32_t* raw, int64_t n, int32_t K,
+                  cudaStream_t st) {
+    int32_t N = 2;
+    while (N < K) N <<= 1;
+    static_assert(kMaxSort * sizeof(unsigned long long) <= 48 * 1024, "the keys fit in default shared memory");
+    k_sort_sources<<<1, std::min(kSortThreads, N / 2), N * sizeof(unsigned long long), st>>>(
+        d, raw, n, e->iperm_d, (int32_t)e->sym.n, K, N, w.src, w.dst, e->err_d);
+    e->launches += 1;
 }
 
 int32_t round_k(int64_t k) { return (int32_t)(((k + fcw::kRhsTile - 1) / fcw::kRhsTile) * fcw::kRhsTile); }
@@ -1405,7 +1446,7 @@ int fcw_compute_distances(fcw_engine* e, const int32_t* sources, int64_t n, int3
     if (precision == FCW_PREC_MIXED && !e->pan_gf) return fail(FCW_E_INVALID, "engine was built without the mixed form");
     const int32_t Kmax = e->prm.block_k;
     const int64_t nv = e->sym.n;
-    std::vector<int32_t> buf;
+    FCW_TRY(check_sources(e, sources, n));
     for (int64_t b0 = 0; b0 < n; b0 += Kmax) {
         const int64_t nb = std::min<int64_t>(Kmax, n - b0);
         const int32_t K = round_k(nb);
@@ -1417,16 +1458,19 @@ int fcw_compute_distances(fcw_engine* e, const int32_t* sources, int64_t n, int3
             e->hcap_dist = nb * nv;
         }
         Workspace& w = e->cw();
-        FCW_TRY(map_sources_host(e, sources + b0, nb, K, w.stream, buf));
+        FCW_CUDA(cudaMemcpyAsync(w.src, sources + b0, (size_t)nb * sizeof(int32_t), cudaMemcpyHostToDevice, w.stream));
         // the chain (solves, divergence, shift, fields back to the caller's order) as one graph
         const std::vector<double> key = {(double)K, (double)precision, -1.0, (double)nb};
         FCW_TRY(run_chain(e, w, key, [&]() -> int {
+            sort_sources(e, w, nullptr, w.src, nb, K, w.stream);
             FCW_TRY(distances_block(e, K, precision, w.stream));
             const int grid = e->num_sms * 8;
             if (precision == FCW_PREC_MIXED)
-                k_fields_out<float><<<grid, 256, 0, w.stream>>>((int32_t)nv, (int32_t)nb, w.dT32, e->iperm_d, e->hdist_d);
+                k_fields_out<float><<<grid, 256, 0, w.stream>>>((int32_t)nv, (int32_t)nb, w.dT32, e->iperm_d, w.dst,
+                                                               e->hdist_d);
             else
-                k_fields_out<double><<<grid, 256, 0, w.stream>>>((int32_t)nv, (int32_t)nb, w.dT64, e->iperm_d, e->hdist_d);
+                k_fields_out<double><<<grid, 256, 0, w.stream>>>((int32_t)nv, (int32_t)nb, w.dT64, e->iperm_d, w.dst,
+                                                                e->hdist_d);
             e->launches += 1;
             return FCW_OK;
         }));
@@ -1642,9 +1686,7 @@ namespace {
 int block_chain(fcw_engine* e, Workspace& w, int32_t K, int32_t precision, fcw::MetricArgs& a,
                 const double* targets, int32_t nt, int32_t nb, double eps) {
     auto launch = [&]() -> int {
-        k_map_block_sources<<<(K + 127) / 128, 128, 0, w.stream>>>(w.desc, e->iperm_d, (int32_t)e->sym.n, K, w.src,
-                                                                   e->err_d);
-        e->launches += 1;
+        sort_sources(e, w, w.desc, nullptr, 0, K, w.stream);
         const int rc = distances_block(e, K, precision, w.stream, &a);
         if (rc != FCW_OK) return rc;
         if (precision == FCW_PREC_MIXED) metrics_block<float>(e, a, w.dT32, w.stream);
@@ -1689,6 +1731,7 @@ int fcw_compute_metrics_device(fcw_engine* e, const int32_t* sources_dev, int64_
         rc = metric_args(e, targets, nt, nb, eps, K, a);
         if (rc != FCW_OK) break;
         a.desc = w.desc;
+        a.dst = w.dst;
         k_set_block<<<1, 1, 0, w.stream>>>(w.desc, sources_dev + b0, nbk, out_dev + b0 * stride);
         e->launches += 1;
         rc = block_chain(e, w, K, precision, a, targets, nt, nb, eps);
@@ -1708,10 +1751,7 @@ int fcw_compute_metrics(fcw_engine* e, const int32_t* sources, int64_t n, int32_
     FCW_TRY(check_engine(e));
     if (n < 0 || (n > 0 && (!sources || !out_host))) return fail(FCW_E_INVALID, "NULL argument");
     if (n == 0) return FCW_OK;
-    for (int64_t k = 0; k < n; ++k)
-        if (sources[k] < 0 || sources[k] >= e->sym.n)
-            return fail(FCW_E_INVALID, "source_idx out of range: " + std::to_string(sources[k]) + " for mesh with " +
-                                           std::to_string(e->sym.n) + " vertices");
+    FCW_TRY(check_sources(e, sources, n));
     if (n == 1 && precision == FCW_PREC_FP64) return narrow_metrics(e, sources[0], targets, nt, nb, eps, out_host);
     const int32_t stride = fcw_metrics_stride(nt, nb);
     if (e->hcap_src < n) {

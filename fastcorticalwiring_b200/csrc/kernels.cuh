@@ -309,6 +309,7 @@ struct MetricArgs {
     double targets[kMaxTargets];
     double fracs[kMaxBetween];
     const int32_t* src = nullptr;       // elimination-order source per column
+    const int32_t* dst = nullptr;       // its record's place (null: the column's)
     int4* band = nullptr;               // nsrc * nf scratch: near faces (face, corners) sorted by sub-bin
     int32_t* longf = nullptr;           // nsrc * nf scratch: near long faces
     double* out = nullptr;              // nsrc * stride

@@ -13,7 +13,7 @@ import pytest
 pytestmark = pytest.mark.gpu
 
 import oracle  # noqa: E402
-from fastcorticalwiring_b200 import engine, mesh as M  # noqa: E402
+from fastcorticalwiring_b200 import _lib, engine, mesh as M  # noqa: E402
 from fastcorticalwiring_b200.meshgen import folded_icosphere  # noqa: E402
 
 
@@ -39,5 +39,47 @@ def test_fields_match_oracle(level, cap, jitter, params, count):
         for precision, tol in (("fp64", 1e-10), ("mixed", 1e-5)):
             d = eng.compute_distances(src, precision=precision)[sel]
             assert np.max(np.abs(d - ref)) <= tol * top, precision
+    finally:
+        eng.close()
+
+
+@pytest.mark.parametrize("block_k,count", [(64, 1), (320, 320), (320, 500), (128, 129)])
+def test_source_order_changes_nothing(block_k, count):
+    """Blocks are solved in elimination order: each source's results, repeated sources' too, are the
+    same wherever it stands in the list (fields bit for bit; records to the near lists' order of
+    summation, FP64)."""
+    g = folded_icosphere(4, seed=5, jitter=0.1, cap_fraction=0.2)
+    pm = M.prepare(g.vertices, g.faces, g.cortex_mask)
+    rng = np.random.default_rng(3)
+    src = rng.integers(0, pm.n_vertices, count).astype(np.int32)
+    src[count // 2] = src[0]
+    perm = rng.permutation(count)
+    eng = engine.HeatEngine(pm.V, pm.F, block_k=block_k, pipeline_depth=2)
+    try:
+        targets = pm.targets(M.RUNNER_SCALES)
+        for precision in ("fp64", "mixed"):
+            a = eng.compute_distances(src, precision=precision)
+            b = eng.compute_distances(src[perm], precision=precision)
+            assert np.array_equal(a[perm], b)
+            assert np.array_equal(a[count // 2], a[0])
+            if count == 1 and precision == "fp64":
+                continue  # one FP64 source takes a chain of its own
+            ra = eng.compute_metrics(src, targets, 2, precision=precision)
+            rb = eng.compute_metrics(src[perm], targets, 2, precision=precision)
+            np.testing.assert_allclose(ra[perm], rb, rtol=1e-12, equal_nan=True)
+    finally:
+        eng.close()
+
+
+def test_invalid_source_is_refused():
+    g = folded_icosphere(3, seed=1)
+    pm = M.prepare(g.vertices, g.faces, g.cortex_mask)
+    eng = engine.HeatEngine(pm.V, pm.F, block_k=64, pipeline_depth=1)
+    try:
+        for bad in (-1, pm.n_vertices):
+            with pytest.raises(_lib.FCWError) as e:
+                eng.compute_distances(np.array([0, bad, 1], np.int32))
+            assert e.value.code == _lib.FCW_E_INVALID
+        assert eng.compute_distances(np.array([1], np.int32))[0, 1] == 0.0
     finally:
         eng.close()
