@@ -9,6 +9,7 @@
 //   reach -> heat forward (delta RHS, pruned) -> heat backward -> divergence
 //   -> Poisson forward/backward -> shift + transpose -> vertex stats -> geometry
 // entirely on one stream.
+#include <algorithm>
 #include <chrono>
 #include <cmath>
 #include <cstring>
@@ -515,6 +516,7 @@ int build_engine(fcw_engine* e, const double* V, int64_t nv, const int32_t* F, i
     FCW_CUDA(cudaSetDevice(e->device));
     FCW_CUDA(cudaDeviceGetAttribute(&e->num_sms, cudaDevAttrMultiProcessorCount, e->device));
     FCW_CUDA(fcw::configure_kernels());
+    FCW_CUDA(fcw::configure_divergence_kernels());
     FCW_CUDA(fcw::configure_front_kernels());
     FCW_CUDA(fcw::configure_solve_kernels());
     FCW_CUDA(fcw::configure_tc_kernels());
@@ -692,15 +694,6 @@ int build_engine(fcw_engine* e, const double* V, int64_t nv, const int32_t* F, i
     std::vector<int32_t> fv(3 * nf), bnd(m.boundary.size());
     for (int64_t i = 0; i < 3 * nf; ++i) fv[i] = S.iperm[m.F[i]];
     for (size_t i = 0; i < m.boundary.size(); ++i) bnd[i] = S.iperm[m.boundary[i]];
-    std::vector<float> coef(4 * nf);
-    for (int64_t f = 0; f < nf; ++f) {
-        const double* g = &m.gb[9 * f];
-        const double c11 = g[3] * g[3] + g[4] * g[4] + g[5] * g[5];
-        const double c12 = g[3] * g[6] + g[4] * g[7] + g[5] * g[8];
-        const double c22 = g[6] * g[6] + g[7] * g[7] + g[8] * g[8];
-        coef[4 * f] = (float)c11; coef[4 * f + 1] = (float)c12; coef[4 * f + 2] = (float)c22;
-        coef[4 * f + 3] = (float)m.grad_area[f];
-    }
     std::vector<int32_t> inc_ptr(n + 1, 0), inc_face(3 * nf);
     std::vector<int8_t> inc_corner(3 * nf);
     for (int64_t i = 0; i < 3 * nf; ++i) inc_ptr[fv[i] + 1]++;
@@ -732,39 +725,55 @@ int build_engine(fcw_engine* e, const double* V, int64_t nv, const int32_t* F, i
     e->area_unscale = 1.0 / area_scale;
     FCW_TRY(e->upload(&e->inc_rec_d, inc_rec));
     FCW_TRY(e->upload(&e->farea_fx_d, farea_fx));
-    std::vector<int4> inc_corners(3 * nf);
-    std::vector<float4> inc_coef(3 * nf);
-    std::vector<float2> inc_w(3 * nf);
+    std::vector<int32_t> fan_ptr;
+    std::vector<fcw::FanStep> fan_steps;
+    fcw::face_fans(m, fv, inc_ptr, inc_face, inc_corner, fan_ptr, fan_steps);
+    // FP64 divergence: faces in the order of their lowest vertices, with their corners and geometry
+    std::vector<int32_t> place(nf), start(n + 1, 0);
+    std::vector<int4> corners(nf), div_rec(3 * nf);
+    std::vector<double> geo(8 * nf, 0.0);
+    if (nf > fcw::kIncFace) return fail(FCW_E_INVALID, "mesh has too many faces");
+    for (int64_t f = 0; f < nf; ++f) start[std::min({fv[3 * f], fv[3 * f + 1], fv[3 * f + 2]}) + 1]++;
+    for (int64_t j = 0; j < n; ++j) start[j + 1] += start[j];
+    for (int64_t f = 0; f < nf; ++f) {
+        const int32_t p = start[std::min({fv[3 * f], fv[3 * f + 1], fv[3 * f + 2]})]++;
+        place[f] = p;
+        corners[p] = make_int4(fv[3 * f], fv[3 * f + 1], fv[3 * f + 2], 0);
+        for (int x = 0; x < 6; ++x) geo[8 * (int64_t)p + x] = m.gb[9 * f + 3 + x];
+        geo[8 * (int64_t)p + 6] = m.grad_area[f];
+    }
     for (int64_t q = 0; q < 3 * nf; ++q) {
         const int32_t f = inc_face[q];
-        const float c11 = coef[4 * f], c12 = coef[4 * f + 1], c22 = coef[4 * f + 2];
-        inc_corners[q] = make_int4(fv[3 * f], fv[3 * f + 1], fv[3 * f + 2], inc_corner[q]);
-        inc_coef[q] = make_float4(c11, c12, c22, coef[4 * f + 3]);
-        // the corner weights in FP32, as the kernel's form defines them
-        if (inc_corner[q] == 0) inc_w[q] = make_float2(-(c11 + c12), -(c12 + c22));
-        else if (inc_corner[q] == 1) inc_w[q] = make_float2(c11, c12);
-        else inc_w[q] = make_float2(c12, c22);
+        div_rec[q] = make_int4(fv[3 * f], fv[3 * f + 1], fv[3 * f + 2],
+                               place[f] | ((int32_t)inc_corner[q] << fcw::kIncCornerShift));
     }
-    int4* inc_corners_d;
-    float4* inc_coef_d;
-    float2* inc_w_d;
-    FCW_TRY(e->upload(&inc_corners_d, inc_corners));
-    FCW_TRY(e->upload(&inc_coef_d, inc_coef));
-    FCW_TRY(e->upload(&inc_w_d, inc_w));
+    fcw::PatchArrays pa;
+    fcw::face_patches(fan_ptr, fan_steps, pa);
+    int4 *corners_d, *div_rec_d;
+    double* geo_d;
+    fcw::Patch* patches_d;
+    int32_t *big_d, *prow_d, *fan_ptr_d;
+    fcw::FanStep* fans_d;
+    FCW_TRY(e->upload(&corners_d, corners));
+    FCW_TRY(e->upload(&div_rec_d, div_rec));
+    FCW_TRY(e->upload(&geo_d, geo));
+    FCW_TRY(e->upload(&patches_d, pa.patches));
+    FCW_TRY(e->upload(&big_d, pa.big));
+    FCW_TRY(e->upload(&prow_d, pa.rows));
+    FCW_TRY(e->upload(&fan_ptr_d, fan_ptr));
+    FCW_TRY(e->upload(&fans_d, fan_steps));
     int32_t *fv_d, *inc_ptr_d, *inc_face_d;
     int8_t* inc_corner_d;
-    double *gb_d, *garea_d;
-    float* coef_d;
     FCW_TRY(e->upload(&fv_d, fv));
-    FCW_TRY(e->upload(&gb_d, m.gb));
-    FCW_TRY(e->upload(&garea_d, m.grad_area));
-    FCW_TRY(e->upload(&coef_d, coef));
     FCW_TRY(e->upload(&inc_ptr_d, inc_ptr));
     FCW_TRY(e->upload(&inc_face_d, inc_face));
     FCW_TRY(e->upload(&inc_corner_d, inc_corner));
-    e->fd.nv = (int32_t)n; e->fd.nf = (int32_t)nf; e->fd.fv = fv_d; e->fd.gb = gb_d; e->fd.garea = garea_d;
-    e->fd.coef = coef_d; e->fd.inc_ptr = inc_ptr_d; e->fd.inc_face = inc_face_d; e->fd.inc_corner = inc_corner_d;
-    e->fd.inc_corners = inc_corners_d; e->fd.inc_coef = inc_coef_d; e->fd.inc_w = inc_w_d;
+    e->fd.nv = (int32_t)n; e->fd.nf = (int32_t)nf; e->fd.fv = fv_d;
+    e->fd.inc_ptr = inc_ptr_d; e->fd.inc_face = inc_face_d; e->fd.inc_corner = inc_corner_d;
+    e->fd.corners = corners_d; e->fd.geo = geo_d; e->fd.inc_rec = div_rec_d;
+    e->fd.npatches = (int32_t)pa.patches.size(); e->fd.nbig = (int32_t)pa.big.size();
+    e->fd.patches = patches_d; e->fd.big = big_d; e->fd.patch_rows = prow_d; e->fd.fan_ptr = fan_ptr_d;
+    e->fd.fans = fans_d;
     FCW_TRY(e->upload(&e->coords_d, coords));
     FCW_TRY(e->upload(&e->varea_d, varea));
     FCW_TRY(e->upload(&e->boundary_d, bnd));
@@ -1098,7 +1107,8 @@ int distances_block(fcw_engine* e, int32_t K, int precision, cudaStream_t st, co
         if (ma) fcw::launch_shift_stats<float, float>(*ma, K, Y, w.dT32, st);
         else fcw::launch_shift_transpose<float, float>(n, K, Y, w.src, w.dT32, st);
     } else {
-        fcw::launch_divergence_fp64(e->fd, w.Bh, w.Bp64, K, st);
+        fcw::launch_divergence_fp64(e->fd, w.Bh, reinterpret_cast<double*>(w.band), w.Bp64, K, st);
+        e->launches += 1;
         FCW_TRY(poisson_solve<double>(e, e->pan_pf, e->pan_pb, w.Bp64, w.Y, K, st));
         mark(e, st, FCW_STAGE_SHIFT);
         if (ma) fcw::launch_shift_stats<double, double>(*ma, K, w.Y, w.dT64, st);
@@ -1909,7 +1919,7 @@ int fcw_divergence_device(fcw_engine* e, const double* u_dev, int32_t k, double*
     FCW_TRY(ensure_workspace(e, K, e->cw().out_stride));
     FCW_CUDA(cudaMemsetAsync(e->cw().Bh, 0, (size_t)e->sym.n * K * sizeof(double), st));
     fcw::launch_permute_rows((int32_t)e->sym.n, k, u_dev, k, nullptr, e->cw().Bh, K, e->iperm_d, st);
-    fcw::launch_divergence_fp64(e->fd, e->cw().Bh, e->cw().Bp64, K, st);
+    fcw::launch_divergence_fp64(e->fd, e->cw().Bh, reinterpret_cast<double*>(e->cw().band), e->cw().Bp64, K, st);
     fcw::launch_permute_rows((int32_t)e->sym.n, k, e->cw().Bp64, K, e->iperm_d, div_dev, k, nullptr, st);
     FCW_CUDA(cudaGetLastError());
     return FCW_OK;

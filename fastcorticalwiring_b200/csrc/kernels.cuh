@@ -8,6 +8,7 @@
 #include <vector>
 
 #include "fronts.h"
+#include "patches.h"
 
 namespace fcw {
 
@@ -249,23 +250,30 @@ void launch_component_level(const ComponentLevel& c, int32_t K, const int32_t* s
                             cudaStream_t st);
 
 // ---- fused gradient -> normalise -> divergence (face.cu) ----
+constexpr int kIncCornerShift = 30, kIncFace = (1 << kIncCornerShift) - 1;
 struct FaceData {
     int32_t nv = 0, nf = 0;
-    const int32_t* fv = nullptr;        // nf*3, elimination-order vertex ids
-    const double* gb = nullptr;         // nf*9 hat-function gradients (fastcw_lean.py:375-391)
-    const double* garea = nullptr;      // nf
-    const float* coef = nullptr;        // nf*4: c11, c12, c22, area (FP32 intrinsic form)
+    const int32_t* fv = nullptr;        // nf*3, elimination-order vertex ids (caller's face order)
     const int32_t* inc_ptr = nullptr;   // nv+1, per elimination-order vertex
     const int32_t* inc_face = nullptr;  // incident faces in ascending face order
     const int8_t* inc_corner = nullptr; // which corner of the face the vertex is
-    // the same incidences as records for the mixed form: the face's corners, its
-    // FP32 intrinsic coefficients (c11, c12, c22, area) and the vertex's corner
-    // weights (w1, w2), so a vertex reads its faces without an index chain
-    const int4* inc_corners = nullptr;
-    const float4* inc_coef = nullptr;
-    const float2* inc_w = nullptr;
+    // FP64 divergence: faces in the order of their lowest vertices, so neighbours are close
+    const int4* corners = nullptr;      // nf: the corners' vertices
+    const double* geo = nullptr;        // nf*8: gradients of corners 1 and 2 (fastcw_lean.py:375-391), area, -
+    const int4* inc_rec = nullptr;      // the incidences: corners' vertices, face place | corner << kIncCornerShift
+    // mixed form: patches of vertices, the vertices with more neighbours than a patch holds, and each
+    // vertex's faces as fans (patches.h; neighbours as patch rows, as vertices at the big ones)
+    int32_t npatches = 0, nbig = 0;
+    const Patch* patches = nullptr;
+    const int32_t* big = nullptr;
+    const int32_t* patch_rows = nullptr;  // the vertices of a patch's rows, its own first
+    const int32_t* fan_ptr = nullptr;     // nv+1
+    const FanStep* fans = nullptr;
 };
-void launch_divergence_fp64(const FaceData& fd, const double* u, double* div, int32_t K, cudaStream_t st);
+cudaError_t configure_divergence_kernels();
+// scale: nf * K doubles of scratch
+void launch_divergence_fp64(const FaceData& fd, const double* u, double* scale, double* div, int32_t K,
+                            cudaStream_t st);
 // One column (K = 1), the same arithmetic per vertex.
 void launch_divergence_fp64_one(const FaceData& fd, const double* u, double* div, cudaStream_t st);
 // grounded (elimination order): the ground vertices, whose divergence is zero

@@ -1,0 +1,129 @@
+// The divergence's view of the mesh (face.cu): each vertex's faces as fans, and patches of vertices.
+#include "patches.h"
+
+namespace fcw {
+
+// Each vertex's incident faces as fans for the mixed divergence (FaceData): walks from face to face
+// over the neighbour they share, first from the neighbours with one face (boundary ends), then around
+// the closed fans. A neighbour with more than two faces at the vertex (a non-manifold edge) ends fans.
+void face_fans(const MeshPrep& m, const std::vector<int32_t>& fv, const std::vector<int32_t>& inc_ptr,
+               const std::vector<int32_t>& inc_face, const std::vector<int8_t>& inc_corner,
+               std::vector<int32_t>& ptr, std::vector<FanStep>& steps) {
+    const int64_t n = (int64_t)inc_ptr.size() - 1;
+    ptr.assign(n + 1, 0);
+    steps.clear();
+    steps.reserve(inc_face.size() + n);
+    std::vector<int32_t> at(n, -1);                   // neighbour -> its slot at the current vertex
+    std::vector<int32_t> slot_face, slot_count, slot_of, done;  // two faces per slot; the faces' two slots
+    for (int64_t v = 0; v < n; ++v) {
+        const int32_t q0 = inc_ptr[v], deg = inc_ptr[v + 1] - q0;
+        slot_face.clear();
+        slot_count.clear();
+        slot_of.assign(2 * deg, 0);
+        done.assign(deg, 0);
+        auto other = [&](int32_t i, int k) {  // neighbour k (0, 1) of the vertex on its i-th face
+            return fv[3 * (int64_t)inc_face[q0 + i] + (inc_corner[q0 + i] + 1 + k) % 3];
+        };
+        for (int32_t i = 0; i < deg; ++i)
+            for (int k = 0; k < 2; ++k) {
+                int32_t& s = at[other(i, k)];
+                if (s < 0) {
+                    s = (int32_t)slot_count.size();
+                    slot_count.push_back(0);
+                    slot_face.insert(slot_face.end(), 2, -1);
+                }
+                if (slot_count[s] < 2) slot_face[2 * s + slot_count[s]] = i;
+                slot_count[s]++;
+                slot_of[2 * i + k] = s;
+            }
+        auto walk = [&](int32_t i, int k) {  // the fan that starts at neighbour k of face i
+            const size_t first = steps.size();
+            steps.push_back({{0.0f, 0.0f}, {0.0f, 0.0f}, {0.0f, 0.0f}, other(i, k), 0});
+            for (;;) {
+                done[i] = 1;
+                const double* g = &m.gb[9 * (int64_t)inc_face[q0 + i]];
+                const double* a = g + 3 * ((inc_corner[q0 + i] + 1 + k) % 3);
+                const double* b = g + 3 * ((inc_corner[q0 + i] + 2 - k) % 3);
+                auto dot = [](const double* x, const double* y) { return x[0] * y[0] + x[1] * y[1] + x[2] * y[2]; };
+                const double area = m.grad_area[inc_face[q0 + i]], aa = area * area;
+                const float c11 = (float)(aa * dot(a, a)), c12 = (float)(aa * dot(a, b)), c22 = (float)(aa * dot(b, b));
+                steps.push_back({{c11, c11}, {c12, c12}, {c22, c22}, other(i, 1 - k), -1});
+                steps[first].faces++;
+                const int32_t s = slot_of[2 * i + 1 - k];
+                if (slot_count[s] != 2) return;
+                const int32_t nxt = slot_face[2 * s] == i ? slot_face[2 * s + 1] : slot_face[2 * s];
+                if (done[nxt]) return;
+                k = slot_of[2 * nxt] == s ? 0 : 1;
+                i = nxt;
+            }
+        };
+        for (int32_t i = 0; i < deg; ++i)
+            for (int k = 0; k < 2; ++k)
+                if (!done[i] && slot_count[slot_of[2 * i + k]] != 2) walk(i, k);
+        for (int32_t i = 0; i < deg; ++i)
+            if (!done[i]) walk(i, 0);
+        for (int32_t i = 0; i < deg; ++i)
+            for (int k = 0; k < 2; ++k) at[other(i, k)] = -1;
+        ptr[v + 1] = (int32_t)steps.size();
+    }
+}
+
+// Consecutive vertices join a patch while its rows and fan steps fit. A vertex's rows are itself and
+// the neighbours its steps name.
+void face_patches(const std::vector<int32_t>& fan_ptr, std::vector<FanStep>& steps, PatchArrays& pa) {
+    const int32_t n = (int32_t)fan_ptr.size() - 1;
+    std::vector<int32_t> row_at(n, -1);  // place in the current patch (0 while it grows)
+    std::vector<int32_t> seen, fresh;    // the patch's rows; those the current vertex would add
+    int32_t v0 = 0;
+    auto close = [&](int32_t v1) {
+        if (v1 == v0) return;
+        Patch p{};
+        p.v0 = v0;
+        p.nv = v1 - v0;
+        p.row0 = (int32_t)pa.rows.size();
+        p.nsteps = fan_ptr[v1] - fan_ptr[v0];
+        for (int32_t v = v0; v < v1; ++v) {
+            row_at[v] = v - v0;
+            pa.rows.push_back(v);
+        }
+        p.nrows = p.nv;
+        for (int32_t v : seen)
+            if (v < v0 || v >= v1) {
+                row_at[v] = p.nrows++;
+                pa.rows.push_back(v);
+            }
+        for (int32_t q = fan_ptr[v0]; q < fan_ptr[v1]; ++q) steps[q].neighbour = row_at[steps[q].neighbour];
+        for (int32_t v : seen) row_at[v] = -1;
+        seen.clear();
+        pa.patches.push_back(p);
+        v0 = v1;
+    };
+    for (int32_t v = 0; v < n; ++v) {
+        for (;;) {
+            fresh.clear();
+            auto visit = [&](int32_t w) {
+                if (row_at[w] < 0) {
+                    row_at[w] = 0;
+                    fresh.push_back(w);
+                }
+            };
+            visit(v);
+            for (int32_t q = fan_ptr[v]; q < fan_ptr[v + 1]; ++q) visit(steps[q].neighbour);
+            if (v - v0 < kPatchVerts && (int32_t)(seen.size() + fresh.size()) <= kPatchRows &&
+                fan_ptr[v + 1] - fan_ptr[v0] <= kPatchSteps) {
+                seen.insert(seen.end(), fresh.begin(), fresh.end());
+                break;
+            }
+            for (int32_t w : fresh) row_at[w] = -1;
+            if (v == v0) {  // not even alone
+                pa.big.push_back(v);
+                v0 = v + 1;
+                break;
+            }
+            close(v);
+        }
+    }
+    close(n);
+}
+
+}  // namespace fcw

@@ -1,0 +1,41 @@
+// Host-side arrays of the divergence kernels (patches.cpp builds them, face.cu reads them).
+#pragma once
+
+#include <stdint.h>
+
+#include <vector>
+
+#include "fcw_internal.h"
+
+namespace fcw {
+
+// A patch: vertices [v0, v0 + nv) with their neighbours' rows and fan steps, as a CTA holds them in
+// shared memory (three CTAs per SM).
+constexpr int kPatchVerts = 64, kPatchRows = 108, kPatchSteps = 512;
+struct Patch {
+    int32_t v0, nv, row0, nrows, nsteps, pad;
+};
+
+// A step of a vertex's fan. The fan's first step names a neighbour and the faces that follow; each of
+// those steps names the next neighbour and holds the coefficients gb_a . gb_b, times the squared
+// area, of the face between it and the step before (a: that step's neighbour, b: this one), twice
+// each, as packed operands.
+struct FanStep {
+    float c11[2], c12[2], c22[2];
+    int32_t neighbour, faces;  // faces: of the fan, in its first step; -1 in the others
+};
+
+struct PatchArrays {
+    std::vector<Patch> patches;
+    std::vector<int32_t> big;   // vertices with more neighbours than a patch holds
+    std::vector<int32_t> rows;  // the vertices of a patch's rows, its own first
+};
+
+// fv: faces (elimination order), inc_*: each vertex's incident faces in ascending face order.
+void face_fans(const MeshPrep& m, const std::vector<int32_t>& fv, const std::vector<int32_t>& inc_ptr,
+               const std::vector<int32_t>& inc_face, const std::vector<int8_t>& inc_corner,
+               std::vector<int32_t>& ptr, std::vector<FanStep>& steps);
+// fv: faces (elimination order). Rewrites the steps' neighbours as patch rows (big vertices keep theirs).
+void face_patches(const std::vector<int32_t>& fan_ptr, std::vector<FanStep>& steps, PatchArrays& pa);
+
+}  // namespace fcw
