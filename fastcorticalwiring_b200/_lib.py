@@ -27,7 +27,7 @@ EXPORTED = (
     "fcw_heat_solve_device", "fcw_divergence_device", "fcw_poisson_solve_device", "fcw_field_metrics_device",
     "fcw_engine_profile", "fcw_engine_graphs", "fcw_engine_stage_times", "fcw_field_metrics_static",
     "fcw_samples_capacity", "fcw_assemble_samples_device", "fcw_assemble_samples", "fcw_tc_product_check",
-    "fcw_intrinsic_operators",
+    "fcw_intrinsic_operators", "fcw_compute_wiring", "fcw_pack_rows",
 )
 STAGES = ("heat_fwd", "heat_bwd", "divergence", "poisson_fwd", "poisson_bwd", "shift", "metrics")
 
@@ -113,6 +113,8 @@ def load():
         "fcw_samples_capacity": (ctypes.c_int, [I32, I32]),
         "fcw_assemble_samples_device": (ctypes.c_int, [P, I64, I32, I32, P, D, P, P, P, P]),
         "fcw_assemble_samples": (ctypes.c_int, [P, P, I64, I32, I32, P, D, P, P, P]),
+        "fcw_compute_wiring": (ctypes.c_int, [P, P, I64, I32, P, I32, I32, D, D, P, I64, P, P, P, P, P, P]),
+        "fcw_pack_rows": (ctypes.c_int, [P, I64, I64, P, P, P]),
         "fcw_tc_product_check": (ctypes.c_int, [P, P, P, I32, I32, I32, I32, I32, P, P, P]),
         "fcw_intrinsic_operators": (ctypes.c_int, [P, I64, P, I64, P, P, P, P, P, P, P, P, P]),
     }
@@ -176,6 +178,11 @@ def mesh_arrays(V, F):
     bf = np.empty(nv, dtype=np.uint8)
     check(load().fcw_mesh_arrays(ptr(V), nv, ptr(F), nf, ptr(va), ptr(la), ptr(g11), ptr(g12), ptr(g22), ptr(bf)))
     return dict(vertex_area=va, lean_area=la, g11=g11, g12=g12, g22=g22, boundary=np.flatnonzero(bf).astype(np.int32))
+
+
+def pack_rows(rows, counts, first, flat):
+    """flat[first[k]:first[k] + counts[k]] = rows[k, :counts[k]] (float32 rows, int32 counts, int64 first)."""
+    check(load().fcw_pack_rows(ptr(rows), rows.shape[0], rows.shape[1], ptr(counts), ptr(first), ptr(flat)))
 
 
 def intrinsic_operators(V, F):

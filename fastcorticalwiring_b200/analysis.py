@@ -19,6 +19,7 @@ import warnings
 
 import numpy as np
 
+from . import _lib
 from . import mesh as M
 from .engine import B200DistanceEngine
 
@@ -88,6 +89,19 @@ def check_interior_nonmanifold(pm, engine_type="b200", allow=False):
             RuntimeWarning,
         )
     return n
+
+
+def _plain_integers(values):
+    """values as an int64 array when it is a list, tuple or array of integers, else None."""
+    if isinstance(values, np.ndarray):
+        ok = values.ndim == 1 and values.dtype.kind == "i"
+        return values.astype(np.int64) if ok else None
+    if isinstance(values, (list, tuple)) and set(map(type, values)) <= {int}:
+        try:
+            return np.array(values, dtype=np.int64)
+        except OverflowError:
+            return None
+    return None
 
 
 class WiringAnalysis:
@@ -177,6 +191,12 @@ class WiringAnalysis:
         if vertex_subset is None:
             return order
         keep = np.zeros(self.mesh.n_vertices, dtype=bool)
+        ids = _plain_integers(vertex_subset)
+        if ids is not None:  # the loop below, all at once
+            ids = ids[(ids >= 0) & (ids < self.n_vertices_full)]
+            sub = self.orig_to_sub[ids[self.cortex_mask_full[ids]]]
+            keep[sub[sub >= 0]] = True
+            return order[keep[order]]
         for raw in vertex_subset:
             try:
                 o = int(raw)
@@ -208,8 +228,18 @@ class WiringAnalysis:
         for b0 in range(0, order.size, self.block_sources):
             tb = time.perf_counter()
             sub = order[b0:b0 + self.block_sources]
-            rec = eng.compute_metrics(sub, targets, n_between=m, eps=self.eps, precision=self.precision)
-            self._absorb(sub, rec, eng.assemble_samples(rec, targets, n_between=m, boundary_cap=cap))
+            # one FP64 source has its own, faster chain; other engines give records only
+            if not hasattr(eng, "compute_wiring") or (sub.size == 1 and self.precision in ("fp64", 0)):
+                rec = eng.compute_metrics(sub, targets, n_between=m, eps=self.eps, precision=self.precision)
+                self._absorb(sub, rec, eng.assemble_samples(rec, targets, n_between=m, boundary_cap=cap))
+            else:
+                orig = self.sub_to_orig[sub]
+                health, r, a, c = eng.compute_wiring(sub, targets, orig, self._maps, self.field_flag, n_between=m,
+                                                     eps=self.eps, precision=self.precision, boundary_cap=cap)
+                bad = self.field_flag[orig] != 0
+                self._flagged.extend(zip(orig[bad].tolist(), health[0, bad].tolist(), health[1, bad].tolist()))
+                self._counts[orig] = c
+                self._rows.append((r, a, orig))
             if verbose:
                 print(f"[{b0 + sub.size}/{order.size}] block of {sub.size} sources: "
                       f"{1e3 * (time.perf_counter() - tb):.2f}ms")
@@ -275,11 +305,11 @@ class WiringAnalysis:
         self.active_scales = scales
         self.n_samples_between_scales = m
         self.boundary_cap_fraction = cap
-        self.msd_unweighted = np.full(n, np.nan, dtype=np.float32)
-        self.msd_weighted = np.full(n, np.nan, dtype=np.float32)
-        self.dist_to_boundary = np.full(n, np.nan, dtype=np.float32)
-        self.radius_function = {float(s): np.full(n, np.nan, dtype=np.float32) for s in scales}
-        self.perimeter_function = {float(s): np.full(n, np.nan, dtype=np.float32) for s in scales}
+        k = len(scales)
+        self._maps = np.full((3 + 2 * k, n), np.nan, dtype=np.float32)  # the arrays below are its rows
+        self.msd_unweighted, self.msd_weighted, self.dist_to_boundary = self._maps[:3]
+        self.radius_function = {float(s): self._maps[3 + i] for i, s in enumerate(scales)}
+        self.perimeter_function = {float(s): self._maps[3 + k + i] for i, s in enumerate(scales)}
         self.field_flag = np.zeros(n, dtype=np.uint8)
         self._counts = np.zeros(n, dtype=np.int64)
         self._rows = []
@@ -316,13 +346,11 @@ class WiringAnalysis:
         self.sample_radii_flat = np.empty(total, dtype=np.float32)
         self.sample_areas_flat = np.empty(total, dtype=np.float32)
         for r, a, orig in self._rows:
-            c = counts[orig]
-            used = np.arange(r.shape[1])[None, :] < c[:, None]
-            dst = (self.sample_indptr[orig][:, None] + np.arange(r.shape[1])[None, :])[used]
-            self.sample_radii_flat[dst] = r[used]
-            self.sample_areas_flat[dst] = a[used]
+            c, first = counts[orig].astype(np.int32), self.sample_indptr[orig]
+            _lib.pack_rows(np.ascontiguousarray(r, np.float32), c, first, self.sample_radii_flat)
+            _lib.pack_rows(np.ascontiguousarray(a, np.float32), c, first, self.sample_areas_flat)
         flagged = self._flagged
-        self._counts, self._rows, self._flagged = None, None, None
+        self._counts, self._rows, self._flagged, self._maps = None, None, None, None
         self.n_flagged_fields = len(flagged)
         if flagged:
             msg = (f"{len(flagged)} of {n_sources} source vertices had corrupted distance fields; "

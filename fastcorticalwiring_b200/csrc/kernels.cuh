@@ -348,6 +348,9 @@ struct SampleArgs {
     int32_t* count_out = nullptr;     // n
 };
 void launch_assemble_samples(const SampleArgs& a, cudaStream_t st);
+// float32 maps (3 + 2 nt) x n, flags (n) and health fractions (2 x n) of n records
+void launch_pack_maps(const double* records, int64_t n, int32_t stride, int32_t nt, float* maps, uint8_t* flags,
+                      double* health, cudaStream_t st);
 // phi (n x K) -> dT (K x n) with phi[source] subtracted, plus per-tile health/MSD
 // partials and the per-source near-vertex lists.
 template <typename Tin, typename Tout>

@@ -108,7 +108,36 @@ __global__ void __launch_bounds__(32 * kWarps) k_assemble_samples(SampleArgs a) 
     if (lane == 0) a.count_out[k] = kept;
 }
 
+// The records' float32 maps, map i of source k at maps[i * n + k] (MSD unweighted and weighted,
+// boundary distance, radii, perimeters), its flag and health fractions (health[k], health[n + k]). A
+// warp reads one record's columns side by side and a CTA's 32 records are written back transposed.
+constexpr int kPackCols = 3 + 2 * kMaxTargets;
+__global__ void __launch_bounds__(256) k_pack_maps(const double* __restrict__ records, int64_t n, int32_t stride,
+                                                   int32_t nt, float* __restrict__ maps,
+                                                   uint8_t* __restrict__ flags, double* __restrict__ health) {
+    __shared__ float t[32][kPackCols + 1];
+    const int64_t k0 = blockIdx.x * (int64_t)32;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, cols = 3 + 2 * nt;
+    for (int r = warp; r < 32 && k0 + r < n; r += 8) {
+        const double* o = records + (k0 + r) * stride;
+        for (int c = lane; c < cols; c += 32) t[r][c] = (float)(c < 3 ? o[c] : o[4 + c]);  // radii from column 7
+        if (lane == 0) {
+            health[k0 + r] = o[3];
+            health[n + k0 + r] = o[4];
+            flags[k0 + r] = o[5] != 0.0;
+        }
+    }
+    __syncthreads();
+    if (k0 + lane < n)
+        for (int c = warp; c < cols; c += 8) maps[c * n + k0 + lane] = t[lane][c];
+}
+
 }  // namespace
+
+void launch_pack_maps(const double* records, int64_t n, int32_t stride, int32_t nt, float* maps, uint8_t* flags,
+                      double* health, cudaStream_t st) {
+    if (n > 0) k_pack_maps<<<(unsigned)((n + 31) / 32), 256, 0, st>>>(records, n, stride, nt, maps, flags, health);
+}
 
 void launch_assemble_samples(const SampleArgs& a, cudaStream_t st) {
     if (a.n <= 0) return;

@@ -160,6 +160,29 @@ class HeatEngine:
                                                     c, _lib.ptr(radii), _lib.ptr(areas), _lib.ptr(counts)))
         return radii, areas, counts
 
+    def compute_wiring(self, sources, targets, vertices, maps, flags, n_between=3, eps=1e-6, precision="mixed",
+                       boundary_cap=None):
+        """The analysis' float32 arrays of the sources, written into maps ((3 + 2 targets) x full
+        vertices) and flags (uint8) at `vertices`, with the flagged sources' maps left as they are.
+        Returns (health (2, n), radii, areas, counts), see include/fcw_b200.h."""
+        src = np.ascontiguousarray(sources, dtype=np.int32).reshape(-1)
+        v = np.ascontiguousarray(vertices, dtype=np.int32).reshape(-1)
+        t = np.ascontiguousarray(targets, dtype=np.float64).reshape(-1)
+        if v.size != src.size or maps.shape[0] != 3 + 2 * t.size or flags.size != maps.shape[1]:
+            raise ValueError("sources, vertices, maps and flags do not fit together")
+        if not (maps.dtype == np.float32 and maps.flags.c_contiguous and flags.dtype == np.uint8):
+            raise ValueError("maps must be a contiguous float32 array and flags uint8")
+        n, cap = src.size, _lib.samples_capacity(t.size, n_between)
+        health = np.empty((2, n))
+        radii, areas = np.empty((n, cap), np.float32), np.empty((n, cap), np.float32)
+        counts = np.empty(n, np.int32)
+        c = float("nan") if boundary_cap is None else float(boundary_cap)
+        _lib.check(_lib.load().fcw_compute_wiring(
+            self.handle, _lib.ptr(src), n, _precision(precision), _lib.ptr(t), t.size, int(n_between), float(eps), c,
+            _lib.ptr(v), maps.shape[1], _lib.ptr(maps), _lib.ptr(flags), _lib.ptr(health), _lib.ptr(radii),
+            _lib.ptr(areas), _lib.ptr(counts)))
+        return health, radii, areas, counts
+
     def graphs(self, enable=True) -> None:
         """Replay each workspace's captured launch chain (the default) or launch blocks directly."""
         _lib.check(_lib.load().fcw_engine_graphs(self.handle, int(bool(enable))))

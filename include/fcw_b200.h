@@ -197,6 +197,21 @@ int fcw_assemble_samples_device(const double* records_dev, int64_t n, int32_t n_
 int fcw_assemble_samples(fcw_engine* e, const double* records, int64_t n, int32_t n_targets, int32_t n_between,
                          const double* targets, double boundary_cap, float* radii, float* areas, int32_t* count);
 
+/* The analysis arrays of n sources (core_analysis.py:1550-1632), float32, over a full mesh of n_full
+ * vertices, source k being vertices[k] of it: map i (MSD unweighted, MSD weighted, distance to
+ * boundary, radii, perimeters: 3 + 2 nt of them) at maps[i * n_full + vertices[k]] and the health flag
+ * at flags[vertices[k]]; other entries, and the maps of flagged sources, keep what they held. health
+ * (2 x n) gets the negative and chord-violation fractions, radii, areas (n x fcw_samples_capacity) and
+ * counts the samples of fcw_assemble_samples. Host arrays; the records stay on the device. */
+int fcw_compute_wiring(fcw_engine* e, const int32_t* sources, int64_t n, int32_t precision, const double* targets,
+                       int32_t n_targets, int32_t n_between, double eps, double boundary_cap,
+                       const int32_t* vertices, int64_t n_full, float* maps, uint8_t* flags, double* health,
+                       float* radii, float* areas, int32_t* counts);
+/* Row k's first counts[k] entries (of n rows of `capacity`) to flat[first[k]]: the CSR values of the
+ * sample rows (core_analysis.py:1619-1632). Host only. */
+int fcw_pack_rows(const float* rows, int64_t n, int64_t capacity, const int32_t* counts, const int64_t* first,
+                  float* flat);
+
 /* CUDA graphs in fcw_compute_metrics(_device): enable (1, the default) / disable (0).
  * Each workspace captures its block's launch chain once per set of arguments (K,
  * precision, targets, n_between, eps) and replays it for later blocks; the block's
