@@ -261,7 +261,7 @@ struct fcw_engine {
     double *coords_d = nullptr, *varea_d = nullptr, *farea_d = nullptr, *g11_d = nullptr, *g12_d = nullptr,
            *g22_d = nullptr;
     int32_t* boundary_d = nullptr;
-    int4* inc_rec_d = nullptr;        // per incidence: face, corners (elimination order)
+    int32_t* fan_walk_d = nullptr;    // per fan step: neighbour, face
     long long* farea_fx_d = nullptr;  // lean face areas in fixed point
     double area_unscale = 0.0;
     int* err_d = nullptr;
@@ -280,6 +280,7 @@ struct fcw_engine {
     double* hdist_d = nullptr;  // staging for the host-buffer distances API (caller order)
     int64_t hcap_dist = 0;
     double analyze_ms = 0.0, factor_ms = 0.0;
+    double chord_slack = 0.0; // MetricArgs::chord_slack
     double lean_total = 0.0;  // sum of the lean face areas (the prefix total of a finite field)
     // stage timeline (CUDA events on the working stream), off unless enabled
     bool prof_on = false;
@@ -711,14 +712,8 @@ int build_engine(fcw_engine* e, const double* V, int64_t nv, const int32_t* F, i
                 fill[v]++;
             }
     }
-    // the same incidences as records holding the face's corners, and the face areas
-    // in a fixed point whose full scale is 2^62 >= the total, so that per-bin
+    // the face areas in a fixed point whose full scale is 2^62 >= the total, so that per-bin
     // sums are exact and independent of the order atomics add them in
-    std::vector<int4> inc_rec(3 * nf);
-    for (int64_t q = 0; q < 3 * nf; ++q) {
-        const int32_t f = inc_face[q];
-        inc_rec[q] = make_int4(f, fv[3 * f], fv[3 * f + 1], fv[3 * f + 2]);
-    }
     double lean_sum = 0.0;
     for (double x : m.lean_area) lean_sum += x;
     const int area_exp = lean_sum > 0.0 ? (int)std::ceil(std::log2(lean_sum)) : 0;
@@ -726,11 +721,11 @@ int build_engine(fcw_engine* e, const double* V, int64_t nv, const int32_t* F, i
     std::vector<long long> farea_fx(nf);
     for (int64_t f = 0; f < nf; ++f) farea_fx[f] = std::llround(m.lean_area[f] * area_scale);
     e->area_unscale = 1.0 / area_scale;
-    FCW_TRY(e->upload(&e->inc_rec_d, inc_rec));
     FCW_TRY(e->upload(&e->farea_fx_d, farea_fx));
     std::vector<int32_t> fan_ptr;
     std::vector<fcw::FanStep> fan_steps;
-    fcw::face_fans(m, fv, inc_ptr, inc_face, inc_corner, fan_ptr, fan_steps);
+    std::vector<int32_t> fan_walk;
+    fcw::face_fans(m, fv, inc_ptr, inc_face, inc_corner, fan_ptr, fan_steps, fan_walk);
     // FP64 divergence: faces in the order of their lowest vertices, with their corners and geometry
     std::vector<int32_t> place(nf), start(n + 1, 0);
     std::vector<int4> corners(nf), div_rec(3 * nf);
@@ -765,18 +760,22 @@ int build_engine(fcw_engine* e, const double* V, int64_t nv, const int32_t* F, i
     FCW_TRY(e->upload(&prow_d, pa.rows));
     FCW_TRY(e->upload(&fan_ptr_d, fan_ptr));
     FCW_TRY(e->upload(&fans_d, fan_steps));
-    int32_t *fv_d, *inc_ptr_d, *inc_face_d;
-    int8_t* inc_corner_d;
+    FCW_TRY(e->upload(&e->fan_walk_d, fan_walk));
+    int32_t *fv_d, *inc_ptr_d;
     FCW_TRY(e->upload(&fv_d, fv));
     FCW_TRY(e->upload(&inc_ptr_d, inc_ptr));
-    FCW_TRY(e->upload(&inc_face_d, inc_face));
-    FCW_TRY(e->upload(&inc_corner_d, inc_corner));
     e->fd.nv = (int32_t)n; e->fd.nf = (int32_t)nf; e->fd.fv = fv_d;
-    e->fd.inc_ptr = inc_ptr_d; e->fd.inc_face = inc_face_d; e->fd.inc_corner = inc_corner_d;
+    e->fd.inc_ptr = inc_ptr_d;
     e->fd.corners = corners_d; e->fd.geo = geo_d; e->fd.inc_rec = div_rec_d;
     e->fd.npatches = (int32_t)pa.patches.size(); e->fd.nbig = (int32_t)pa.big.size();
     e->fd.patches = patches_d; e->fd.big = big_d; e->fd.patch_rows = prow_d; e->fd.fan_ptr = fan_ptr_d;
     e->fd.fans = fans_d;
+    {
+        // two coordinates rounded to FP32 (2^-24 each) in three dimensions: 2.1e-7 of the largest
+        double top = 0.0;
+        for (double x : coords) top = std::max(top, std::fabs(x));
+        e->chord_slack = 4e-7 * top;
+    }
     FCW_TRY(e->upload(&e->coords_d, coords));
     FCW_TRY(e->upload(&e->varea_d, varea));
     FCW_TRY(e->upload(&e->boundary_d, bnd));
@@ -908,6 +907,17 @@ int build_engine(fcw_engine* e, const double* V, int64_t nv, const int32_t* F, i
     return FCW_OK;
 }
 
+// Statistics records that any block of at most K columns writes.
+int64_t stat_partials(int64_t n, int64_t K) {
+    int64_t most = 0;
+    for (int64_t k = 32; k <= K; k += 32) {
+        const int64_t t = fcw::stat_tile(n, k);
+        most = std::max(most, (n + t - 1) / t * k);
+    }
+    const int64_t one = fcw::stat_tile(n, 1);
+    return std::max(most, (n + one - 1) / one);
+}
+
 int ensure_one(fcw_engine* e, Workspace& w, int32_t K, int32_t stride) {
     if (w.K >= K && w.out_stride >= stride) return FCW_OK;
     const int32_t Kn = std::max(K, w.K);
@@ -935,8 +945,7 @@ int ensure_one(fcw_engine* e, Workspace& w, int32_t K, int32_t stride) {
     FCW_TRY(e->dalloc(&w.band, (size_t)nf * Kn));
     FCW_TRY(e->dalloc(&w.longf, (size_t)nf * Kn));
     FCW_TRY(e->dalloc(&w.out, (size_t)sn * Kn));
-    const int64_t ntiles = (n + fcw::kStatVTile - 1) / fcw::kStatVTile;
-    FCW_TRY(e->dalloc(&w.partials, (size_t)ntiles * Kn * 8));
+    FCW_TRY(e->dalloc(&w.partials, (size_t)stat_partials(n, Kn) * 8));
     FCW_TRY(e->dalloc(&w.near_list, (size_t)n * Kn));
     FCW_TRY(e->dalloc(&w.near_count, (size_t)Kn));
     const int64_t urows = e->prm.tc_sweeps ? std::max(e->fr.n_urows, e->n_urows) : e->fr.n_urows;
@@ -1140,10 +1149,8 @@ int metric_args(fcw_engine* e, const double* targets, int32_t nt, int32_t nb, do
     a.vertex_area = e->varea_d;
     a.boundary = e->boundary_d;
     a.fv = e->fd.fv;
-    a.inc_ptr = e->fd.inc_ptr;
-    a.inc_face = e->fd.inc_face;
-    a.inc_corner = e->fd.inc_corner;
-    a.inc_rec = e->inc_rec_d;
+    a.fan_ptr = e->fd.fan_ptr;
+    a.fan_walk = reinterpret_cast<const int2*>(e->fan_walk_d);
     a.farea_fx = e->farea_fx_d;
     a.area_unscale = e->area_unscale;
     a.total_area = e->lean_total;
@@ -1153,13 +1160,15 @@ int metric_args(fcw_engine* e, const double* targets, int32_t nt, int32_t nb, do
     a.g22 = e->g22_d;
     a.width = e->mesh.bin_width;
     a.health_h = e->mesh.health_h;
+    a.chord_slack = e->chord_slack;
     a.eps = eps;
     a.rtol = 1e-10;
     a.max_iter = 60;
     for (int32_t i = 0; i < nt; ++i) a.targets[i] = targets[i];
     for (int32_t j = 0; j < nb; ++j) a.fracs[j] = (double)(j + 1) / ((double)nb + 1.0);
     a.K = nsrc;
-    a.ntiles = (int32_t)((e->sym.n + fcw::kStatVTile - 1) / fcw::kStatVTile);
+    a.vtile = fcw::stat_tile(e->sym.n, nsrc);
+    a.ntiles = (int32_t)((e->sym.n + a.vtile - 1) / a.vtile);
     a.partials = e->cw().partials;
     a.near_list = e->cw().near_list;
     a.near_count = e->cw().near_count;
@@ -2151,6 +2160,8 @@ extern "C" int fcw_field_metrics_static(fcw_engine* e, const double* d_dev, cons
     cudaStream_t st = static_cast<cudaStream_t>(stream);
     fcw::MetricArgs a;
     FCW_TRY(metric_args(e, targets, nt, nb, eps, K, a));
+    a.vtile = fcw::kStatVTile;
+    a.ntiles = (int32_t)ntiles;
     a.src = src;
     a.band = band;
     a.longf = longf;

@@ -254,13 +254,11 @@ constexpr int kIncCornerShift = 30, kIncFace = (1 << kIncCornerShift) - 1;
 struct FaceData {
     int32_t nv = 0, nf = 0;
     const int32_t* fv = nullptr;        // nf*3, elimination-order vertex ids (caller's face order)
-    const int32_t* inc_ptr = nullptr;   // nv+1, per elimination-order vertex
-    const int32_t* inc_face = nullptr;  // incident faces in ascending face order
-    const int8_t* inc_corner = nullptr; // which corner of the face the vertex is
+    const int32_t* inc_ptr = nullptr;   // nv+1, per elimination-order vertex: its incident faces
     // FP64 divergence: faces in the order of their lowest vertices, so neighbours are close
     const int4* corners = nullptr;      // nf: the corners' vertices
     const double* geo = nullptr;        // nf*8: gradients of corners 1 and 2 (fastcw_lean.py:375-391), area, -
-    const int4* inc_rec = nullptr;      // the incidences: corners' vertices, face place | corner << kIncCornerShift
+    const int4* inc_rec = nullptr;      // in ascending face order: corners' vertices, place | corner << kIncCornerShift
     // mixed form: patches of vertices, the vertices with more neighbours than a patch holds, and each
     // vertex's faces as fans (patches.h; neighbours as patch rows, as vertices at the big ones)
     int32_t npatches = 0, nbig = 0;
@@ -301,10 +299,8 @@ struct MetricArgs {
     const double* vertex_area = nullptr;
     const int32_t* boundary = nullptr;  // elimination-order ids
     const int32_t* fv = nullptr;
-    const int32_t* inc_ptr = nullptr;   // vertex -> incident faces (elimination order)
-    const int32_t* inc_face = nullptr;
-    const int8_t* inc_corner = nullptr;
-    const int4* inc_rec = nullptr;      // per incidence (inc_face order): face, its three corners
+    const int32_t* fan_ptr = nullptr;   // vertex -> its fans' steps (patches.h, elimination order)
+    const int2* fan_walk = nullptr;     // per step: neighbour, the face it closes (-1: a fan's first)
     const long long* farea_fx = nullptr;  // lean face areas in fixed point (exact order-free sums)
     double area_unscale = 0.0;          // fixed point -> area
     double total_area = 0.0;            // sum of the lean face areas
@@ -313,6 +309,7 @@ struct MetricArgs {
     const double* g12 = nullptr;
     const double* g22 = nullptr;
     double width = 0.0, health_h = 0.0, eps = 1e-6, rtol = 1e-10;
+    double chord_slack = 0.0;           // bound on the error of a straight distance formed in FP32
     int32_t max_iter = 60;
     double targets[kMaxTargets];
     double fracs[kMaxBetween];
@@ -325,7 +322,7 @@ struct MetricArgs {
     int* err = nullptr;
     // shift + statistics (k_shift_stats) -> per-source kernel
     int32_t K = 0;                      // columns of the block (partials' leading dimension)
-    int32_t ntiles = 0;                 // vertex tiles of kStatVTile vertices
+    int32_t ntiles = 0, vtile = 0;      // vertex tiles of vtile vertices (stat_tile)
     double* partials = nullptr;         // ntiles x K x 8 partial statistics
     double near_radius = 0.0;           // = near_bins * width
     int32_t near_bins = 0;
@@ -333,7 +330,9 @@ struct MetricArgs {
     int32_t* near_list = nullptr;       // K x n: vertices closer than near_radius, per source
     int32_t* near_count = nullptr;      // K
 };
-constexpr int kStatVTile = 1024;   // vertices per shift-statistics CTA
+constexpr int kStatVTile = 1024;   // most vertices per shift-statistics CTA
+// Vertices per CTA for n vertices and K columns: fewer while the grid would leave the chip idle.
+int32_t stat_tile(int64_t n, int64_t K);
 
 // ---- per-source sample assembly (samples.cu) ----
 constexpr int kMaxSamples = kMaxTargets + (kMaxTargets - 1) * kMaxBetween;

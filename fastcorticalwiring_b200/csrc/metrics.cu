@@ -8,6 +8,8 @@
 // the source (see its comment for why that restriction is exact).
 #include <math.h>
 
+#include <algorithm>
+
 #include "kernels.cuh"
 
 namespace fcw {
@@ -43,12 +45,24 @@ __device__ __forceinline__ double dadd(double a, double b) { return __dadd_rn(a,
 // Per-(vertex tile, source) partial statistics written by k_shift_stats.
 enum { P_SUM_D, P_SUM_DA, P_SUM_A, P_CNT, P_NEG, P_VIOL, P_NONFINITE, P_DMAX, P_N };
 
+// Whether d < 0.9 |x - x_s| - h. The test compares squares and takes the reference's sqrt form only
+// within a 1e-10 band of the threshold, so it decides as the reference does.
+__device__ __forceinline__ bool chord_violation(double di, double vx, double vy, double vz, double sx, double sy,
+                                                double sz, double h) {
+    const double dx = vx - sx, dy = vy - sy, dz = vz - sz;
+    const double c2 = dadd(dadd(dmul(dx, dx), dmul(dy, dy)), dmul(dz, dz));
+    const double t = di + h;
+    if (t < 0.0) return true;
+    const double lhs = t * t, rhs = 0.81 * c2;
+    if (lhs < rhs * (1.0 - 1e-10)) return true;
+    if (lhs > rhs * (1.0 + 1e-10)) return false;
+    return di < __dsub_rn(dmul(0.9, __dsqrt_rn(c2)), h);
+}
+
 // One vertex's share of the health screen and MSD sums (lean_geometry.py:343-357,
 // core_analysis.py:1573-1581) for the distance di at a vertex (vx, vy, vz) of area va from
 // a source at (sx, sy, sz): counts of non-finite values, of d < -h and of d < 0.9 |x - x_s| - h,
-// the valid-distance sums and the maximum. The chord test compares squares and takes the
-// reference's sqrt form only within a 1e-10 band of the threshold, so the counts match the
-// reference exactly. Returns whether the vertex is nearer than R0.
+// the valid-distance sums and the maximum. Returns whether the vertex is nearer than R0.
 __device__ __forceinline__ bool vertex_stats(double di, double vx, double vy, double vz, double va, double sx,
                                              double sy, double sz, double h, double eps, double R0, double& sd,
                                              double& sda, double& sa, double& dm, int& cnt, int& ng, int& vi,
@@ -58,19 +72,7 @@ __device__ __forceinline__ bool vertex_stats(double di, double vx, double vy, do
         return false;
     }
     if (di < -h) ++ng;
-    const double dx = vx - sx, dy = vy - sy, dz = vz - sz;
-    const double c2 = dadd(dadd(dmul(dx, dx), dmul(dy, dy)), dmul(dz, dz));
-    const double t = di + h;
-    bool viol;
-    if (t < 0.0) {
-        viol = true;
-    } else {
-        const double lhs = t * t, rhs = 0.81 * c2;
-        if (lhs < rhs * (1.0 - 1e-10)) viol = true;
-        else if (lhs > rhs * (1.0 + 1e-10)) viol = false;
-        else viol = di < __dsub_rn(dmul(0.9, __dsqrt_rn(c2)), h);
-    }
-    if (viol) ++vi;
+    if (chord_violation(di, vx, vy, vz, sx, sy, sz, h)) ++vi;
     if (di > eps) {
         sd += di;
         sda += di * va;
@@ -81,78 +83,124 @@ __device__ __forceinline__ bool vertex_stats(double di, double vx, double vy, do
     return di < R0;
 }
 
+// The comparisons of vertex_stats for one field type, from thresholds rounded once: for a FP32 value
+// d, (double)d < x exactly when d < x rounded up to FP32, and (double)d > x when d > x rounded down.
+template <typename T>
+struct Thresholds {
+    T h, eps, R0;  // d < h: negative (h = -health_h); d > eps: valid; d < R0: near
+};
+template <typename T>
+__device__ __forceinline__ Thresholds<T> thresholds(const MetricArgs& a) {
+    if constexpr (sizeof(T) == 4)
+        return {__double2float_ru(-a.health_h), __double2float_rd(a.eps), __double2float_ru(a.near_radius)};
+    else
+        return {-a.health_h, a.eps, a.near_radius};
+}
+
 // The shift + transpose of one kStatVTile-vertex x 32-source tile, fused with the per-vertex
 // work of the health screen and MSD (lean_geometry.py:343-357, core_analysis.py:1573-1581):
 // counts of d < -h and of d < 0.9 |x - x_s| - h, the valid-distance sums and the maximum.
-// The chord test compares squares and takes the reference's sqrt form only within a
-// 1e-10 band of the threshold, so the counts match the reference exactly. Vertices
-// closer than the near radius are appended to their source's near list: per tile and
-// source, one atomic reserves the run, written in vertex order (which keeps the
-// per-source kernel's near-vertex walk local).
+// The chord test runs in FP32 first: with E = a.chord_slack bounding the error of the FP32 straight
+// distance and 0.1% for its other roundings, d + h - E > 0.901 |x - x_s| leaves no violation. That
+// decides nearly every value of a healthy field, which stays above the straight distance; the others
+// take the FP64 test, so the counts are the reference's. Sub-tiles arrive by
+// cp.async, two ahead. 147k vertices, 1024 columns: 0.92 to 0.69 ms (FP64 1.01 to 0.75), bound by issue;
+// four CTAs per SM (64 registers) spill and are slower. Vertices closer than the near radius
+// are appended to their source's near list: per tile and source, one atomic reserves the run, written
+// in vertex order (which keeps the per-source kernel's near-vertex walk local).
 template <typename Tin, typename Tout>
 __global__ void __launch_bounds__(256, 3) k_shift_stats(MetricArgs a, int32_t K, const Tin* __restrict__ phi,
                                                      Tout* __restrict__ dT) {
-    __shared__ Tin tile[32][33];
+    constexpr int S = 3;  // sub-tiles in flight
+    __shared__ Tin tiles[S][32][33];
     __shared__ Tin sh[32];
     __shared__ double sc[32][3];
+    __shared__ float4 scf[32];  // the source's position, FP32
     __shared__ int srcv[32];
     __shared__ unsigned nearmask[32][kStatVTile / 32];  // per source and sub-tile: lanes (vertices) near it
     const int n = a.n;
     const int k0 = blockIdx.y * 32;
     const int tx = threadIdx.x, ty = threadIdx.y;
-    const int vbase = blockIdx.x * kStatVTile;
+    const int vbase = blockIdx.x * a.vtile;
     for (int q = ty; q < kStatVTile / 32; q += 8) nearmask[tx][q] = 0u;
     if (ty == 0) {
         const int sidx = a.src[k0 + tx];
         srcv[tx] = sidx;
         sh[tx] = sidx >= 0 ? phi[(int64_t)sidx * K + k0 + tx] : Tin(0);
         for (int c = 0; c < 3; ++c) sc[tx][c] = sidx >= 0 ? a.coords[3 * (int64_t)sidx + c] : 0.0;
+        scf[tx] = make_float4((float)sc[tx][0], (float)sc[tx][1], (float)sc[tx][2], 0.0f);
     }
-    double sd[4], sda[4], sa[4], dm[4];
+    double sd[4], sda[4], sa[4];
+    Tout dm[4];
     int cnt[4], ng[4], vi[4], nf[4];
 #pragma unroll
-    for (int j = 0; j < 4; ++j) { sd[j] = sda[j] = sa[j] = 0.0; dm[j] = 0.0; cnt[j] = ng[j] = vi[j] = nf[j] = 0; }
-    const double h = a.health_h, R0 = a.near_radius;
+    for (int j = 0; j < 4; ++j) { sd[j] = sda[j] = sa[j] = 0.0; dm[j] = Tout(0); cnt[j] = ng[j] = vi[j] = nf[j] = 0; }
+    const Thresholds<Tout> th = thresholds<Tout>(a);
+    const float hf = (float)(a.health_h - a.chord_slack);
     const unsigned lanes_below = (1u << tx) - 1u;
-    // the field values of the next 32-vertex sub-tile are loaded while this one is processed
-    Tin nxt[4];
-#pragma unroll
-    for (int j = 0; j < 4; ++j) {
-        const int v = vbase + ty + 8 * j;
-        nxt[j] = v < n ? phi[(int64_t)v * K + k0 + tx] : Tin(0);
-    }
-    for (int sub = 0; sub < kStatVTile / 32; ++sub) {
-        const int v0 = vbase + sub * 32;
-        if (v0 >= n) break;
-        __syncthreads();  // the previous sub-tile's reads of `tile` are done
-#pragma unroll
-        for (int j = 0; j < 4; ++j) tile[ty + 8 * j][tx] = nxt[j];
-        if (sub + 1 < kStatVTile / 32) {
+    // the field values of the next sub-tiles are copied while this one is processed
+    const int nsub = min(a.vtile / 32, (n - vbase + 31) / 32);
+    auto request = [&](int sub) {
+        if (sub < nsub) {
 #pragma unroll
             for (int j = 0; j < 4; ++j) {
-                const int v = v0 + 32 + ty + 8 * j;
-                nxt[j] = v < n ? phi[(int64_t)v * K + k0 + tx] : Tin(0);
+                const int v = min(vbase + sub * 32 + ty + 8 * j, n - 1);
+                asm volatile("cp.async.ca.shared.global [%0], [%1], %2;\n" ::"r"(
+                                 (unsigned)__cvta_generic_to_shared(&tiles[sub % S][ty + 8 * j][tx])),
+                             "l"(phi + (int64_t)v * K + k0 + tx), "n"(sizeof(Tin))
+                             : "memory");
             }
         }
+        asm volatile("cp.async.commit_group;\n" ::: "memory");
+    };
+    for (int q = 0; q < S - 1; ++q) request(q);
+    for (int sub = 0; sub < nsub; ++sub) {
+        const int v0 = vbase + sub * 32;
+        Tin(*tile)[33] = tiles[sub % S];
         const int v = v0 + tx;
         const bool in = v < n;
-        double vx = 0.0, vy = 0.0, vz = 0.0, va = 0.0;
+        double va = 0.0;
+        float fx = 0.0f, fy = 0.0f, fz = 0.0f;
         if (in) {
-            vx = a.coords[3 * (int64_t)v];
-            vy = a.coords[3 * (int64_t)v + 1];
-            vz = a.coords[3 * (int64_t)v + 2];
+            fx = (float)a.coords[3 * (int64_t)v];
+            fy = (float)a.coords[3 * (int64_t)v + 1];
+            fz = (float)a.coords[3 * (int64_t)v + 2];
             va = a.vertex_area[v];
         }
-        __syncthreads();
+        asm volatile("cp.async.wait_group %0;\n" ::"n"(S - 2) : "memory");
+        __syncthreads();  // this sub-tile is in; every thread is done with the one before
+        request(sub + S - 1);
 #pragma unroll
         for (int j = 0; j < 4; ++j) {
             const int r = ty + 8 * j, k = k0 + r;
             const Tout dv = (Tout)(tile[tx][r] - sh[r]);
             if (in) dT[(int64_t)k * n + v] = dv;
             if (srcv[r] < 0) continue;  // warp-uniform (one source per warp)
-            const double di = (double)dv;
-            const bool near = in && vertex_stats(di, vx, vy, vz, va, sc[r][0], sc[r][1], sc[r][2], h, a.eps, R0,
-                                                 sd[j], sda[j], sa[j], dm[j], cnt[j], ng[j], vi[j], nf[j]);
+            bool near = false;
+            if (in) {
+                if (!isfinite(dv)) {
+                    ++nf[j];
+                } else {
+                    const float4 o = scf[r];
+                    const float dx = fx - o.x, dy = fy - o.y, dz = fz - o.z;
+                    const float t = (float)dv + hf, c2 = dx * dx + dy * dy + dz * dz;
+                    if (!(t > 0.0f && t * t > 0.8118f * c2 + 1e-30f)) {
+                        if (chord_violation((double)dv, a.coords[3 * (int64_t)v], a.coords[3 * (int64_t)v + 1],
+                                            a.coords[3 * (int64_t)v + 2], sc[r][0], sc[r][1], sc[r][2], a.health_h))
+                            ++vi[j];
+                    }
+                    if (dv < th.h) ++ng[j];
+                    if (dv > th.eps) {
+                        const double di = (double)dv;
+                        sd[j] += di;
+                        sda[j] += di * va;
+                        sa[j] += va;
+                        ++cnt[j];
+                    }
+                    dm[j] = dv > dm[j] ? dv : dm[j];
+                    near = dv < th.R0;
+                }
+            }
             const unsigned mask = __ballot_sync(0xffffffffu, near);
             if (tx == 0) nearmask[r][sub] = mask;
         }
@@ -164,7 +212,8 @@ __global__ void __launch_bounds__(256, 3) k_shift_stats(MetricArgs a, int32_t K,
             sd[j] += __shfl_down_sync(0xffffffffu, sd[j], off);
             sda[j] += __shfl_down_sync(0xffffffffu, sda[j], off);
             sa[j] += __shfl_down_sync(0xffffffffu, sa[j], off);
-            dm[j] = fmax(dm[j], __shfl_down_sync(0xffffffffu, dm[j], off));
+            const Tout o = __shfl_down_sync(0xffffffffu, dm[j], off);
+            dm[j] = o > dm[j] ? o : dm[j];
             cnt[j] += __shfl_down_sync(0xffffffffu, cnt[j], off);
             ng[j] += __shfl_down_sync(0xffffffffu, ng[j], off);
             vi[j] += __shfl_down_sync(0xffffffffu, vi[j], off);
@@ -174,7 +223,8 @@ __global__ void __launch_bounds__(256, 3) k_shift_stats(MetricArgs a, int32_t K,
             const int k = k0 + ty + 8 * j;
             double* q = a.partials + ((int64_t)blockIdx.x * K + k) * P_N;
             q[P_SUM_D] = sd[j]; q[P_SUM_DA] = sda[j]; q[P_SUM_A] = sa[j]; q[P_CNT] = (double)cnt[j];
-            q[P_NEG] = (double)ng[j]; q[P_VIOL] = (double)vi[j]; q[P_NONFINITE] = (double)nf[j]; q[P_DMAX] = dm[j];
+            q[P_NEG] = (double)ng[j]; q[P_VIOL] = (double)vi[j]; q[P_NONFINITE] = (double)nf[j];
+            q[P_DMAX] = (double)dm[j];
         }
     }
     // the tile's near vertices of each source, appended to its list with one atomic, in vertex order
@@ -195,8 +245,7 @@ __global__ void __launch_bounds__(256, 3) k_shift_stats(MetricArgs a, int32_t K,
         if (tx == 0) base = atomicAdd(&a.near_count[k], total);
         base = __shfl_sync(0xffffffffu, base, 0);
         const int excl = incl - c;
-#pragma unroll
-        for (int sb = 0; sb < NS; ++sb) {
+        for (int sb = 0; sb < nsub; ++sb) {
             const unsigned m = nearmask[r][sb];
             const int off = __shfl_sync(0xffffffffu, excl, sb);
             if (m & (1u << tx))
@@ -206,25 +255,27 @@ __global__ void __launch_bounds__(256, 3) k_shift_stats(MetricArgs a, int32_t K,
 }
 
 // One field (the single-source path): the same shift, statistics and near list for the one
-// column of phi (n, elimination order) into d. A CTA takes kStatVTile vertices, a warp 32
+// column of phi (n, elimination order) into d. A CTA takes a.vtile vertices, a warp 32
 // consecutive ones per step; the tile's near vertices are appended in vertex order with one
 // atomic, as k_shift_stats appends them.
 __global__ void __launch_bounds__(256) k_shift_stats_one(MetricArgs a, const double* __restrict__ phi,
                                                          double* __restrict__ d) {
-    constexpr int NG = kStatVTile / 32;  // 32-vertex groups of a tile
+    constexpr int NG = kStatVTile / 32;  // most 32-vertex groups of a tile
     static_assert(NG == 32, "one lane per group in the near-list scan");
     __shared__ unsigned gmask[NG];
     __shared__ int gbase[NG];
     __shared__ double wred[8][4];
     __shared__ int wcnt[8][4];
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    const int n = a.n, vbase = blockIdx.x * kStatVTile;
+    const int n = a.n, vbase = blockIdx.x * a.vtile, ngroups = a.vtile / 32;
+    if (tid < NG) gmask[tid] = 0u;
+    __syncthreads();
     const int se = a.src[0];
     const double p0 = phi[se];
     const double sx = a.coords[3 * (int64_t)se], sy = a.coords[3 * (int64_t)se + 1], sz = a.coords[3 * (int64_t)se + 2];
     double sd = 0.0, sda = 0.0, sa = 0.0, dm = 0.0;
     int cnt = 0, ng = 0, vi = 0, nf = 0;
-    for (int g = warp; g < NG; g += 8) {
+    for (int g = warp; g < ngroups; g += 8) {
         const int v = vbase + 32 * g + lane;
         bool near = false;
         if (v < n) {
@@ -279,7 +330,7 @@ __global__ void __launch_bounds__(256) k_shift_stats_one(MetricArgs a, const dou
     }
     __syncthreads();
     const unsigned below = (1u << lane) - 1u;
-    for (int g = warp; g < NG; g += 8) {
+    for (int g = warp; g < ngroups; g += 8) {
         const unsigned m = gmask[g];
         if (m & (1u << lane)) a.near_list[gbase[g] + __popc(m & below)] = vbase + 32 * g + lane;
     }
@@ -289,6 +340,8 @@ __global__ void __launch_bounds__(256) k_shift_stats_one(MetricArgs a, const dou
 // geometry
 // ---------------------------------------------------------------------------
 
+__device__ __forceinline__ void face_cdf_ordered(double lo, double mi, double hi, double A, double r, double& ar,
+                                                 double& da);
 // Area of {d <= r} in a linear face and its derivative (lean_geometry.py:66-88).
 __device__ __forceinline__ void face_cdf(double d0, double d1, double d2, double A, double r, double& ar,
                                          double& da) {
@@ -296,6 +349,10 @@ __device__ __forceinline__ void face_cdf(double d0, double d1, double d2, double
     if (lo > mi) { t = lo; lo = mi; mi = t; }
     if (mi > hi) { t = mi; mi = hi; hi = t; }
     if (lo > mi) { t = lo; lo = mi; mi = t; }
+    face_cdf_ordered(lo, mi, hi, A, r, ar, da);
+}
+__device__ __forceinline__ void face_cdf_ordered(double lo, double mi, double hi, double A, double r, double& ar,
+                                                 double& da) {
     // both partial cases in one branch-free form (one division): x = r - lo below the
     // middle corner, y = hi - r from it on
     const bool below = r < mi;
@@ -345,6 +402,7 @@ __device__ __forceinline__ double key_lo(int k) { return (double)__int_as_float(
 struct SrcShared {
     union {
         unsigned long long hist[kMaxBins + 1];  // face areas per sub-bin, fixed point (order-free sums)
+        uint2 histw[kMaxBins + 1];              // the same as 32-bit halves
         double pre[kMaxBins + 1];               // then the exclusive prefix sums of the sub-bins' areas
     };
     int ptr[kMaxBins + 1];     // faces per sub-bin -> exclusive prefix -> (counting sort) inclusive prefix
@@ -357,6 +415,21 @@ struct SrcShared {
     int sb;                    // sub-bins per bin
     int nstage;                // binned faces staged (unsorted) at the top of the band array
 };
+
+// A band record. FP32 fields: the face's corner distances in order and the face, (lo, mi, hi, f), so an
+// evaluation reads consecutive records and the face's area, and the sort needs no other load. FP64
+// distances do not fit in 16 bytes: (f, nearest corner, the other two). Forming areas and slopes
+// once per face too (56 bytes) halved an evaluation's instructions but took the bands of the sources in
+// flight from L2 to DRAM: 147k vertices, 1024 sources, 1.8 to 3.6 ms.
+template <typename T>
+constexpr bool ordered_band() { return sizeof(T) == 4; }
+template <typename T>
+__device__ __forceinline__ int4 band_record(T lo, T mi, T hi, int f, int v0, int v1, int v2) {
+    if constexpr (ordered_band<T>())
+        return make_int4(__float_as_int(lo), __float_as_int(mi), __float_as_int(hi), f);
+    else
+        return make_int4(f, v0, v1, v2);
+}
 
 // Sub-bins per bin for nbb complete bins: as many as the shared arrays hold.
 __device__ __forceinline__ int sub_bins(int nbb) {
@@ -379,7 +452,7 @@ struct Field {
     const T* d;
     const MetricArgs* a;
     SrcShared* s;
-    const int4* band;      // near faces (face, corners) sorted by sub-bin
+    const int4* band;      // near faces' records sorted by sub-bin
     const int32_t* longf;  // near faces whose distance extent exceeds the bin width
 
     __device__ double dv(int v) const { return (double)d[v]; }
@@ -402,17 +475,12 @@ struct Field {
         }
     }
 
-    // face_term of a band record (face, corners): no lookup of the face's corners
-    __device__ void rec_term(const int4& q, double d0, double d1, double d2, double r, int mode, double& x1,
-                             double& x2) const {
+    // the area and its derivative of a FP64 field's band record
+    __device__ void rec_term(const int4& q, double d0, double d1, double d2, double r, double& x1, double& x2) const {
         double ar, da;
         face_cdf(d0, d1, d2, a->farea[q.x], r, ar, da);
-        if (mode == 0) {
-            x1 += ar;
-            x2 += da;
-        } else if (da > 0.0) {
-            x1 += da * grad_norm(d0, d1, d2, a->g11[q.x], a->g12[q.x], a->g22[q.x]);
-        }
+        x1 += ar;
+        x2 += da;
     }
 
     // Faces with bin in [kr, kend) plus long faces with bin >= kend, summed by one warp;
@@ -436,6 +504,24 @@ struct Field {
             // sub-bin j's faces are band[ptr[j-1], ptr[j]) after the counting sort
             int j = (j0 > 0 ? s->ptr[j0 - 1] : 0) + lane;
             const int je = s->ptr[j1 - 1];
+            if (mode == 1) {  // |grad d| goes by the face's own corner order
+                for (; j < je; j += 32) face_term(ordered_band<T>() ? band[j].w : band[j].x, r, mode, x1, x2);
+            } else if (ordered_band<T>()) {
+                auto term = [&](const int4& q, double A) {
+                    double ar, da;
+                    face_cdf_ordered((double)__int_as_float(q.x), (double)__int_as_float(q.y),
+                                     (double)__int_as_float(q.z), A, r, ar, da);
+                    x1 += ar;
+                    x2 += da;
+                };
+                for (; j + 32 < je; j += 64) {  // two faces per lane in flight
+                    const int4 q0 = band[j], q1 = band[j + 32];
+                    const double A0 = a->farea[q0.w], A1 = a->farea[q1.w];
+                    term(q0, A0);
+                    term(q1, A1);
+                }
+                for (; j < je; j += 32) term(band[j], a->farea[band[j].w]);
+            }
             // two records per lane in flight
             for (; j + 32 < je; j += 64) {
                 int4 q[2];
@@ -449,11 +535,11 @@ struct Field {
                     dd[u][2] = dv(q[u].w);
                 }
 #pragma unroll
-                for (int u = 0; u < 2; ++u) rec_term(q[u], dd[u][0], dd[u][1], dd[u][2], r, mode, x1, x2);
+                for (int u = 0; u < 2; ++u) rec_term(q[u], dd[u][0], dd[u][1], dd[u][2], r, x1, x2);
             }
             for (; j < je; j += 32) {
                 const int4 q0 = band[j];
-                rec_term(q0, dv(q0.y), dv(q0.z), dv(q0.w), r, mode, x1, x2);
+                rec_term(q0, dv(q0.y), dv(q0.z), dv(q0.w), r, x1, x2);
             }
         } else {  // beyond the complete bins: scan every face (not reached for healthy fields)
             inside = prefix_at(kr);
@@ -546,12 +632,15 @@ struct Field {
 //   1. the health screen, MSD and global max from the shift kernel's partial sums,
 //      and the distance to boundary;
 //   2. the faces that have a corner closer than rc*w (rc starts at a first cut inside
-//      the radius of the shift kernel's near lists), each emitted once by its first
-//      near corner through the vertex->face incidence lists: their area histogram,
-//      counting sort by sub-bin and the long-face list (lean_geometry.py:117-180 on
-//      these faces). Bins below rc are complete. If the largest target is not enclosed
-//      two bins below rc, rc grows (to the near lists' radius, then up to every bin,
-//      scanning all vertices) and step 2 repeats;
+//      the radius of the shift kernel's near lists), each emitted once by its nearest
+//      corner through the vertices' fans and staged; their area histogram, counting sort
+//      by sub-bin and the long-face list (lean_geometry.py:117-180 on these faces), one
+//      pass over the staged records each. Bins below rc are complete. If the largest
+//      target is not enclosed two bins below rc, rc grows (to the near lists' radius,
+//      then up to every bin, scanning all vertices) and step 2 repeats;
+//      Walking every incidence of every near vertex twice (three gathers each, a
+//      64-bit shared atomic per face) took 60% of the kernel; 147k vertices, 1024
+//      sources: 1.79 to 1.38 ms (FP64 1.93 to 1.74), 9k: 0.26 to 0.21 ms;
 //   3. one warp per target: bracket + safeguarded Newton + perimeter; then the samples.
 template <typename T, int NT>
 __global__ void __launch_bounds__(NT, 1024 / NT) k_source_metrics(MetricArgs a, const T* __restrict__ dT) {
@@ -658,135 +747,168 @@ __global__ void __launch_bounds__(NT, 1024 / NT) k_source_metrics(MetricArgs a, 
         const bool listed = rc <= a.near_bins && rc < nbins;
         const int nv_scan = listed ? a.near_count[k] : a.n;
         const int32_t* nl = a.near_list + (int64_t)k * a.n;
-        for (int pass = 0; pass < 2; ++pass) {  // 0: histogram + long faces, 1: counting sort
-            // pass 0 also stages each binned face at the top of the band array; while the
-            // staged list and the sorted one (both ntot long) cannot overlap, pass 1 sorts
-            // the staged list instead of walking the incidences again
-            if (pass == 1 && 2 * S.ntot <= a.nf) {
-                const int ntot = S.ntot;
-                for (int p = tid; p < ntot; p += bs) {
-                    const int4 rq = band[a.nf - 1 - p];
-                    const double d0 = (double)d[rq.y], d1 = (double)d[rq.z], d2 = (double)d[rq.w];
-                    double hi = d0;  // as in pass 0
-                    if (d1 > hi) hi = d1;
-                    if (d2 > hi) hi = d2;
-                    const double q = hi / w;
-                    const int kb = q < 1.0 ? 0 : (int)q;
-                    band[atomicAdd(&S.ptr[kb * sb + sub_of(q, kb, sb)], 1)] = rq;
-                }
-                __syncthreads();
-                continue;
-            }
+        // Each face with a corner closer than R, once, from its nearest corner (the lowest vertex of
+        // equals): f(corner distances in order, the record of a sorted band). The vertices walk their
+        // fans, a thread each, so a neighbour's distance is loaded once for the two faces beside it; the
+        // next vertex's list entry and fan are loaded ahead.
+        auto walk = [&](auto&& f) {
+            auto open = [&](int ii, int& v, int& q0, int& q1) {
+                v = -1;
+                if (ii >= nv_scan) return;
+                v = listed ? nl[ii] : ii;
+                q0 = a.fan_ptr[v];
+                q1 = a.fan_ptr[v + 1];
+            };
+            int v, q0 = 0, q1 = 0;
+            open(tid, v, q0, q1);
             for (int ii = tid; ii < nv_scan; ii += bs) {
-                const int i = listed ? nl[ii] : ii;
-                const double di = (double)d[i];
-                if (!(di < R)) continue;
-                const int q1 = a.inc_ptr[i + 1];
-                constexpr int QB = sizeof(T) == 4 ? 4 : 2;
-                // the vertex's incidences in groups of QB: the records, then their corner
-                // distances, are loaded together before any is used
-                for (int qb = a.inc_ptr[i]; qb < q1; qb += QB) {
-                    int4 rec[QB];
-                    int cc[QB];
-                    T dd[QB][3];
-                    long long fx[QB];
+                int vn, qn0 = 0, qn1 = 0;
+                open(ii + bs, vn, qn0, qn1);
+                const T dv = d[v];
+                if ((double)dv < R) {
+                    int pv = -1;
+                    T pd = T(0);
+                    bool beyond = false;  // the previous neighbour is farther than the vertex
+                    for (int qb = q0; qb < q1; qb += 4) {
+                        int2 st[4];
+                        T dn[4];
 #pragma unroll
-                    for (int u = 0; u < QB; ++u)
-                        if (qb + u < q1) {
-                            rec[u] = a.inc_rec[qb + u];
-                            cc[u] = a.inc_corner[qb + u];
-                        }
+                        for (int u = 0; u < 4; ++u)
+                            if (qb + u < q1) st[u] = a.fan_walk[qb + u];
 #pragma unroll
-                    for (int u = 0; u < QB; ++u)
-                        if (qb + u < q1) {
-                            dd[u][0] = d[rec[u].y];
-                            dd[u][1] = d[rec[u].z];
-                            dd[u][2] = d[rec[u].w];
-                            if (pass == 0) fx[u] = a.farea_fx[rec[u].x];
-                        }
+                        for (int u = 0; u < 4; ++u)
+                            if (qb + u < q1) dn[u] = d[st[u].x];
 #pragma unroll
-                    for (int u = 0; u < QB; ++u) {
-                        if (qb + u >= q1) continue;
-                        const int f = rec[u].x;
-                        const int c = cc[u];
-                        const double d0 = (double)dd[u][0], d1 = (double)dd[u][1], d2 = (double)dd[u][2];
-                        if (c >= 1 && d0 < R) continue;   // an earlier corner emits it
-                        if (c == 2 && d1 < R) continue;
-                        // (every value is finite here: a field with a non-finite value is flagged above)
-                        double lo = d0, hi = d0;
-                        if (d1 < lo) lo = d1;
-                        if (d1 > hi) hi = d1;
-                        if (d2 < lo) lo = d2;
-                        if (d2 > hi) hi = d2;
-                        const double q = hi / w;  // F.bin_of's quotient
-                        const int kb = q < 1.0 ? 0 : (int)q;
-                        const int jb = kb * sb + sub_of(q, kb, sb);
-                        if (pass == 0) {
-                            if (hi - lo > w) longf[atomicAdd(&S.nlong, 1)] = f;
-                            if (kb < nbb) {
-                                atomicAdd(&S.hist[jb], (unsigned long long)fx[u]);
-                                atomicAdd(&S.ptr[jb], 1);
-                                atomicMin(&S.minlo[jb], lo_key(lo));
-                                band[a.nf - 1 - atomicAdd(&S.nstage, 1)] = rec[u];
+                        for (int u = 0; u < 4; ++u) {
+                            if (qb + u >= q1) continue;
+                            const bool far = dv < dn[u] || (dv == dn[u] && v < st[u].x);
+                            if (st[u].y >= 0 && far && beyond) {
+                                const T mi = pd < dn[u] ? pd : dn[u], hi = pd < dn[u] ? dn[u] : pd;
+                                f(dv, mi, hi, band_record(dv, mi, hi, st[u].y, v, pv, st[u].x));
                             }
-                        } else if (kb < nbb) {
-                            band[atomicAdd(&S.ptr[jb], 1)] = rec[u];  // ptr[jb] ends at the next sub-bin's start
+                            pv = st[u].x;
+                            pd = dn[u];
+                            beyond = far;
                         }
                     }
                 }
+                v = vn;
+                q0 = qn0;
+                q1 = qn1;
             }
-            __syncthreads();
-            if (pass == 0) {
-                // exclusive prefix sums over the sub-bins [0, nsub) by warp 0, exact in
-                // fixed point, each rounded once to an area
-                if (warp == 0) {
-                    const int chunk = (nsub + 31) / 32;
-                    const int b0 = min(lane * chunk, nsub), b1 = min(b0 + chunk, nsub);
-                    unsigned long long sa = 0ull;
-                    int sc = 0;
-                    for (int b = b0; b < b1; ++b) { sa += S.hist[b]; sc += S.ptr[b]; }
-                    unsigned long long ea = sa;
-                    int ec = sc;
-                    for (int off = 1; off < 32; off <<= 1) {
-                        const unsigned long long ta = __shfl_up_sync(0xffffffffu, ea, off);
-                        const int tc = __shfl_up_sync(0xffffffffu, ec, off);
-                        if (lane >= off) { ea += ta; ec += tc; }
-                    }
-                    unsigned long long ra = ea - sa;
-                    int rcn = ec - sc;
-                    for (int b = b0; b < b1; ++b) {
-                        const unsigned long long xa = S.hist[b];
-                        const int xc = S.ptr[b];
-                        S.pre[b] = (double)ra * a.area_unscale;
-                        S.ptr[b] = rcn;
-                        ra += xa;
-                        rcn += xc;
-                    }
-                    if (lane == 31) {
-                        S.ntot = ec;
-                        S.pre[nsub] = (double)ea * a.area_unscale;
-                        S.ptr[nsub] = ec;
-                    }
-                } else if (warp == 1) {
-                    // suffix minima of the sub-bins' lower bounds of lo
-                    const int chunk = (nsub + 31) / 32;
-                    const int b0 = min(lane * chunk, nsub), b1 = min(b0 + chunk, nsub);
-                    int mk = kInfKey;
-                    for (int b = b0; b < b1; ++b) mk = min(mk, S.minlo[b]);
-                    for (int off = 1; off < 32; off <<= 1) {
-                        const int t = __shfl_down_sync(0xffffffffu, mk, off);
-                        if (lane + off < 32) mk = min(mk, t);
-                    }
-                    int after = __shfl_down_sync(0xffffffffu, mk, 1);
-                    if (lane == 31) after = kInfKey;
-                    for (int b = b1 - 1; b >= b0; --b) {
-                        after = min(after, S.minlo[b]);
-                        S.minlo[b] = after;
-                    }
-                }
-                __syncthreads();
+        };
+        auto sub_bin = [&](double hi, int& kb) {
+            const double q = hi / w;  // F.bin_of's quotient
+            kb = q < 1.0 ? 0 : (int)q;
+            return kb * sb + sub_of(q, kb, sb);
+        };
+        // the near faces, staged at the top of the band array as they are found
+        walk([&](T, T, T, const int4& rec) {
+            const unsigned m = __activemask();
+            const int leader = __ffs(m) - 1;
+            int base = 0;
+            if (lane == leader) base = atomicAdd(&S.nstage, __popc(m));
+            base = __shfl_sync(m, base, leader) + __popc(m & ((1u << lane) - 1u));
+            band[a.nf - 1 - base] = rec;
+        });
+        __syncthreads();
+        const int nstage = S.nstage;
+        // histogram of the complete bins, long faces
+        auto distances = [&](const int4& rec, double& lo, double& hi) {
+            if constexpr (ordered_band<T>()) {
+                lo = (double)__int_as_float(rec.x);
+                hi = (double)__int_as_float(rec.z);
+            } else {  // the nearest corner is the first
+                lo = (double)d[rec.y];
+                hi = fmax((double)d[rec.z], (double)d[rec.w]);
+            }
+        };
+        for (int p = tid; p < nstage; p += bs) {
+            const int4 rec = band[a.nf - 1 - p];
+            const int f = ordered_band<T>() ? rec.w : rec.x;
+            double lo, hi;
+            distances(rec, lo, hi);
+            int kb;
+            const int jb = sub_bin(hi, kb);
+            if (hi - lo > w) longf[atomicAdd(&S.nlong, 1)] = f;
+            if (kb < nbb) {
+                const unsigned long long fx = (unsigned long long)a.farea_fx[f];
+                // two 32-bit adds (the carry from the returned value) in place of a 64-bit one, a
+                // compare-and-swap loop in shared memory
+                const unsigned lo32 = (unsigned)fx, old = atomicAdd(&S.histw[jb].x, lo32);
+                atomicAdd(&S.histw[jb].y, (unsigned)(fx >> 32) + (old + lo32 < old ? 1u : 0u));
+                atomicAdd(&S.ptr[jb], 1);
+                atomicMin(&S.minlo[jb], lo_key(lo));
             }
         }
+        __syncthreads();
+        // exclusive prefix sums over the sub-bins [0, nsub) by warp 0, exact in
+        // fixed point, each rounded once to an area
+        if (warp == 0) {
+            const int chunk = (nsub + 31) / 32;
+            const int b0 = min(lane * chunk, nsub), b1 = min(b0 + chunk, nsub);
+            unsigned long long sa = 0ull;
+            int sc = 0;
+            for (int b = b0; b < b1; ++b) { sa += S.hist[b]; sc += S.ptr[b]; }
+            unsigned long long ea = sa;
+            int ec = sc;
+            for (int off = 1; off < 32; off <<= 1) {
+                const unsigned long long ta = __shfl_up_sync(0xffffffffu, ea, off);
+                const int tc = __shfl_up_sync(0xffffffffu, ec, off);
+                if (lane >= off) { ea += ta; ec += tc; }
+            }
+            unsigned long long ra = ea - sa;
+            int rcn = ec - sc;
+            for (int b = b0; b < b1; ++b) {
+                const unsigned long long xa = S.hist[b];
+                const int xc = S.ptr[b];
+                S.pre[b] = (double)ra * a.area_unscale;
+                S.ptr[b] = rcn;
+                ra += xa;
+                rcn += xc;
+            }
+            if (lane == 31) {
+                S.ntot = ec;
+                S.pre[nsub] = (double)ea * a.area_unscale;
+                S.ptr[nsub] = ec;
+            }
+        } else if (warp == 1) {
+            // suffix minima of the sub-bins' lower bounds of lo
+            const int chunk = (nsub + 31) / 32;
+            const int b0 = min(lane * chunk, nsub), b1 = min(b0 + chunk, nsub);
+            int mk = kInfKey;
+            for (int b = b0; b < b1; ++b) mk = min(mk, S.minlo[b]);
+            for (int off = 1; off < 32; off <<= 1) {
+                const int t = __shfl_down_sync(0xffffffffu, mk, off);
+                if (lane + off < 32) mk = min(mk, t);
+            }
+            int after = __shfl_down_sync(0xffffffffu, mk, 1);
+            if (lane == 31) after = kInfKey;
+            for (int b = b1 - 1; b >= b0; --b) {
+                after = min(after, S.minlo[b]);
+                S.minlo[b] = after;
+            }
+        }
+        __syncthreads();
+        // counting sort of the complete bins' faces: from the staged list while the two lists cannot
+        // overlap, else by another walk
+        if (nstage + S.ntot <= a.nf) {
+            for (int p = tid; p < nstage; p += bs) {
+                const int4 rec = band[a.nf - 1 - p];
+                double lo, hi;
+                distances(rec, lo, hi);
+                int kb;
+                const int jb = sub_bin(hi, kb);
+                if (kb < nbb) band[atomicAdd(&S.ptr[jb], 1)] = rec;  // ptr[jb] ends at the next sub-bin's start
+            }
+        } else {
+            walk([&](T, T, T hi, const int4& rec) {
+                int kb;
+                const int jb = sub_bin((double)hi, kb);
+                if (kb < nbb) band[atomicAdd(&S.ptr[jb], 1)] = rec;
+            });
+        }
+        __syncthreads();
         // enough? the largest target must be enclosed two bins below the cut
         bool ok = rc >= nbins || (rc >= 2 && S.pre[(rc - 2) * sb] >= tmax);
         if (ok) break;
@@ -801,7 +923,9 @@ __global__ void __launch_bounds__(NT, 1024 / NT) k_source_metrics(MetricArgs a, 
     __syncthreads();
 
     // 3. radii + perimeters, one warp per target (lean_geometry.py:315-324)
-    for (int t = warp; t < nt; t += nwarps) {
+    // (the largest targets, with the most faces near them, first: the short ones fill the last round)
+    for (int i = warp; i < nt; i += nwarps) {
+        const int t = nt - 1 - i;
         int ev = 0;
         const double r = F.solve_radius(a.targets[t], ev);
         double p = nan;
@@ -848,6 +972,16 @@ __global__ void k_permute_rows(int32_t n, int32_t cols, const double* __restrict
 
 }  // namespace
 
+// At least two waves of three CTAs per SM: a CTA walks its vertices 32 at a time, about 1.5 us a step,
+// so on few columns or small meshes the walk, not the chip, sets the time. 9k vertices, 64 columns:
+// 68 to 18 us; 1024 columns 94 to 70.
+int32_t stat_tile(int64_t n, int64_t K) {
+    const int64_t slices = std::max<int64_t>(1, K / 32);
+    for (int32_t t = kStatVTile; t > 128; t /= 2)
+        if ((n + t - 1) / t * slices >= 888) return t;
+    return 128;
+}
+
 template <typename Tin, typename Tout>
 void launch_shift_transpose(int32_t n, int32_t K, const Tin* phi, const int32_t* src, Tout* dT, cudaStream_t st) {
     if (n <= 0 || K <= 0) return;
@@ -879,9 +1013,10 @@ void launch_shift_stats_one(const MetricArgs& a, const double* phi, double* d, c
 template <typename T>
 void launch_source_metrics(const MetricArgs& a, const T* dT, cudaStream_t st) {
     if (a.nsrc <= 0) return;
-    // a lone source (the single-source path) gets a CTA of 1024 threads: its binning, sort and
-    // targets spread over 32 warps instead of waiting on one CTA's 8
-    if (a.nsrc == 1) k_source_metrics<T, 1024><<<1, 1024, 0, st>>>(a, dT);
+    // While there is an SM for each source, its binning, sort and targets spread over 32 warps instead of
+    // waiting on 8 (64 sources at 147k vertices: 0.82 to 0.25 ms); then over 16 while two share an SM.
+    if (a.nsrc <= 148) k_source_metrics<T, 1024><<<a.nsrc, 1024, 0, st>>>(a, dT);
+    else if (a.nsrc <= 296) k_source_metrics<T, 512><<<a.nsrc, 512, 0, st>>>(a, dT);
     else k_source_metrics<T, kMetricThreads><<<a.nsrc, kMetricThreads, 0, st>>>(a, dT);
 }
 

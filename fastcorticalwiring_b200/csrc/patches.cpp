@@ -8,11 +8,13 @@ namespace fcw {
 // the closed fans. A neighbour with more than two faces at the vertex (a non-manifold edge) ends fans.
 void face_fans(const MeshPrep& m, const std::vector<int32_t>& fv, const std::vector<int32_t>& inc_ptr,
                const std::vector<int32_t>& inc_face, const std::vector<int8_t>& inc_corner,
-               std::vector<int32_t>& ptr, std::vector<FanStep>& steps) {
+               std::vector<int32_t>& ptr, std::vector<FanStep>& steps, std::vector<int32_t>& walked) {
     const int64_t n = (int64_t)inc_ptr.size() - 1;
     ptr.assign(n + 1, 0);
     steps.clear();
     steps.reserve(inc_face.size() + n);
+    walked.clear();
+    walked.reserve(2 * (inc_face.size() + n));
     std::vector<int32_t> at(n, -1);                   // neighbour -> its slot at the current vertex
     std::vector<int32_t> slot_face, slot_count, slot_of, done;  // two faces per slot; the faces' two slots
     for (int64_t v = 0; v < n; ++v) {
@@ -39,6 +41,7 @@ void face_fans(const MeshPrep& m, const std::vector<int32_t>& fv, const std::vec
         auto walk = [&](int32_t i, int k) {  // the fan that starts at neighbour k of face i
             const size_t first = steps.size();
             steps.push_back({{0.0f, 0.0f}, {0.0f, 0.0f}, {0.0f, 0.0f}, other(i, k), 0});
+            walked.insert(walked.end(), {other(i, k), -1});
             for (;;) {
                 done[i] = 1;
                 const double* g = &m.gb[9 * (int64_t)inc_face[q0 + i]];
@@ -49,6 +52,7 @@ void face_fans(const MeshPrep& m, const std::vector<int32_t>& fv, const std::vec
                 const float c11 = (float)(aa * dot(a, a)), c12 = (float)(aa * dot(a, b)), c22 = (float)(aa * dot(b, b));
                 steps.push_back({{c11, c11}, {c12, c12}, {c22, c22}, other(i, 1 - k), -1});
                 steps[first].faces++;
+                walked.insert(walked.end(), {other(i, 1 - k), inc_face[q0 + i]});
                 const int32_t s = slot_of[2 * i + 1 - k];
                 if (slot_count[s] != 2) return;
                 const int32_t nxt = slot_face[2 * s] == i ? slot_face[2 * s + 1] : slot_face[2 * s];

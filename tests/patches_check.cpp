@@ -41,7 +41,9 @@ static int check(const char* path) {
         }
     std::vector<int32_t> fan_ptr;
     std::vector<FanStep> steps;
-    face_fans(m, F, ptr, face, corner, fan_ptr, steps);
+    std::vector<int32_t> walk;
+    face_fans(m, F, ptr, face, corner, fan_ptr, steps, walk);
+    CHECK(walk.size() == 2 * steps.size());
     // each face once per corner, as the pair of neighbours of two consecutive steps
     for (int64_t v = 0; v < nv; ++v) {
         std::multiset<std::pair<int, int>> want, got;
@@ -53,11 +55,14 @@ static int check(const char* path) {
         for (int e = fan_ptr[v]; e < fan_ptr[v + 1]; ++e) {
             if (left == 0) {  // a fan's first step
                 left = steps[e].faces;
+                CHECK(walk[2 * e] == steps[e].neighbour && walk[2 * e + 1] == -1);
                 CHECK(left > 0);
                 continue;
             }
             --left;
-            CHECK(steps[e].faces == -1);
+            CHECK(steps[e].faces == -1 && walk[2 * e] == steps[e].neighbour);
+            const int32_t* w = &F[3 * (size_t)walk[2 * e + 1]];
+            CHECK(std::set<int>({w[0], w[1], w[2]}) == std::set<int>({(int)v, steps[e - 1].neighbour, steps[e].neighbour}));
             const int p = steps[e - 1].neighbour;
             got.insert({std::min(p, steps[e].neighbour), std::max(p, steps[e].neighbour)});
             // the coefficients are the two neighbours' hat gradients' products times the squared area
