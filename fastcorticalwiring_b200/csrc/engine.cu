@@ -190,20 +190,19 @@ struct Workspace {
 struct NarrowState {
     bool ready = false;
     fcw::NarrowLaunch L;
-    int64_t* at_ptr = nullptr;
     double *at_h = nullptr, *at_p = nullptr;    // forward layouts of the heat and Poisson factors
     double *atb_h = nullptr, *atb_p = nullptr;  // backward layouts
-    int4 *ftasks = nullptr, *btasks = nullptr;
+    fcw::NarrowTask *ftasks = nullptr, *btasks = nullptr;
     int32_t n_ftasks = 0, n_btasks = 0;
     double *u = nullptr, *div = nullptr, *y = nullptr, *out = nullptr;
     double* pend = nullptr;       // entries a sweep's readers poll: heat and Poisson update entries, heat
                                   // and Poisson solutions (set pending at the start of each call)
     int* sync = nullptr;          // the four sweeps' ticket counters
     // the heat forward's work list, built on the host per call: the source's elimination
-    // index, the path's task count, then (task, previous supernode on the path) pairs
+    // index, the path's task count, then (task, previous front on the path) pairs
     int32_t* order = nullptr;
     int32_t* horder = nullptr;    // pinned host staging of the list
-    std::vector<int32_t> fwd_first, nfwd_h;  // per supernode: first forward task, count
+    std::vector<int32_t> fwd_first, nfwd_h;  // per front: first forward task, count
     cudaGraphExec_t exec = nullptr;
     int64_t launches = 0;         // kernels per call
 };
@@ -246,7 +245,7 @@ struct fcw_engine {
     int64_t* uoff_d = nullptr;
     int64_t* poff_d = nullptr;
     int32_t* nsplit_d = nullptr;
-    int32_t *gm_ptr_d = nullptr, *gm_src_d = nullptr, *gm_child_d = nullptr;
+    int32_t *gm_ptr_d = nullptr, *gm_src_d = nullptr;
     int64_t n_urows = 0, n_parts = 0;
     double *val_h = nullptr, *inv_h = nullptr, *val_p = nullptr, *inv_p = nullptr;
     fcw::CsrOperator lg;  // the grounded Poisson operator in FP64, elimination order (refinement residuals)
@@ -265,6 +264,7 @@ struct fcw_engine {
     long long* farea_fx_d = nullptr;  // lean face areas in fixed point
     double area_unscale = 0.0;
     int* err_d = nullptr;
+    int* err_h = nullptr;  // page-locked copy
     std::vector<Workspace> pool;  // blocks in flight: workspace i runs on pool[i].stream
     size_t cur_ws = 0;
     Workspace& cw() { return pool[cur_ws]; }
@@ -348,6 +348,7 @@ struct fcw_engine {
         if (nar.exec) cudaGraphExecDestroy(nar.exec);
         if (nar.horder) cudaFreeHost(nar.horder);
         if (hmap_h) cudaFreeHost(hmap_h);
+        if (err_h) cudaFreeHost(err_h);
         for (cudaEvent_t ev : event_pool) cudaEventDestroy(ev);
         if (stream) cudaStreamDestroy(stream);
     }
@@ -355,10 +356,11 @@ struct fcw_engine {
 
 namespace {
 
+// Waits for e->stream and reports the errors the kernels raised.
 int check_kernel_errors(fcw_engine* e, const char* where) {
-    int h = 0;
-    FCW_CUDA(cudaMemcpyAsync(&h, e->err_d, sizeof(int), cudaMemcpyDeviceToHost, e->stream));
+    FCW_CUDA(cudaMemcpyAsync(e->err_h, e->err_d, sizeof(int), cudaMemcpyDeviceToHost, e->stream));
     FCW_CUDA(cudaStreamSynchronize(e->stream));
+    const int h = *e->err_h;
     if (h) {
         FCW_CUDA(cudaMemsetAsync(e->err_d, 0, sizeof(int), e->stream));
         std::string what;
@@ -532,6 +534,7 @@ int build_engine(fcw_engine* e, const double* V, int64_t nv, const int32_t* F, i
         FCW_CUDA(cudaEventCreateWithFlags(&w.done, cudaEventDisableTiming));
     }
     FCW_TRY(e->dalloc(&e->err_d, 1));
+    FCW_CUDA(cudaHostAlloc(reinterpret_cast<void**>(&e->err_h), sizeof(int), cudaHostAllocDefault));
     FCW_CUDA(cudaMemset(e->err_d, 0, sizeof(int)));
 
     // structure
@@ -621,9 +624,9 @@ int build_engine(fcw_engine* e, const double* V, int64_t nv, const int32_t* F, i
         FCW_TRY(e->upload(&e->asm_rows_d, f.asm_rows));
     }
 
-    // the supernodes' update rows and the per-front-row gather lists of the single-source and
-    // tensor-core sweeps, and the latter's tasks (see solve_tc.cu)
-    {
+    // the tensor-core sweeps' update rows, per-front-row gather lists and tasks, over supernodes (see
+    // solve_tc.cu)
+    if (e->prm.tc_sweeps) {
         const int32_t NS = S.nsuper;
         std::vector<int64_t> uoff(NS + 1, 0), poff(NS, 0);
         std::vector<int32_t> nsplit(NS, 1);
@@ -636,8 +639,8 @@ int build_engine(fcw_engine* e, const double* V, int64_t nv, const int32_t* F, i
             if (nsplit[s] > 1) parts += nsplit[s];
         }
         e->n_urows = uoff[NS];
-        e->n_parts = e->prm.tc_sweeps ? parts : 0;
-        if (e->prm.tc_sweeps) {
+        e->n_parts = parts;
+        {
             std::vector<int2> bt, tft;
             e->tc_fwd_ptr.assign(S.nlevels + 1, 0);
             e->tc_bwd_ptr.assign(S.nlevels + 1, 0);
@@ -660,7 +663,7 @@ int build_engine(fcw_engine* e, const double* V, int64_t nv, const int32_t* F, i
             FCW_TRY(e->upload(&e->nsplit_d, nsplit));
         }
         const int64_t nfront = S.sn_rowptr[NS];
-        std::vector<int32_t> gptr(nfront + 1, 0), gsrc(e->n_urows), gchild(e->n_urows);
+        std::vector<int32_t> gptr(nfront + 1, 0), gsrc(e->n_urows);
         for (int32_t c = 0; c < NS; ++c) {
             const int32_t p = S.sn_parent[c];
             const int32_t nsc = S.sn_c0[c + 1] - S.sn_c0[c];
@@ -675,7 +678,6 @@ int build_engine(fcw_engine* e, const double* V, int64_t nv, const int32_t* F, i
                 for (int64_t q = S.sn_rowptr[c] + nsc; q < S.sn_rowptr[c + 1]; ++q) {
                     const int64_t g = S.sn_rowptr[p] + S.relind[q];
                     gsrc[fill[g]] = (int32_t)(uoff[c] + (q - S.sn_rowptr[c] - nsc));
-                    gchild[fill[g]] = c;
                     fill[g]++;
                 }
             }
@@ -684,7 +686,6 @@ int build_engine(fcw_engine* e, const double* V, int64_t nv, const int32_t* F, i
         FCW_TRY(e->upload(&e->uoff_d, uoff));
         FCW_TRY(e->upload(&e->gm_ptr_d, gptr));
         FCW_TRY(e->upload(&e->gm_src_d, gsrc));
-        FCW_TRY(e->upload(&e->gm_child_d, gchild));
     }
 
     // mesh arrays in elimination order
@@ -1513,7 +1514,7 @@ namespace {
 int narrow_chain(fcw_engine* e, cudaStream_t st) {
     NarrowState& q = e->nar;
     const int64_t n = e->sym.n;
-    const int64_t nu = std::max<int64_t>(e->n_urows, 1);
+    const int64_t nu = std::max<int64_t>(e->fr.n_urows, 1);
     double* U_h = q.pend;
     double* U_p = q.pend + nu;
     double* X_h = q.pend + 2 * nu;
@@ -1522,13 +1523,11 @@ int narrow_chain(fcw_engine* e, cudaStream_t st) {
     FCW_CUDA(cudaMemsetAsync(q.pend, 0xFF, (size_t)(2 * nu + 2 * n) * sizeof(double), st));  // pending
     FCW_CUDA(cudaMemsetAsync(q.u, 0, (size_t)n * sizeof(double), st));
     fcw::NarrowArgs a;
-    a.p = e->plan;
-    a.at_ptr = q.at_ptr;
-    a.uoff = e->uoff_d;
-    a.gm_ptr = e->gm_ptr_d;
-    a.gm_src = e->gm_src_d;
-    a.gm_child = e->gm_child_d;
-    a.iperm = e->iperm_d;
+    a.strip = q.L.strip;
+    a.rec = reinterpret_cast<const int4*>(e->rec_d);
+    a.rec_child = e->rec_child_d;
+    a.more = e->more_d;
+    a.rows = e->front_rows_d;
     a.err = e->err_d;
     // heat: the path's forward tasks, then the whole backward
     mark(e, st, FCW_STAGE_HEAT_FWD);
@@ -1577,38 +1576,41 @@ int narrow_chain(fcw_engine* e, cudaStream_t st) {
 int narrow_ready(fcw_engine* e) {
     NarrowState& q = e->nar;
     if (q.ready) return FCW_OK;
-    const auto& S = e->sym;
-    const int32_t NS = S.nsuper;
-    const int64_t n = S.n;
-    if (fcw::configure_narrow_kernels(S.max_m, e->num_sms, &q.L) != cudaSuccess) {
-        cudaGetLastError();
-        return fail(FCW_E_INVALID, "front too large for the single-source kernels (max_m " + std::to_string(S.max_m) +
-                                       ")");
+    const int64_t n = e->sym.n;
+    int32_t max_ns = 1, max_m = 1;
+    for (int32_t t = 0; t < e->fr.nf; ++t) {
+        max_ns = std::max(max_ns, e->fr.c0[t + 1] - e->fr.c0[t]);
+        max_m = std::max(max_m, e->fr.m[t]);
     }
-    std::vector<int64_t> ptr((size_t)NS + 1);
-    const int64_t total = fcw::narrow_layout(S.sn_c0.data(), S.sn_m.data(), NS, ptr.data());
-    std::vector<int4> ft, bt;
-    std::vector<int32_t> fptr, nf, nb;
-    fcw::narrow_tasks(S.sn_c0.data(), S.sn_m.data(), NS, S.level_nodes.data(), ft, fptr, nf, bt, nb);
+    if (fcw::configure_narrow_kernels(max_ns, max_m, e->num_sms, &q.L) != cudaSuccess) {
+        cudaGetLastError();
+        return fail(FCW_E_INVALID, "front too large for the single-source kernels (" + std::to_string(max_m) + " rows)");
+    }
+    std::vector<fcw::NarrowTask> ft, bt;
+    int64_t nfd = 0, nbd = 0;
+    fcw::narrow_tasks(e->fr, ft, q.fwd_first, q.nfwd_h, bt, &nfd, &nbd);
     q.n_ftasks = (int32_t)ft.size();
     q.n_btasks = (int32_t)bt.size();
-    FCW_TRY(e->upload(&q.at_ptr, ptr));
     FCW_TRY(e->upload(&q.ftasks, ft));
     FCW_TRY(e->upload(&q.btasks, bt));
-    q.fwd_first = fptr;
-    q.nfwd_h = nf;
-    for (double** arr : {&q.at_h, &q.at_p, &q.atb_h, &q.atb_p}) {
-        FCW_TRY(e->dalloc(arr, (size_t)total));
-        FCW_CUDA(cudaMemsetAsync(*arr, 0, (size_t)total * sizeof(double), e->stream));
+    double* rows;
+    FCW_TRY(e->dalloc(&rows, (size_t)e->frp.entries));
+    for (int which = 0; which < 2; ++which) {
+        double*& f = which ? q.at_p : q.at_h;
+        double*& b = which ? q.atb_p : q.atb_h;
+        FCW_TRY(e->dalloc(&f, (size_t)nfd));
+        FCW_TRY(e->dalloc(&b, (size_t)nbd));
+        fcw::launch_front_rows(e->plan, e->frp, which ? e->val_p : e->val_h, which ? e->inv_p : e->inv_h, rows, e->stream);
+        fcw::launch_pack_narrow(e->frp, true, q.ftasks, q.n_ftasks, rows, f, e->stream);
+        fcw::launch_pack_narrow(e->frp, false, q.btasks, q.n_btasks, rows, b, e->stream);
     }
-    fcw::launch_build_narrow(e->plan, e->val_h, e->inv_h, q.at_ptr, q.at_h, q.atb_h, e->stream);
-    fcw::launch_build_narrow(e->plan, e->val_p, e->inv_p, q.at_ptr, q.at_p, q.atb_p, e->stream);
     FCW_CUDA(cudaGetLastError());
+    e->release(rows);
     FCW_TRY(e->dalloc(&q.u, (size_t)n));
     FCW_TRY(e->dalloc(&q.div, (size_t)n));
     FCW_TRY(e->dalloc(&q.y, (size_t)n));
     FCW_TRY(e->dalloc(&q.out, (size_t)n));
-    FCW_TRY(e->dalloc(&q.pend, (size_t)(2 * std::max<int64_t>(e->n_urows, 1) + 2 * n)));
+    FCW_TRY(e->dalloc(&q.pend, (size_t)(2 * std::max<int64_t>(e->fr.n_urows, 1) + 2 * n)));
     FCW_TRY(e->dalloc(&q.sync, 4));
     const size_t cap = 2 + 2 * (size_t)q.n_ftasks;
     FCW_TRY(e->dalloc(&q.order, cap));
@@ -1641,12 +1643,11 @@ int narrow_run(fcw_engine* e, int32_t source) {
     FCW_TRY(narrow_ready(e));
     NarrowState& q = e->nar;
     cudaStream_t st = e->stream;
-    // the source's path to the root, bottom-up, with each supernode's forward tasks
-    const auto& S = e->sym;
+    // the source's path to the root, bottom-up, with each front's forward tasks
     int32_t* o = q.horder;
     int32_t len = 0, prev = -1;
-    o[0] = S.iperm[source];
-    for (int32_t s = S.col_sn[o[0]]; s >= 0; prev = s, s = S.sn_parent[s])
+    o[0] = e->sym.iperm[source];
+    for (int32_t s = e->fr.col_front[o[0]]; s >= 0; prev = s, s = e->fr.parent[s])
         for (int32_t t = q.fwd_first[s]; t < q.fwd_first[s] + q.nfwd_h[s]; ++t) {
             o[2 + 2 * len] = t;
             o[3 + 2 * len] = prev;
@@ -1672,7 +1673,7 @@ int narrow_metrics(fcw_engine* e, int32_t source, const double* targets, int32_t
     FCW_TRY(narrow_run(e, source));
     NarrowState& q = e->nar;
     cudaStream_t st = e->stream;
-    const int64_t n = e->sym.n, nu = std::max<int64_t>(e->n_urows, 1);
+    const int64_t n = e->sym.n, nu = std::max<int64_t>(e->fr.n_urows, 1);
     const double* X_p = q.pend + 2 * nu + n;  // the Poisson solution (elimination order)
     a.src = q.order;                           // its first entry: the source's elimination index
     fcw::launch_shift_stats_one(a, X_p, e->cw().dT64, st);
@@ -1680,7 +1681,6 @@ int narrow_metrics(fcw_engine* e, int32_t source, const double* targets, int32_t
     e->launches += 2;
     FCW_CUDA(cudaGetLastError());
     FCW_CUDA(cudaMemcpyAsync(out_host, a.out, (size_t)stride * sizeof(double), cudaMemcpyDeviceToHost, st));
-    FCW_CUDA(cudaStreamSynchronize(st));
     return check_kernel_errors(e, "metrics");
 }
 
@@ -1696,7 +1696,6 @@ int fcw_compute_distance(fcw_engine* e, int32_t source, double* out_host) {
     NarrowState& q = e->nar;
     cudaStream_t st = e->stream;
     FCW_CUDA(cudaMemcpyAsync(out_host, q.out, (size_t)e->sym.n * sizeof(double), cudaMemcpyDeviceToHost, st));
-    FCW_CUDA(cudaStreamSynchronize(st));
     return check_kernel_errors(e, "distance");
 }
 

@@ -174,44 +174,49 @@ void launch_build_cores(const DevPlan& p, const double* val, const double* inv, 
                         float* hi, float* lo, float* hiT, float* loT, cudaStream_t st);
 
 // ---- one right-hand side: the single-source drop-in (solve_narrow.cu) ----
-constexpr int kNarrowRows = 64;            // stacked rows per chunk of the narrow layout
-constexpr int kNarrowTaskDoubles = 12288;  // panel data of one task (96 KB); fronts up to this many rows
+constexpr int kNarrowTaskDoubles = 11264;  // panel data of one task (88 KB)
+// Forward: rows [r0, r0 + h) of [inv(L_ss); Q_s] times the first `depth` entries of the front's
+// right-hand side. Backward: columns [r0, r0 + h) of X_s, depth = the front's rows from r0 down.
+struct NarrowTask {
+    int64_t off;                      // its panel
+    int64_t row0, urow;               // front-row index of the front's first row; its first update entry
+    int32_t front, r0, h, depth;
+    int32_t c0, ns;
+    int32_t pend;                     // one past the last column of the front's parent
+    int32_t pad;
+};
 struct NarrowArgs {
-    DevPlan p;
-    const double* at = nullptr;       // per supernode [inv(L_ss); Q_s]: forward, 64-row column-major chunks;
-                                      // backward, column-major over all rows
-    const int64_t* at_ptr = nullptr;  // per supernode: offset (doubles, even) in either layout
-    const int4* tasks = nullptr;      // forward: (s, first chunk, chunks); backward: (s, j0, j1)
+    const double* at = nullptr;       // the sweep's panels
+    const NarrowTask* tasks = nullptr;
     int32_t ntasks = 0;
+    int32_t strip = 0;                // backward: doubles a strip may take in shared memory
     // heat forward: the source's elimination index, the path's task count, then (task,
-    // previous supernode on the path) pairs bottom-up
+    // previous front on the path) pairs bottom-up
     const int32_t* order = nullptr;
     const double* R = nullptr;        // forward right-hand side (n)
     double* B = nullptr;              // forward result (n)
     double* X = nullptr;              // backward: the solution (n), pending on entry
-    double* U = nullptr;              // forward update entries (sum nr), pending on entry
-    const int64_t* uoff = nullptr;
-    const int32_t* gm_ptr = nullptr;
-    const int32_t* gm_src = nullptr;
-    const int32_t* gm_child = nullptr;
+    double* U = nullptr;              // forward update entries, pending on entry
+    const int4* rec = nullptr;        // GatherRec per front row
+    const int32_t* rec_child = nullptr;
+    const int32_t* more = nullptr;
+    const int32_t* rows = nullptr;    // elimination row of each front row
     int* ticket = nullptr;            // zero when a sweep starts
-    const int32_t* iperm = nullptr;
     int* err = nullptr;
 };
 struct NarrowLaunch {
-    int grid_fwd = 0, grid_bwd = 0;
+    int grid_fwd = 0, grid_bwd = 0, strip = 0;
     size_t fwd_smem = 0, bwd_smem = 0;
 };
-// Chunk offsets of the narrow layout (nsuper + 1 entries); returns the doubles it holds.
-int64_t narrow_layout(const int32_t* sn_c0, const int32_t* sn_m, int32_t nsuper, int64_t* at_ptr);
-// Forward tasks in level order (supernode s's are the nfwd[s] from fwd_first[s]), backward
-// tasks in reversed level order, and each supernode's task counts.
-void narrow_tasks(const int32_t* sn_c0, const int32_t* sn_m, int32_t nsuper, const int32_t* level_nodes,
-                  std::vector<int4>& fwd, std::vector<int32_t>& fwd_first, std::vector<int32_t>& nfwd,
-                  std::vector<int4>& bwd, std::vector<int32_t>& nbwd);
-void launch_build_narrow(const DevPlan& p, const double* val, const double* inv, const int64_t* at_ptr,
-                         double* at_f, double* at_b, cudaStream_t st);
-cudaError_t configure_narrow_kernels(int max_m, int num_sms, NarrowLaunch* L);
+// Forward tasks in level order (front s's are the nfwd[s] from fwd_first[s]), backward tasks in
+// reversed level order, and the doubles their panels take.
+void narrow_tasks(const Fronts& f, std::vector<NarrowTask>& fwd, std::vector<int32_t>& fwd_first,
+                  std::vector<int32_t>& nfwd, std::vector<NarrowTask>& bwd, int64_t* fwd_doubles,
+                  int64_t* bwd_doubles);
+// The tasks' panels from the fronts' rows (launch_front_rows).
+void launch_pack_narrow(const FrontPlan& f, bool fwd, const NarrowTask* tasks, int32_t ntasks, const double* rows,
+                        double* out, cudaStream_t st);
+cudaError_t configure_narrow_kernels(int max_ns, int max_m, int num_sms, NarrowLaunch* L);
 // Forward sweep (delta: the identity column of a.order's source over its path's tasks; B
 // zero on entry), backward sweep.
 // overlap: start while the stream's previous kernel finishes (programmatic dependent launch);
