@@ -18,7 +18,7 @@
 // Children's rows are added in ascending child order, so results are deterministic.
 //
 // Backward (root -> leaves): X_s = A_s^T [y_s; -X_r], X_r the structure rows (ancestors, final). A
-// task is up to 64 of the front's columns over all rows below them, gathered in 32-row chunks, three
+// task is up to 64 of the front's columns over all rows below them, gathered in 32-row chunks, two
 // chunks in flight. The solution goes to an array of its own, so tasks of one front need no order.
 //
 // Each task's part of A_s is stored as it is used: k-major (for each depth row, the task's rows or
@@ -348,9 +348,23 @@ __global__ void __launch_bounds__(NT, 2) k_fwd(SweepArgs<T> a, int32_t t0) {
             urec[i] = t.r0 + i >= t.ns ? live_record(a, t.row0 + t.r0 + i, tile) : make_int4(-1, -1, -1, -1);
     }
     if (!a.reach) wait_predecessor();
-    __syncthreads();
+    __syncthreads();  // the barriers are initialised, the records are in
 
-    if constexpr (!WIDE) {
+    if (!WIDE && !a.gathers && !a.delta_src) {
+        // a leaf's W is its rows of R: all of them in flight at once
+        for (int e = tid; e < depth4 * VPR; e += NT) {
+            const int f = e / VPR, v = e - f * VPR;
+            T* dst = Vs + f * LW + v * G;
+            if (f < t.depth) {
+                copy16_async(dst, a.R + (int64_t)(t.c0 + f) * a.K + k0 + v * G);
+            } else {
+                T z[G] = {};
+                st_n<T, G>(dst, z);
+            }
+        }
+        copy_async_commit();
+        copy_async_wait<0>();
+    } else if constexpr (!WIDE) {
         // W, four rows per thread in flight
         const int v = tid % VPR, rr = tid / VPR;
         int delta[G];
@@ -468,9 +482,13 @@ __global__ void __launch_bounds__(NT) k_assemble(SweepArgs<T> a, int32_t r0, int
 // ---------------------------------------------------------------------------
 // Backward
 // ---------------------------------------------------------------------------
+// Two chunks in flight: a third leaves an SM two FP64 CTAs instead of three (147k vertices, 1024
+// columns: 1.12 against 1.32 ms for the heat solve) and gains FP32 nothing (1.12 ms either way; 64
+// columns 0.24 against 0.28 ms).
+constexpr int kBwdStages = 2;
 template <typename T, int KT, int M>
-__global__ void __launch_bounds__(NT, sizeof(T) == 8 ? 2 : 3) k_bwd(SweepArgs<T> a, int32_t t0) {
-    constexpr int G = vec<T>(), VPR = KT / G, LW = ld_rhs<T, KT>(), S = 3;
+__global__ void __launch_bounds__(NT, 3) k_bwd(SweepArgs<T> a, int32_t t0) {
+    constexpr int G = vec<T>(), VPR = KT / G, LW = ld_rhs<T, KT>(), S = kBwdStages;
     constexpr int PS = panel_stage<T, M>(), VS = DC * LW;
     extern __shared__ __align__(128) unsigned char smraw[];
     T* Ps = reinterpret_cast<T*>(smraw);
@@ -564,7 +582,7 @@ constexpr size_t fwd_smem() {
 }
 template <typename T, int KT, int M>
 size_t bwd_smem(int max_depth) {
-    return (size_t)3 * (panel_stage<T, M>() + DC * ld_rhs<T, KT>()) * sizeof(T) + (size_t)max_depth * sizeof(int32_t);
+    return (size_t)kBwdStages * (panel_stage<T, M>() + DC * ld_rhs<T, KT>()) * sizeof(T) + (size_t)max_depth * sizeof(int32_t);
 }
 constexpr size_t kSmemMax = 227 * 1024 - 4096;  // static shared memory is kept apart
 

