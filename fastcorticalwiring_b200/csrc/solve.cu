@@ -11,10 +11,11 @@
 //   W   = b_s - the children's update rows that land on s's columns
 //   X_s = inv(L_ss) W                                   (written to Y)
 //   U_s = Q_s W + the children's update rows that land on s's structure
-// and leaves U_s for its parent. A task is up to 128 stacked rows of A_s. On the levels whose fronts
-// are at most 64 columns wide each task gathers W itself, into shared memory; a leaf's A_s has 88
-// rows on average, so one task mostly does the whole front. The wider fronts near the root have many
-// tasks, so there W is assembled once (k_assemble) and the products read it in 32-row chunks.
+// and leaves U_s for its parent. A task is a group of stacked rows of A_s: a leaf's first 128 (its A_s
+// has 88 rows on average, so mostly all of it), 64 elsewhere, 32 where a level has few. On the levels
+// whose fronts are at most 64 columns wide each task gathers W itself, into shared memory. The wider
+// fronts near the root have many tasks, so there W is assembled once (k_assemble) and the products read
+// it in 32-row chunks.
 // Children's rows are added in ascending child order, so results are deterministic.
 //
 // Backward (root -> leaves): X_s = A_s^T [y_s; -X_r], X_r the structure rows (ancestors, final). A
@@ -311,9 +312,9 @@ __device__ __forceinline__ void gather_rows(const SweepArgs<T>& a, const int4* r
 // Forward
 // ---------------------------------------------------------------------------
 template <typename T, int KT, int M, bool WIDE>
-__global__ void __launch_bounds__(NT, 2) k_fwd(SweepArgs<T> a, int32_t t0) {
+__global__ void __launch_bounds__(NT, M == 128 ? 2 : 3) k_fwd(SweepArgs<T> a, int32_t t0) {
     constexpr int G = vec<T>(), VPR = KT / G, RPP = NT / VPR, LW = ld_rhs<T, KT>();
-    constexpr int S = WIDE ? 3 : kNarrowCols / DC;  // a narrow front's chunks are all resident
+    constexpr int S = 2;  // chunks resident: all of a narrow front's (kNarrowCols / DC)
     constexpr int PS = panel_stage<T, M>(), VS = DC * LW;
     extern __shared__ __align__(128) unsigned char smraw[];
     T* Ps = reinterpret_cast<T*>(smraw);
@@ -576,9 +577,9 @@ __global__ void k_reach(const int32_t* __restrict__ col_front, const int32_t* __
     }
 }
 
-template <typename T, int KT, int M, bool WIDE>
+template <typename T, int KT, int M>
 constexpr size_t fwd_smem() {
-    return (size_t)(WIDE ? 3 : kNarrowCols / DC) * (panel_stage<T, M>() + DC * ld_rhs<T, KT>()) * sizeof(T);
+    return (size_t)2 * (panel_stage<T, M>() + DC * ld_rhs<T, KT>()) * sizeof(T);
 }
 template <typename T, int KT, int M>
 size_t bwd_smem(int max_depth) {
@@ -603,34 +604,28 @@ void launch_overlapped(Kern kern, dim3 grid, size_t smem, cudaStream_t st, Args.
     cudaLaunchKernelEx(&cfg, kern, args...);
 }
 
-template <typename T, int KT, int M>
-cudaError_t set_smem() {
-    cudaError_t e = cudaFuncSetAttribute(k_fwd<T, KT, M, true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                         (int)fwd_smem<T, KT, M, true>());
-    if constexpr (M == 128)
-        if (e == cudaSuccess)
-            e = cudaFuncSetAttribute(k_fwd<T, KT, M, false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                     (int)fwd_smem<T, KT, M, false>());
-    if constexpr (M <= 64)
-        if (e == cudaSuccess)
-            e = cudaFuncSetAttribute(k_bwd<T, KT, M>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmemMax);
-    return e;
+template <typename Kern>
+cudaError_t allow_smem(Kern kern, size_t bytes) {
+    return cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
 }
 template <typename T, int KT>
-cudaError_t set_smem_tiles() {
+cudaError_t set_smem() {
     cudaError_t e;
-    if ((e = set_smem<T, KT, 128>())) return e;
-    if ((e = set_smem<T, KT, 64>())) return e;
-    return set_smem<T, KT, 32>();
+    if ((e = allow_smem(k_fwd<T, KT, 128, false>, fwd_smem<T, KT, 128>()))) return e;
+    if ((e = allow_smem(k_fwd<T, KT, 64, false>, fwd_smem<T, KT, 64>()))) return e;
+    if ((e = allow_smem(k_fwd<T, KT, 64, true>, fwd_smem<T, KT, 64>()))) return e;
+    if ((e = allow_smem(k_fwd<T, KT, 32, true>, fwd_smem<T, KT, 32>()))) return e;
+    if ((e = allow_smem(k_bwd<T, KT, 64>, kSmemMax))) return e;
+    return allow_smem(k_bwd<T, KT, 32>, kSmemMax);
 }
 
 template <typename T, int KT>
 void fwd_tile(const SweepArgs<T>& a, int32_t t0, int32_t n, int32_t rows, bool wide, cudaStream_t st) {
     const dim3 grid(n, a.K / KT);
-    if (!wide) launch_overlapped(k_fwd<T, KT, 128, false>, grid, fwd_smem<T, KT, 128, false>(), st, a, t0);
-    else if (rows == 128) launch_overlapped(k_fwd<T, KT, 128, true>, grid, fwd_smem<T, KT, 128, true>(), st, a, t0);
-    else if (rows == 64) launch_overlapped(k_fwd<T, KT, 64, true>, grid, fwd_smem<T, KT, 64, true>(), st, a, t0);
-    else launch_overlapped(k_fwd<T, KT, 32, true>, grid, fwd_smem<T, KT, 32, true>(), st, a, t0);
+    if (!wide && rows == 128) launch_overlapped(k_fwd<T, KT, 128, false>, grid, fwd_smem<T, KT, 128>(), st, a, t0);
+    else if (!wide) launch_overlapped(k_fwd<T, KT, 64, false>, grid, fwd_smem<T, KT, 64>(), st, a, t0);
+    else if (rows == 64) launch_overlapped(k_fwd<T, KT, 64, true>, grid, fwd_smem<T, KT, 64>(), st, a, t0);
+    else launch_overlapped(k_fwd<T, KT, 32, true>, grid, fwd_smem<T, KT, 32>(), st, a, t0);
 }
 template <typename T, int KT>
 void bwd_tile(const SweepArgs<T>& a, int32_t t0, int32_t n, int32_t rows, int32_t max_depth, cudaStream_t st) {
@@ -648,9 +643,9 @@ void asm_tile(const SweepArgs<T>& a, int32_t r0, int32_t n, cudaStream_t st) {
 
 cudaError_t configure_solve_kernels() {
     cudaError_t e;
-    if ((e = set_smem_tiles<double, 64>())) return e;
-    if ((e = set_smem_tiles<float, 64>())) return e;
-    return set_smem_tiles<float, 128>();
+    if ((e = set_smem<double, 64>())) return e;
+    if ((e = set_smem<float, 64>())) return e;
+    return set_smem<float, 128>();
 }
 
 int32_t max_front_rows() { return (int32_t)((kSmemMax - bwd_smem<double, 64, 64>(0)) / sizeof(int32_t)); }

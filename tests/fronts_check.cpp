@@ -81,7 +81,7 @@ static int check(const char* path, int leaf, int width, int relax) {
             CHECK(level[a.front] == l && a.h > 0 && a.h <= t.fwd_rows[l] && a.r0 % 16 == 0);
             CHECK(a.off64 == o64 && a.off32 == o32 && o64 % 16 == 0 && o32 % 16 == 0);
             CHECK(a.depth > 0 && a.depth <= a.ns && (a.r0 + a.h <= a.ns || a.depth == a.ns));
-            if (l < t.first_wide) CHECK(a.depth <= 64 && a.depth == a.ns && t.fwd_rows[l] == 128);
+            if (l < t.first_wide) CHECK(a.depth <= 64);
             else CHECK(a.wrow + a.ns <= t.n_wrows);
             for (int r = a.r0; r < a.r0 + a.h; ++r) {
                 char& w = r < a.ns ? y[a.c0 + r] : u[a.urow + r - a.ns];
