@@ -1010,6 +1010,8 @@ void sweep(fcw_engine* e, fcw::SweepArgs<T> a, const T* fwd, const T* bwd, const
     a.rows = e->front_rows_d;
     a.asm_rows = reinterpret_cast<const int4*>(e->asm_rows_d);
     a.err = e->err_d;
+    const int32_t leaf_f = (int32_t)(sizeof(T) == 8 ? f.leaf_fwd64 : f.leaf_fwd32);
+    const int32_t leaf_b = (int32_t)(sizeof(T) == 8 ? f.leaf_bwd64 : f.leaf_bwd32);
     mark(e, st, stage_fwd);
     a.tasks = e->fwd_tasks;
     a.panel = fwd;
@@ -1017,14 +1019,17 @@ void sweep(fcw_engine* e, fcw::SweepArgs<T> a, const T* fwd, const T* bwd, const
         const bool wide = l >= f.first_wide;
         a.gathers = l > 0;
         if (wide) fcw::launch_assemble<T>(a, f.asm_ptr[l], f.asm_ptr[l + 1] - f.asm_ptr[l], st);
+        if (l == 0 && !wide && fcw::launch_leaves<T>(a, false, f.fwd_ptr[1], f.fwd_rows[0], leaf_f, 0, st)) continue;
         fcw::launch_fwd_level<T>(a, f.fwd_ptr[l], f.fwd_ptr[l + 1] - f.fwd_ptr[l], f.fwd_rows[l], wide, st);
     }
     a.delta_src = nullptr;
     mark(e, st, stage_bwd);
     a.tasks = e->bwd_tasks;
     a.panel = bwd;
-    for (int32_t l = f.nlevels - 1; l >= 0; --l)
+    for (int32_t l = f.nlevels - 1; l >= 0; --l) {
+        if (l == 0 && fcw::launch_leaves<T>(a, true, f.bwd_ptr[1], f.bwd_rows[0], leaf_b, e->bwd_depth[0], st)) continue;
         fcw::launch_bwd_level<T>(a, f.bwd_ptr[l], f.bwd_ptr[l + 1] - f.bwd_ptr[l], f.bwd_rows[l], e->bwd_depth[l], st);
+    }
     e->launches += 2 * (int64_t)f.nlevels + (f.nlevels - f.first_wide);
 }
 

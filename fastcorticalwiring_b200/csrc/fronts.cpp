@@ -250,6 +250,16 @@ int build_fronts(const Symbolic& S, Fronts& f, std::string& err) {
                 f.bwd.push_back(k);
             }
         }
+        if (l == 0) {
+            for (const SweepTask& k : f.fwd) {
+                f.leaf_fwd64 = std::max(f.leaf_fwd64, padded_depth(k.depth) * panel_ld(k.h, true));
+                f.leaf_fwd32 = std::max(f.leaf_fwd32, padded_depth(k.depth) * panel_ld(k.h, false));
+            }
+            for (const SweepTask& k : f.bwd) {
+                f.leaf_bwd64 = std::max(f.leaf_bwd64, padded_depth(k.depth) * panel_ld(k.h, true));
+                f.leaf_bwd32 = std::max(f.leaf_bwd32, padded_depth(k.depth) * panel_ld(k.h, false));
+            }
+        }
         f.fwd_ptr.push_back((int32_t)f.fwd.size());
         f.bwd_ptr.push_back((int32_t)f.bwd.size());
         f.asm_ptr.push_back((int32_t)(f.asm_rows.size() / 4));

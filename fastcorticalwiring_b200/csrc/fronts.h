@@ -60,6 +60,7 @@ struct Fronts {
     std::vector<int32_t> asm_rows;  // 4 per row: front row index, elimination row, front, -
     int64_t n_urows = 0, n_wrows = 0;
     int64_t fwd64 = 0, bwd64 = 0, fwd32 = 0, bwd32 = 0;  // entries of the panel arrays
+    int64_t leaf_fwd64 = 0, leaf_bwd64 = 0, leaf_fwd32 = 0, leaf_bwd32 = 0;  // most of one task of level 0
 };
 
 int build_fronts(const Symbolic& S, Fronts& f, std::string& err);

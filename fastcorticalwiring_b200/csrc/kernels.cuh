@@ -123,6 +123,12 @@ void launch_assemble(const SweepArgs<T>& a, int32_t r0, int32_t nrows, cudaStrea
 template <typename T>
 void launch_bwd_level(const SweepArgs<T>& a, int32_t t0, int32_t ntasks, int32_t rows, int32_t max_depth,
                       cudaStream_t st);
+// The leaf level of either sweep (tasks [0, ntasks) of `rows` rows; panel: the most entries of a task's
+// panel) by CTAs that keep a task's panel over several column tiles. False: no such form for these sizes,
+// nothing was launched.
+template <typename T>
+bool launch_leaves(const SweepArgs<T>& a, bool back, int32_t ntasks, int32_t rows, int32_t panel, int32_t max_depth,
+                   cudaStream_t st);
 void launch_reach(const int32_t* col_front, const int32_t* parent, int32_t nfronts, int32_t nlevels,
                   const int32_t* src, int32_t K, uint8_t* reach, cudaStream_t st);
 

@@ -67,6 +67,11 @@ __device__ __forceinline__ void wait_predecessor() { asm volatile("griddepcontro
 __device__ __forceinline__ void copy16_async(void* smem, const void* gmem) {
     asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(tc::smem_u32(smem)), "l"(gmem) : "memory");
 }
+__device__ __forceinline__ void copy16_async_or_zero(void* smem, const void* gmem, bool copy) {
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;\n" ::"r"(tc::smem_u32(smem)), "l"(gmem),
+                 "r"(copy ? 16 : 0)
+                 : "memory");
+}
 __device__ __forceinline__ void copy_async_commit() { asm volatile("cp.async.commit_group;\n" ::: "memory"); }
 template <int N>
 __device__ __forceinline__ void copy_async_wait() { asm volatile("cp.async.wait_group %0;\n" ::"n"(N) : "memory"); }
@@ -559,6 +564,227 @@ __global__ void __launch_bounds__(NT, 3) k_bwd(SweepArgs<T> a, int32_t t0) {
     acc.visit(t.h, [&](int r, int c, T* v) { st_n<T, A::V>(x + (int64_t)r * a.K + c, v); });
 }
 
+// ---------------------------------------------------------------------------
+// Leaves, panel resident
+// ---------------------------------------------------------------------------
+// Half the flops of a sweep are the leaves'. With a CTA per task and column tile, each CTA fetched its
+// panel again, waited for its right-hand sides before it multiplied, and its warps waited for the
+// longest one's rows at every chunk (the triangle makes them unequal; 5.5 of 8 had rows at all): 860 us
+// forward and 740 backward for 460 us of FP64 tensor work each (147k vertices, 1024 columns). Here a CTA keeps its task's panel over many columns, and each warp takes column
+// groups of its own (8 or 16 columns, all rows) with its own asynchronous ring of right-hand sides:
+// warps have equal work and never meet, and loads run ahead across groups. Rows are cut at 8 instead of
+// 16 (tiles no depth reaches are branched past: a predicated-off matrix instruction still takes its
+// slot). Bound by issue around the matrix instructions (tensor pipe 60-66% busy). Poisson forward 2.12 to 1.96 ms and
+// backward 1.48 to 1.36, heat backward 1.11 to 1.04; FP32 backward 1.12 to 1.08. FP32 forward takes the
+// general kernel: more shared-memory reads per product here, 1.54 against 1.44 ms.
+constexpr int kLeafStages = 3, LD = 16;  // a warp's ring: chunks, depth rows per chunk
+
+// Products of one warp: C (h rows x CW columns) += P V, P k-major in the CTA's panel, V the warp's own
+// [depth][CW] rows. Row tiles are numbered so that the ones a depth reaches are the last: forward, the
+// rows below the diagonal, so a task's last tile is the accumulators' last; backward, the columns left of
+// it, so the order is reversed. A case per first tile then keeps every register index static.
+struct WarpF32 {  // backward, 64 columns of X_s
+    static constexpr int CW = 32, TC = 4, NQ = 4, V = TC;  // TC: a thread's columns
+    unsigned long long c[NQ][2][TC];  // rows 4i + {0, 1}, {2, 3} of tile q
+    static __device__ __forceinline__ int slot(int, int col) { return col; }
+    __device__ __forceinline__ void zero() {
+#pragma unroll
+        for (int q = 0; q < NQ; ++q)
+#pragma unroll
+            for (int e = 0; e < 2 * TC; ++e) c[q][e / TC][e % TC] = 0ull;
+    }
+    static __device__ __forceinline__ int row(int q) { return 16 * (NQ - 1 - q); }
+    template <int Q0>
+    __device__ __forceinline__ void tiles(const float* pp, int ld, const float* vp, int nd) {
+#pragma unroll 2
+        for (int d = 0; d < nd; ++d) {
+            float w[TC];
+            ld_n<float, TC>(vp + d * CW, w);
+            unsigned long long w2[TC];
+#pragma unroll
+            for (int e = 0; e < TC; ++e) asm("mov.b64 %0, {%1, %1};" : "=l"(w2[e]) : "f"(w[e]));
+#pragma unroll
+            for (int q = Q0; q < NQ; ++q) {
+                const ulonglong2 x = *reinterpret_cast<const ulonglong2*>(pp + d * ld - 16 * q);
+#pragma unroll
+                for (int e = 0; e < TC; ++e) {
+                    asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(c[q][0][e]) : "l"(x.x), "l"(w2[e]));
+                    asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(c[q][1][e]) : "l"(x.y), "l"(w2[e]));
+                }
+            }
+        }
+    }
+    template <int A = 0, int B = NQ>  // q0 in [A, B)
+    __device__ __forceinline__ void from(int q0, const float* pp, int ld, const float* vp, int nd) {
+        constexpr int H = (A + B) / 2;
+        if constexpr (B - A == 1) tiles<A>(pp, ld, vp, nd);
+        else if (q0 < H) from<A, H>(q0, pp, ld, vp, nd);
+        else from<H, B>(q0, pp, ld, vp, nd);
+    }
+    // depths [base, base + nd) of the task, P at its depth `base`
+    __device__ __forceinline__ void run(const float* P, int ld, const float* Vm, int base, int, int nd, int h) {
+        const int lane = threadIdx.x & 31, q0 = NQ - min((h + 15) / 16, (base + LD - 1) / 16 + 1);
+        from(q0, P + 4 * (lane >> 3) + row(0), ld, Vm + TC * (lane & 7), nd);
+    }
+    // f(row, col, float* v): V adjacent columns
+    template <class F>
+    __device__ __forceinline__ void visit(int h, F&& f) {
+        const int lane = threadIdx.x & 31, i = lane >> 3, k = TC * (lane & 7);
+#pragma unroll
+        for (int q = 0; q < NQ; ++q)
+#pragma unroll
+            for (int p = 0; p < 2; ++p) {
+                float a[TC], b[TC];
+#pragma unroll
+                for (int e = 0; e < TC; ++e) asm("mov.b64 {%0, %1}, %2;" : "=f"(a[e]), "=f"(b[e]) : "l"(c[q][p][e]));
+                const int r = row(q) + 4 * i + 2 * p;
+                if (r < h) f(r, k, a);
+                if (r + 1 < h) f(r + 1, k, b);
+            }
+    }
+};
+template <int M, bool BACK>
+struct WarpF64 {
+    static constexpr int CW = M == 128 ? 8 : 16, NM = M / 8, NN = CW / 8, V = 2;
+    double c[NM][NN][2];
+    // where column `col` of depth row d lies: fragment reads (4 depths x 8 columns) hit distinct banks
+    static __device__ __forceinline__ int slot(int d, int col) { return CW == 8 ? col ^ (4 * ((d >> 1) & 1)) : col ^ (4 * (d & 3)); }
+    __device__ __forceinline__ void zero() {
+#pragma unroll
+        for (int m = 0; m < NM; ++m)
+#pragma unroll
+            for (int n = 0; n < NN; ++n) c[m][n][0] = c[m][n][1] = 0.0;
+    }
+    static __device__ __forceinline__ int row(int m, int h) { return 8 * (BACK ? NM - 1 - m : m - NM + (h + 7) / 8); }
+    template <int M0>
+    __device__ __forceinline__ void tiles(const double* pp, int ld, const double* vp, int nd) {
+#pragma unroll 1
+        for (int d = 0; d < nd; d += 4) {
+            double a[NM], b[NN];
+#pragma unroll
+            for (int n = 0; n < NN; ++n) b[n] = vp[d * CW + slot(threadIdx.x & 3, 8 * n + ((threadIdx.x >> 2) & 7))];
+#pragma unroll
+            for (int m = M0; m < NM; ++m) a[m] = pp[d * ld + (BACK ? -8 : 8) * m];
+#pragma unroll
+            for (int m = M0; m < NM; ++m)
+#pragma unroll
+                for (int n = 0; n < NN; ++n)
+                    asm("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0, %1}, {%2}, {%3}, {%0, %1};\n"
+                        : "+d"(c[m][n][0]), "+d"(c[m][n][1])
+                        : "d"(a[m]), "d"(b[n]));
+        }
+    }
+    template <int A = 0, int B = NM>  // m0 in [A, B)
+    __device__ __forceinline__ void from(int m0, const double* pp, int ld, const double* vp, int nd) {
+        constexpr int H = (A + B) / 2;
+        if constexpr (B - A == 1) tiles<A>(pp, ld, vp, nd);
+        else if (m0 < H) from<A, H>(m0, pp, ld, vp, nd);
+        else from<H, B>(m0, pp, ld, vp, nd);
+    }
+    __device__ __forceinline__ void run(const double* P, int ld, const double* Vm, int base, int r0, int nd, int h) {
+        const int lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3, nm = (h + 7) / 8;
+        for (int d = 0; d < nd; d += 8) {
+            const int m0 = BACK ? NM - min(nm, (base + d + 7) / 8 + 1) : NM - nm + max(0, (base + d - r0) / 8);
+            from(m0, P + (d + t) * ld + g + row(0, h), ld, Vm + (d + t) * CW, min(8, nd - d));
+        }
+    }
+    template <class F>
+    __device__ __forceinline__ void visit(int h, F&& f) {
+        const int lane = threadIdx.x & 31, k = 2 * (lane & 3);
+#pragma unroll
+        for (int m = 0; m < NM; ++m) {
+            const int r = row(m, h) + (lane >> 2);
+            if (r >= 0 && r < h)
+#pragma unroll
+                for (int n = 0; n < NN; ++n) f(r, k + 8 * n, c[m][n]);
+        }
+    }
+};
+template <typename T, int M, bool BACK>
+using WarpAcc = std::conditional_t<sizeof(T) == 8, WarpF64<M, BACK>, WarpF32>;
+
+// per: the column groups of this CTA's warps together
+template <typename T, int M, bool BACK>
+__global__ void __launch_bounds__(NT, 2) k_leaf(SweepArgs<T> a, int32_t per, int32_t panel_max) {
+    using A = WarpAcc<T, M, BACK>;
+    constexpr int G = vec<T>(), CW = A::CW, VPR = CW / G, S = kLeafStages, VS = LD * CW;
+    extern __shared__ __align__(128) unsigned char smraw[];
+    T* Ps = reinterpret_cast<T*>(smraw);
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    T* Vs = Ps + panel_max + warp * (S * VS);
+    int32_t* idx = reinterpret_cast<int32_t*>(Ps + panel_max + NT / 32 * (S * VS));  // backward: the depth rows
+    __shared__ __align__(8) uint64_t bar;
+    allow_dependents();
+    const SweepTask t = a.tasks[blockIdx.x];
+    const int own = BACK ? t.ns - t.r0 : 0;  // backward: depth rows [0, own) are y_s, then the structure rows
+    const int ld = panel_stride<T>(t.h), depth4 = (t.depth + 3) & ~3;
+    const int g0 = blockIdx.y * per, g1 = min(g0 + per, a.K / CW);
+    if (tid == 0) {
+        tc::mbar_init(&bar, 1);
+        tc::fence_mbar_init();
+        const uint32_t bytes = (uint32_t)(depth4 * ld * (int)sizeof(T));
+        tc::mbar_arrive_expect_tx(&bar, bytes);
+        tc::bulk_load(Ps, a.panel + (sizeof(T) == 8 ? t.off64 : t.off32), bytes, &bar);
+    }
+    if constexpr (BACK)
+        for (int i = tid; i < t.depth; i += NT) idx[i] = a.rows[t.row0 + t.r0 + i];
+    wait_predecessor();
+    __syncthreads();
+    // a group's leading depth rows with a zero right-hand side: y_s = 0 off the sources' paths (reach was
+    // written launches ago); whole steps of four are left out
+    auto zeros = [&](int g) { return (BACK && a.reach && !reached(a, t.front, g * CW / kReachCols)) ? own : 0; };
+    int pg = g0 + warp, pz = pg < g1 ? zeros(pg) : 0, pd = pz & ~3, ps = 0;  // next chunk to load: group, depth, stage
+    auto load_next = [&]() {
+        while (pg < g1 && pd >= t.depth) {
+            pg += NT / 32;
+            if (pg < g1) pz = zeros(pg);
+            pd = pz & ~3;
+        }
+        if (pg < g1) {
+            T* V = Vs + ps * VS;
+            const int off = pg * CW + G * (lane % VPR);
+            const T *ry = (BACK ? a.Y : a.R + (int64_t)t.c0 * a.K) + off, *rx = a.X + off;
+#pragma unroll
+            for (int f = lane / VPR; f < LD; f += 32 / VPR) {
+                const int d = min(pd + f, t.depth - 1);
+                const T* src = BACK ? (d < own ? ry : rx) + (int64_t)idx[d] * a.K : ry + (int64_t)d * a.K;
+                copy16_async_or_zero(V + f * CW + A::slot(f, G * (lane % VPR)), src, pd + f < t.depth && pd + f >= pz);
+            }
+            pd += LD;
+            ps = ps + 1 == S ? 0 : ps + 1;
+        }
+        copy_async_commit();
+    };
+#pragma unroll
+    for (int s = 0; s < S - 1; ++s) load_next();
+    wait_panel(&bar, 0, a.err);
+    A acc;
+    int cs = 0;
+    for (int g = g0 + warp; g < g1; g += NT / 32) {
+        acc.zero();
+        for (int base = zeros(g) & ~3; base < t.depth; base += LD) {
+            copy_async_wait<S - 2>();
+            __syncwarp();
+            acc.run(Ps + base * ld, ld, Vs + cs * VS, base, t.r0, min(LD, t.depth - base), t.h);
+            __syncwarp();  // the stage is free
+            load_next();
+            cs = cs + 1 == S ? 0 : cs + 1;
+        }
+        const int k0 = g * CW;
+        if constexpr (BACK) {
+            T* x = a.X + (int64_t)(t.c0 + t.r0) * a.K + k0;
+            acc.visit(t.h, [&](int r, int c, T* v) { st_n<T, A::V>(x + (int64_t)r * a.K + c, v); });
+        } else {
+            T* y = a.Y + (int64_t)t.c0 * a.K + k0;
+            T* u = a.U + (t.urow - t.ns) * (int64_t)a.K + k0;
+            acc.visit(t.h, [&](int r, int c, T* v) {
+                const int R = t.r0 + r;
+                st_n<T, A::V>((R < t.ns ? y : u) + (int64_t)R * a.K + c, v);
+            });
+        }
+    }
+}
+
 // reach[f * tiles + t]: some source of column tile t (kReachCols columns) has front f on its path
 // to the root.
 __global__ void k_reach(const int32_t* __restrict__ col_front, const int32_t* __restrict__ parent,
@@ -585,6 +811,16 @@ template <typename T, int KT, int M>
 size_t bwd_smem(int max_depth) {
     return (size_t)kBwdStages * (panel_stage<T, M>() + DC * ld_rhs<T, KT>()) * sizeof(T) + (size_t)max_depth * sizeof(int32_t);
 }
+constexpr size_t kLeafSmem = 113 * 1024 - 1024;  // of two CTAs per SM
+constexpr int64_t kLeafCtas = 2368;               // eight waves of them
+// Least tasks times column rounds (a warp's groups) for which k_leaf is the faster: with fewer, its
+// CTAs, each with all of a panel to fetch first, do not fill the chip. 147k vertices FP64, backward:
+// 2066 rounds (128 columns) 0.324 against 0.334 ms, 16528 (1024) 1.36 against 1.48; 37k vertices: 1038
+// rounds equal, 2076 0.241 against 0.245; 9k vertices, forward: 2096 0.160 against 0.163, 131 0.069
+// against 0.064. With reach flags rounds differ in length, so more are needed: 147k vertices 16528
+// 1.04 against 1.11 ms, 8264 0.612 against 0.633, 4132 0.403 against 0.400; 37k vertices 4152 0.306
+// against 0.297.
+constexpr int64_t kLeafRounds = 1184, kLeafRoundsReach = 5920;
 constexpr size_t kSmemMax = 227 * 1024 - 4096;  // static shared memory is kept apart
 
 // A launch that may start while the stream's previous kernel finishes; its reads of that kernel's
@@ -615,6 +851,9 @@ cudaError_t set_smem() {
     if ((e = allow_smem(k_fwd<T, KT, 64, false>, fwd_smem<T, KT, 64>()))) return e;
     if ((e = allow_smem(k_fwd<T, KT, 64, true>, fwd_smem<T, KT, 64>()))) return e;
     if ((e = allow_smem(k_fwd<T, KT, 32, true>, fwd_smem<T, KT, 32>()))) return e;
+    if constexpr (sizeof(T) == 8)
+        if ((e = allow_smem(k_leaf<T, 128, false>, kLeafSmem))) return e;
+    if ((e = allow_smem(k_leaf<T, 64, true>, kLeafSmem))) return e;
     if ((e = allow_smem(k_bwd<T, KT, 64>, kSmemMax))) return e;
     return allow_smem(k_bwd<T, KT, 32>, kSmemMax);
 }
@@ -632,6 +871,21 @@ void bwd_tile(const SweepArgs<T>& a, int32_t t0, int32_t n, int32_t rows, int32_
     const dim3 grid(n, a.K / KT);
     if (rows == 64) launch_overlapped(k_bwd<T, KT, 64>, grid, bwd_smem<T, KT, 64>(max_depth), st, a, t0);
     else launch_overlapped(k_bwd<T, KT, 32>, grid, bwd_smem<T, KT, 32>(max_depth), st, a, t0);
+}
+// The leaf level with its panels resident, where two CTAs fit an SM; false: not taken.
+template <typename T, int M, bool BACK>
+bool leaf_groups(const SweepArgs<T>& a, int32_t n, int32_t panel, int32_t max_depth, cudaStream_t st) {
+    using A = WarpAcc<T, M, BACK>;
+    constexpr int W = NT / 32;
+    const size_t smem = ((size_t)panel + W * kLeafStages * LD * A::CW) * sizeof(T) +
+                        (BACK ? (size_t)max_depth * sizeof(int32_t) : 0);
+    const int rounds = a.K / A::CW / W;  // column groups per warp, were a CTA to take them all
+    if (smem > kLeafSmem || (int64_t)n * rounds < (a.reach ? kLeafRoundsReach : kLeafRounds)) return false;
+    const int want = (int)std::max<int64_t>(1, std::min<int64_t>(rounds, (int64_t)n * rounds / kLeafCtas));
+    const int ny = (rounds + want - 1) / want, per = W * ((rounds + ny - 1) / ny);
+    const int groups = a.K / A::CW;
+    launch_overlapped(k_leaf<T, M, BACK>, dim3(n, (groups + per - 1) / per), smem, st, a, per, panel);
+    return true;
 }
 template <typename T, int KT>
 void asm_tile(const SweepArgs<T>& a, int32_t r0, int32_t n, cudaStream_t st) {
@@ -656,6 +910,14 @@ void launch_fwd_level(const SweepArgs<T>& a, int32_t t0, int32_t ntasks, int32_t
     constexpr int W = wide_tile<T>();
     if (W != 64 && a.K % W == 0) fwd_tile<T, W>(a, t0, ntasks, rows, wide, st);
     else fwd_tile<T, 64>(a, t0, ntasks, rows, wide, st);
+}
+template <typename T>
+bool launch_leaves(const SweepArgs<T>& a, bool back, int32_t ntasks, int32_t rows, int32_t panel, int32_t max_depth,
+                   cudaStream_t st) {
+    if (ntasks <= 0 || a.K <= 0 || rows > (back ? 64 : 128) || a.delta_src) return false;
+    if (back) return leaf_groups<T, 64, true>(a, ntasks, panel, max_depth, st);
+    if constexpr (sizeof(T) == 8) return leaf_groups<T, 128, false>(a, ntasks, panel, max_depth, st);
+    return false;
 }
 template <typename T>
 void launch_assemble(const SweepArgs<T>& a, int32_t r0, int32_t nrows, cudaStream_t st) {
@@ -683,6 +945,7 @@ void launch_reach(const int32_t* col_front, const int32_t* parent, int32_t nfron
 #define FCW_SWEEPS(T)                                                                                           \
     template void launch_fwd_level<T>(const SweepArgs<T>&, int32_t, int32_t, int32_t, bool, cudaStream_t);      \
     template void launch_assemble<T>(const SweepArgs<T>&, int32_t, int32_t, cudaStream_t);                      \
+    template bool launch_leaves<T>(const SweepArgs<T>&, bool, int32_t, int32_t, int32_t, int32_t, cudaStream_t); \
     template void launch_bwd_level<T>(const SweepArgs<T>&, int32_t, int32_t, int32_t, int32_t, cudaStream_t);
 FCW_SWEEPS(double)
 FCW_SWEEPS(float)

@@ -71,6 +71,28 @@ def test_source_order_changes_nothing(block_k, count):
         eng.close()
 
 
+@pytest.mark.parametrize("count,params", [
+    (1000, dict(leaf_size=16, max_width=20, relax=8)),  # thousands of leaves: both sweeps, reach flags too
+    (600, {}),                                          # 64-column leaves, a ragged number of column groups
+])
+def test_resident_leaves_match_general_sweeps(count, params):
+    """Many leaves and columns keep the leaves' panels in shared memory; a few columns of the same
+    engine take the general kernels. Same factor, same depth order: FP64 to 1e-12 of the maximum, mixed
+    to the 1e-5 above."""
+    g = folded_icosphere(6, seed=4, jitter=0.2)
+    pm = M.prepare(g.vertices, g.faces, g.cortex_mask)
+    src = np.random.default_rng(count).permutation(pm.n_vertices)[:count].astype(np.int32)
+    eng = engine.HeatEngine(pm.V, pm.F, block_k=1024, pipeline_depth=1, **params)
+    try:
+        sel = np.arange(7, count, 97)
+        for precision, tol in (("fp64", 1e-12), ("mixed", 1e-5)):
+            ref = eng.compute_distances(src[sel], precision=precision)
+            d = eng.compute_distances(src, precision=precision)[sel]
+            assert np.max(np.abs(d - ref)) <= tol * np.max(np.abs(ref)), precision
+    finally:
+        eng.close()
+
+
 def test_invalid_source_is_refused():
     g = folded_icosphere(3, seed=1)
     pm = M.prepare(g.vertices, g.faces, g.cortex_mask)
