@@ -447,13 +447,35 @@ __device__ __forceinline__ int sub_of(double q, int kb, int sb) {
 
 // A source's distance field with its near-face bins (lean_geometry.py:117-299 restated over
 // the faces that can matter): bins [0, rc) are complete, larger bins are never queried.
-template <typename T>
+// TEAM: `team` warps evaluate together (each a share of the faces, partial sums exchanged through
+// S.red, every warp of the team with the same results).
+template <typename T, bool TEAM>
 struct Field {
     const T* d;
     const MetricArgs* a;
     SrcShared* s;
     const int4* band;      // near faces' records sorted by sub-bin
     const int32_t* longf;  // near faces whose distance extent exceeds the bin width
+    int team = 1, member = 0;
+    mutable int parity = 0;
+
+    __device__ int step() const { return TEAM ? 32 * team : 32; }
+    __device__ int first() const { return (threadIdx.x & 31) + (TEAM ? 32 * member : 0); }
+    __device__ void team_sum(double& s1, double& s2) const {
+        if (!TEAM || team == 1) return;
+        const int warp = threadIdx.x >> 5, w0 = warp - member;
+        parity ^= 2;  // the other half is still being read by slower warps of the team
+        if ((threadIdx.x & 31) == 0) {
+            s->red[warp][parity] = s1;
+            s->red[warp][parity + 1] = s2;
+        }
+        asm volatile("bar.sync %0, %1;" ::"r"(1 + w0 / team), "r"(32 * team) : "memory");
+        s1 = s2 = 0.0;
+        for (int w = w0; w < w0 + team; ++w) {
+            s1 += s->red[w][parity];
+            s2 += s->red[w][parity + 1];
+        }
+    }
 
     __device__ double dv(int v) const { return (double)d[v]; }
     __device__ int bin_of(double dmax) const {
@@ -483,13 +505,13 @@ struct Field {
         x2 += da;
     }
 
-    // Faces with bin in [kr, kend) plus long faces with bin >= kend, summed by one warp;
+    // Faces with bin in [kr, kend) plus long faces with bin >= kend, summed by one warp (or team);
     // `inside` + s1 is the area (mode 0). Within complete bins only the sub-bins
     // [j0, j1) are visited: every face of a lower sub-bin has hi < r (face_cdf would
     // return its whole area, summed into `inside` from the prefix), and every face
     // from sub-bin j1 on has lo >= r (both of its terms are exactly zero).
     __device__ void band_sum(int kr, int kend, double r, int mode, double& s1, double& s2, double& inside) const {
-        const int lane = threadIdx.x & 31;
+        const int lane = threadIdx.x & 31, first = this->first(), step = this->step();
         double x1 = 0.0, x2 = 0.0;
         const int* fv = a->fv;
         if (kend <= s->rc) {
@@ -502,10 +524,10 @@ struct Field {
             const int j1 = far ? j0 + __ffs(far) : jend;
             inside = s->pre[j0];
             // sub-bin j's faces are band[ptr[j-1], ptr[j]) after the counting sort
-            int j = (j0 > 0 ? s->ptr[j0 - 1] : 0) + lane;
+            int j = (j0 > 0 ? s->ptr[j0 - 1] : 0) + first;
             const int je = s->ptr[j1 - 1];
             if (mode == 1) {  // |grad d| goes by the face's own corner order
-                for (; j < je; j += 32) face_term(ordered_band<T>() ? band[j].w : band[j].x, r, mode, x1, x2);
+                for (; j < je; j += step) face_term(ordered_band<T>() ? band[j].w : band[j].x, r, mode, x1, x2);
             } else if (ordered_band<T>()) {
                 auto term = [&](const int4& q, double A) {
                     double ar, da;
@@ -514,20 +536,20 @@ struct Field {
                     x1 += ar;
                     x2 += da;
                 };
-                for (; j + 32 < je; j += 64) {  // two faces per lane in flight
-                    const int4 q0 = band[j], q1 = band[j + 32];
+                for (; j + step < je; j += 2 * step) {  // two faces per lane in flight
+                    const int4 q0 = band[j], q1 = band[j + step];
                     const double A0 = a->farea[q0.w], A1 = a->farea[q1.w];
                     term(q0, A0);
                     term(q1, A1);
                 }
-                for (; j < je; j += 32) term(band[j], a->farea[band[j].w]);
+                for (; j < je; j += step) term(band[j], a->farea[band[j].w]);
             }
             // two records per lane in flight
-            for (; j + 32 < je; j += 64) {
+            for (; j + step < je; j += 2 * step) {
                 int4 q[2];
                 double dd[2][3];
 #pragma unroll
-                for (int u = 0; u < 2; ++u) q[u] = band[j + 32 * u];
+                for (int u = 0; u < 2; ++u) q[u] = band[j + step * u];
 #pragma unroll
                 for (int u = 0; u < 2; ++u) {
                     dd[u][0] = dv(q[u].y);
@@ -537,26 +559,27 @@ struct Field {
 #pragma unroll
                 for (int u = 0; u < 2; ++u) rec_term(q[u], dd[u][0], dd[u][1], dd[u][2], r, x1, x2);
             }
-            for (; j < je; j += 32) {
+            for (; j < je; j += step) {
                 const int4 q0 = band[j];
                 rec_term(q0, dv(q0.y), dv(q0.z), dv(q0.w), r, x1, x2);
             }
         } else {  // beyond the complete bins: scan every face (not reached for healthy fields)
             inside = prefix_at(kr);
-            for (int f = lane; f < a->nf; f += 32) {
+            for (int f = first; f < a->nf; f += step) {
                 const double d0 = dv(fv[3 * f]), d1 = dv(fv[3 * f + 1]), d2 = dv(fv[3 * f + 2]);
                 if (!(isfinite(d0) && isfinite(d1) && isfinite(d2))) continue;
                 const int kb = bin_of(fmax(fmax(d0, d1), d2));
                 if (kb >= kr && kb < kend) face_term(f, r, mode, x1, x2);
             }
         }
-        for (int j = lane; j < s->nlong; j += 32) {
+        for (int j = first; j < s->nlong; j += step) {
             const int f = longf[j];
             const double d0 = dv(fv[3 * f]), d1 = dv(fv[3 * f + 1]), d2 = dv(fv[3 * f + 2]);
             if (bin_of(fmax(fmax(d0, d1), d2)) >= kend) face_term(f, r, mode, x1, x2);
         }
         s1 = warp_sum(x1);
         s2 = warp_sum(x2);
+        team_sum(s1, s2);
     }
 
     // lean_geometry.py:183-212
@@ -642,7 +665,7 @@ struct Field {
 //      64-bit shared atomic per face) took 60% of the kernel; 147k vertices, 1024
 //      sources: 1.79 to 1.38 ms (FP64 1.93 to 1.74), 9k: 0.26 to 0.21 ms;
 //   3. one warp per target: bracket + safeguarded Newton + perimeter; then the samples.
-template <typename T, int NT>
+template <typename T, int NT, bool TEAM>
 __global__ void __launch_bounds__(NT, 1024 / NT) k_source_metrics(MetricArgs a, const T* __restrict__ dT) {
     __shared__ SrcShared S;
     const int k = blockIdx.x;
@@ -729,7 +752,7 @@ __global__ void __launch_bounds__(NT, 1024 / NT) k_source_metrics(MetricArgs a, 
         if (a.targets[t] > tmax && a.targets[t] <= S.total * (1.0 + 1e-12)) tmax = a.targets[t];
 
     // 2. near faces, with a growing cut if the margin was not enough
-    Field<T> F{d, &a, &S, band, longf};
+    Field<T, TEAM> F{d, &a, &S, band, longf};
     for (int attempt = 0; attempt < 32; ++attempt) {
         const int rc = S.rc;
         const int nbb = min(rc + 1, nbins);  // complete bins [0, nbb)
@@ -924,13 +947,22 @@ __global__ void __launch_bounds__(NT, 1024 / NT) k_source_metrics(MetricArgs a, 
 
     // 3. radii + perimeters, one warp per target (lean_geometry.py:315-324)
     // (the largest targets, with the most faces near them, first: the short ones fill the last round)
-    for (int i = warp; i < nt; i += nwarps) {
+    // TEAM: two or four warps per target while that leaves a team for each (15: named barriers), so that
+    // 12 targets do not leave 20 of 32 warps idle.
+    int team = 1;
+    if constexpr (TEAM)
+        while (team < 4 && min(nwarps / (2 * team), 15) >= nt) team *= 2;
+    const int nteams = team > 1 ? min(nwarps / team, 15) : nwarps, mine = warp / team;
+    F.team = team;
+    F.member = warp - mine * team;
+    const bool lead = lane == 0 && F.member == 0;
+    for (int i = mine; i < nt && mine < nteams; i += nteams) {
         const int t = nt - 1 - i;
         int ev = 0;
         const double r = F.solve_radius(a.targets[t], ev);
         double p = nan;
         if (r == r) p = F.perimeter_at(r);
-        if (lane == 0) {
+        if (lead) {
             S.radii[t] = r;
             o[7 + t] = r;
             o[7 + nt + t] = p;
@@ -939,7 +971,7 @@ __global__ void __launch_bounds__(NT, 1024 / NT) k_source_metrics(MetricArgs a, 
     }
     __syncthreads();
     // supplementary samples between consecutive radii (lean_geometry.py:325-339)
-    for (int idx = warp; idx < ne; idx += nwarps) {
+    for (int idx = mine; idx < ne && mine < nteams; idx += nteams) {
         const int si = idx / m, j = idx - si * m;
         const double r0 = S.radii[si], r1 = S.radii[si + 1];
         double rr = nan, ar = nan;
@@ -947,9 +979,9 @@ __global__ void __launch_bounds__(NT, 1024 / NT) k_source_metrics(MetricArgs a, 
             rr = exp(log(r0) + a.fracs[j] * (log(r1) - log(r0)));
             double dA;
             F.area_at(rr, ar, dA);
-            if (lane == 0) atomicAdd(&S.n_eval, 1);
+            if (lead) atomicAdd(&S.n_eval, 1);
         }
-        if (lane == 0) {
+        if (lead) {
             o[7 + 2 * nt + idx] = rr;
             o[7 + 2 * nt + ne + idx] = ar;
         }
@@ -1010,14 +1042,19 @@ void launch_shift_stats_one(const MetricArgs& a, const double* phi, double* d, c
     k_shift_stats_one<<<a.ntiles, 256, 0, st>>>(a, phi, d);
 }
 
+constexpr int kTeamFaces = 65536;
 template <typename T>
 void launch_source_metrics(const MetricArgs& a, const T* dT, cudaStream_t st) {
     if (a.nsrc <= 0) return;
     // While there is an SM for each source, its binning, sort and targets spread over 32 warps instead of
     // waiting on 8 (64 sources at 147k vertices: 0.82 to 0.25 ms); then over 16 while two share an SM.
-    if (a.nsrc <= 148) k_source_metrics<T, 1024><<<a.nsrc, 1024, 0, st>>>(a, dT);
-    else if (a.nsrc <= 296) k_source_metrics<T, 512><<<a.nsrc, 512, 0, st>>>(a, dT);
-    else k_source_metrics<T, kMetricThreads><<<a.nsrc, kMetricThreads, 0, st>>>(a, dT);
+    // With 32 warps, several evaluate a target together where the bands are long enough to pay for the
+    // exchange: one source at 37k vertices (74k faces) 0.134 to 0.113 ms, at 147k 0.288 to 0.256, 64
+    // sources at 147k 0.310 to 0.293 (FP32 fields 0.249 to 0.227); 9k vertices equal, 2k 39 to 45 us.
+    if (a.nsrc <= 148 && a.nf >= kTeamFaces) k_source_metrics<T, 1024, true><<<a.nsrc, 1024, 0, st>>>(a, dT);
+    else if (a.nsrc <= 148) k_source_metrics<T, 1024, false><<<a.nsrc, 1024, 0, st>>>(a, dT);
+    else if (a.nsrc <= 296) k_source_metrics<T, 512, false><<<a.nsrc, 512, 0, st>>>(a, dT);
+    else k_source_metrics<T, kMetricThreads, false><<<a.nsrc, kMetricThreads, 0, st>>>(a, dT);
 }
 
 template void launch_shift_transpose<double, double>(int32_t, int32_t, const double*, const int32_t*, double*,

@@ -44,6 +44,32 @@ def test_metrics_match_oracle(mesh, count, scales):
             np.testing.assert_allclose(r["dist_b"][j], ref["dist_b"], rtol=tol)
 
 
+@pytest.fixture(scope="module")
+def large():
+    g = folded_icosphere(6, seed=4, jitter=0.1)
+    pm = M.prepare(g.vertices, g.faces, g.cortex_mask)
+    eng = engine.HeatEngine(pm.V, pm.F, block_k=512, pipeline_depth=1)
+    yield pm, eng
+    eng.close()
+
+
+@pytest.mark.parametrize("n_targets", [1, 4, 7, 8, 12, 15, 16, 32])
+def test_teams_match_one_warp_per_target(large, n_targets):
+    """A few sources on a large mesh evaluate each target with four, two or (from 16 targets) one warp;
+    a large block of the same sources takes a warp per target. Same bracket and Newton steps; sums differ
+    in order only (1e-9 relative, as above)."""
+    pm, eng = large
+    src = np.random.default_rng(n_targets).permutation(pm.n_vertices)[:400].astype(np.int32)
+    targets = pm.targets(np.geomspace(0.002, 0.1, n_targets))
+    for precision in ("fp64", "mixed"):
+        many = engine.split_records(eng.compute_metrics(src, targets, 3, precision=precision), n_targets, 3)
+        for few in (1, 9):
+            r = engine.split_records(eng.compute_metrics(src[:few], targets, 3, precision=precision), n_targets, 3)
+            for k in ("radii", "perim", "extra_r", "extra_a"):
+                np.testing.assert_allclose(r[k], many[k][:few], rtol=1e-9, err_msg=f"{precision} {k}")
+            assert np.array_equal(r["n_eval"], many["n_eval"][:few])
+
+
 def test_far_from_the_origin():
     """The chord test's FP32 form must not decide where the coordinates' magnitude swamps it: health
     counts on a mesh moved 1e6 mm away are the oracle's."""
