@@ -45,14 +45,14 @@ L2_BYTES = 126 * 1024 * 1024
 # DRAM bytes (read + write) per 1024-source block of each stage, mixed precision, from one
 # ncu capture on the small L6 workload (36,866 cortical vertices; about 3.5 GB on the device):
 #   ncu --metrics gpu__time_duration.sum,dram__bytes_read.sum,dram__bytes_write.sum --clock-control none
-#       -c 90 -k 'regex:^k_(fwd|bwd|div_mixed|shift_stats|source_metrics|reach)$' --csv
+#       -c 90 -k 'regex:^k_(fwd|bwd|leaf|assemble|div_mixed|shift_stats|source_metrics|reach)' --csv
 #       python bench.py --workload L6 --batch 1024 --steps 1 --warmup 3 --quick --cpu-sample 0 --pipeline-depth 1
 # (the first block's launches). Every stage moves n x K right-hand-side rows, so other meshes
 # report these bytes scaled by their vertex count (n / 36,866), labelled as scaled.
 TRAFFIC_L6_N = 36866
 TRAFFIC_L6 = {
-    "heat_fwd": 0.0720e9, "heat_bwd": 0.4775e9, "divergence": 0.4658e9, "poisson_fwd": 0.5230e9,
-    "poisson_bwd": 0.3583e9, "shift": 0.2889e9, "metrics": 0.4322e9,
+    "heat_fwd": 0.0238e9, "heat_bwd": 0.4266e9, "divergence": 0.4471e9, "poisson_fwd": 0.5107e9,
+    "poisson_bwd": 0.3629e9, "shift": 0.2749e9, "metrics": 0.3973e9,
 }
 
 
