@@ -1480,7 +1480,10 @@ int fcw_compute_distances(fcw_engine* e, const int32_t* sources, int64_t n, int3
         const int32_t K = round_k(nb);
         FCW_TRY(ensure_workspace(e, K, e->cw().out_stride));
         if (e->hcap_dist < nb * nv) {
-            if (e->hdist_d) e->release(e->hdist_d);
+            if (e->hdist_d) {
+                e->release(e->hdist_d);
+                for (Workspace& w : e->pool) w.drop_graph();  // captured chains write the old buffer
+            }
             e->hdist_d = nullptr;
             FCW_TRY(e->dalloc(&e->hdist_d, (size_t)(nb * nv)));
             e->hcap_dist = nb * nv;
