@@ -92,11 +92,12 @@ def check_interior_nonmanifold(pm, engine_type="b200", allow=False):
 
 
 def _plain_integers(values):
-    """values as an int64 array when it is a list, tuple or array of integers, else None."""
-    if isinstance(values, np.ndarray):
+    """values as an int64 array when it is a list, tuple or array of integers, else None. Subclasses may
+    iterate as something else (a masked array's masked elements are not integers): None."""
+    if type(values) is np.ndarray:
         ok = values.ndim == 1 and values.dtype.kind == "i"
         return values.astype(np.int64) if ok else None
-    if isinstance(values, (list, tuple)) and set(map(type, values)) <= {int}:
+    if type(values) in (list, tuple) and set(map(type, values)) <= {int}:
         try:
             return np.array(values, dtype=np.int64)
         except OverflowError:
