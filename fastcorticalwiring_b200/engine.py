@@ -168,10 +168,12 @@ class HeatEngine:
         src = np.ascontiguousarray(sources, dtype=np.int32).reshape(-1)
         v = np.ascontiguousarray(vertices, dtype=np.int32).reshape(-1)
         t = np.ascontiguousarray(targets, dtype=np.float64).reshape(-1)
-        if v.size != src.size or maps.shape[0] != 3 + 2 * t.size or flags.size != maps.shape[1]:
+        if (v.size != src.size or maps.ndim != 2 or maps.shape[0] != 3 + 2 * t.size
+                or flags.shape != maps.shape[1:]):
             raise ValueError("sources, vertices, maps and flags do not fit together")
-        if not (maps.dtype == np.float32 and maps.flags.c_contiguous and flags.dtype == np.uint8):
-            raise ValueError("maps must be a contiguous float32 array and flags uint8")
+        for name, x, dtype in (("maps", maps, np.float32), ("flags", flags, np.uint8)):  # written in place
+            if not (x.dtype == dtype and x.flags.c_contiguous and x.flags.writeable):
+                raise ValueError(f"{name} must be a contiguous, writeable {np.dtype(dtype)} array")
         n, cap = src.size, _lib.samples_capacity(t.size, n_between)
         health = np.empty((2, n))
         radii, areas = np.empty((n, cap), np.float32), np.empty((n, cap), np.float32)
