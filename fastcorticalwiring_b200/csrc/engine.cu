@@ -21,6 +21,7 @@
 #include "fcw_b200.h"
 #include "fcw_internal.h"
 #include "kernels.cuh"
+#include "staging.h"
 
 namespace {
 
@@ -274,9 +275,9 @@ struct fcw_engine {
     int64_t hcap_src = 0, hcap_out = 0;
     float *hsr_d = nullptr, *hsa_d = nullptr;  // staging for the host-buffer sample assembly
     int32_t* hcnt_d = nullptr;
-    int64_t hcap_smp = 0, hcap_cnt = 0;
+    int64_t hcap_sr = 0, hcap_sa = 0, hcap_cnt = 0;
     unsigned char *hmap_d = nullptr, *hmap_h = nullptr;  // staging for the wiring maps: device, page-locked host
-    int64_t hcap_map = 0;
+    int64_t hcap_map_d = 0, hcap_map_h = 0;
     double* hdist_d = nullptr;  // staging for the host-buffer distances API (caller order)
     int64_t hcap_dist = 0;
     double analyze_ms = 0.0, factor_ms = 0.0;
@@ -333,6 +334,23 @@ struct fcw_engine {
                 allocs.erase(allocs.begin() + (long)i);
                 return;
             }
+    }
+    // Staging that grows: on the device, and page-locked on the host (its readers have been waited for).
+    template <typename T>
+    int grow(T*& p, int64_t& cap, int64_t need) {
+        return fcw::grow_staging(p, cap, need, [&](T** q, int64_t n) { return dalloc(q, (size_t)n); },
+                                 [&](T* q) { release(q); });
+    }
+    int grow_host(unsigned char*& p, int64_t& cap, int64_t need) {
+        return fcw::grow_staging(
+            p, cap, need,
+            [](unsigned char** q, int64_t n) -> int {
+                if (cudaHostAlloc(reinterpret_cast<void**>(q), (size_t)n, cudaHostAllocDefault) == cudaSuccess)
+                    return FCW_OK;
+                cudaGetLastError();
+                return fail(FCW_E_NOMEM, "page-locked allocation of " + std::to_string(n) + " bytes failed");
+            },
+            [](unsigned char* q) { cudaFreeHost(q); });
     }
     ~fcw_engine() {
         sync_streams();
@@ -1479,15 +1497,11 @@ int fcw_compute_distances(fcw_engine* e, const int32_t* sources, int64_t n, int3
         const int64_t nb = std::min<int64_t>(Kmax, n - b0);
         const int32_t K = round_k(nb);
         FCW_TRY(ensure_workspace(e, K, e->cw().out_stride));
-        if (e->hcap_dist < nb * nv) {
-            if (e->hdist_d) {
-                e->release(e->hdist_d);
-                for (Workspace& w : e->pool) w.drop_graph();  // captured chains write the old buffer
-            }
-            e->hdist_d = nullptr;
-            FCW_TRY(e->dalloc(&e->hdist_d, (size_t)(nb * nv)));
-            e->hcap_dist = nb * nv;
+        if (e->hdist_d && e->hcap_dist < nb * nv) {
+            e->sync_streams();
+            for (Workspace& w : e->pool) w.drop_graph();  // captured chains write the old buffer
         }
+        FCW_TRY(e->grow(e->hdist_d, e->hcap_dist, nb * nv));
         Workspace& w = e->cw();
         FCW_CUDA(cudaMemcpyAsync(w.src, sources + b0, (size_t)nb * sizeof(int32_t), cudaMemcpyHostToDevice, w.stream));
         // the chain (solves, divergence, shift, fields back to the caller's order) as one graph
@@ -1783,18 +1797,8 @@ int fcw_compute_metrics(fcw_engine* e, const int32_t* sources, int64_t n, int32_
     FCW_TRY(check_sources(e, sources, n));
     if (n == 1 && precision == FCW_PREC_FP64) return narrow_metrics(e, sources[0], targets, nt, nb, eps, out_host);
     const int32_t stride = fcw_metrics_stride(nt, nb);
-    if (e->hcap_src < n) {
-        if (e->hsrc_d) e->release(e->hsrc_d);
-        e->hsrc_d = nullptr;
-        FCW_TRY(e->dalloc(&e->hsrc_d, (size_t)n));
-        e->hcap_src = n;
-    }
-    if (e->hcap_out < n * stride) {
-        if (e->hout_d) e->release(e->hout_d);
-        e->hout_d = nullptr;
-        FCW_TRY(e->dalloc(&e->hout_d, (size_t)n * stride));
-        e->hcap_out = n * stride;
-    }
+    FCW_TRY(e->grow(e->hsrc_d, e->hcap_src, n));
+    FCW_TRY(e->grow(e->hout_d, e->hcap_out, n * stride));
     FCW_CUDA(cudaMemcpyAsync(e->hsrc_d, sources, n * sizeof(int32_t), cudaMemcpyHostToDevice, e->stream));
     FCW_TRY(fcw_compute_metrics_device(e, e->hsrc_d, n, precision, targets, nt, nb, eps, e->hout_d, e->stream));
     FCW_CUDA(cudaMemcpyAsync(out_host, e->hout_d, n * stride * sizeof(double), cudaMemcpyDeviceToHost, e->stream));
@@ -1852,26 +1856,10 @@ int fcw_assemble_samples(fcw_engine* e, const double* records, int64_t n, int32_
     FCW_TRY(sample_args(records, n, n_targets, n_between, targets, boundary_cap, radii, areas, count, a));
     if (n == 0) return FCW_OK;
     const int64_t stride = a.stride, cap = a.capacity;
-    if (e->hcap_out < n * stride) {
-        if (e->hout_d) e->release(e->hout_d);
-        e->hout_d = nullptr;
-        FCW_TRY(e->dalloc(&e->hout_d, (size_t)(n * stride)));
-        e->hcap_out = n * stride;
-    }
-    if (e->hcap_smp < n * cap) {
-        if (e->hsr_d) e->release(e->hsr_d);
-        if (e->hsa_d) e->release(e->hsa_d);
-        e->hsr_d = e->hsa_d = nullptr;
-        FCW_TRY(e->dalloc(&e->hsr_d, (size_t)(n * cap)));
-        FCW_TRY(e->dalloc(&e->hsa_d, (size_t)(n * cap)));
-        e->hcap_smp = n * cap;
-    }
-    if (e->hcap_cnt < n) {
-        if (e->hcnt_d) e->release(e->hcnt_d);
-        e->hcnt_d = nullptr;
-        FCW_TRY(e->dalloc(&e->hcnt_d, (size_t)n));
-        e->hcap_cnt = n;
-    }
+    FCW_TRY(e->grow(e->hout_d, e->hcap_out, n * stride));
+    FCW_TRY(e->grow(e->hsr_d, e->hcap_sr, n * cap));
+    FCW_TRY(e->grow(e->hsa_d, e->hcap_sa, n * cap));
+    FCW_TRY(e->grow(e->hcnt_d, e->hcap_cnt, n));
     FCW_CUDA(cudaMemcpyAsync(e->hout_d, records, n * stride * sizeof(double), cudaMemcpyHostToDevice, e->stream));
     a.records = e->hout_d;
     a.radii_out = e->hsr_d;
@@ -1905,27 +1893,10 @@ int fcw_compute_wiring(fcw_engine* e, const int32_t* sources, int64_t n, int32_t
     const int64_t per = 2 * (int64_t)sizeof(double) + (cols + 2 * cap) * (int64_t)sizeof(float) + (int64_t)sizeof(int32_t) + 1;
     for (int64_t b0 = 0; b0 < n; b0 += kMapChunk) {
         const int64_t m = std::min(kMapChunk, n - b0), bytes = m * per;
-        if (e->hcap_src < m) {
-            if (e->hsrc_d) e->release(e->hsrc_d);
-            e->hsrc_d = nullptr;
-            FCW_TRY(e->dalloc(&e->hsrc_d, (size_t)m));
-            e->hcap_src = m;
-        }
-        if (e->hcap_out < m * stride) {
-            if (e->hout_d) e->release(e->hout_d);
-            e->hout_d = nullptr;
-            FCW_TRY(e->dalloc(&e->hout_d, (size_t)(m * stride)));
-            e->hcap_out = m * stride;
-        }
-        if (e->hcap_map < bytes) {
-            if (e->hmap_d) e->release(e->hmap_d);
-            if (e->hmap_h) cudaFreeHost(e->hmap_h);
-            e->hmap_d = e->hmap_h = nullptr;
-            e->hcap_map = 0;
-            FCW_TRY(e->dalloc(&e->hmap_d, (size_t)bytes));
-            FCW_CUDA(cudaHostAlloc(reinterpret_cast<void**>(&e->hmap_h), (size_t)bytes, cudaHostAllocDefault));
-            e->hcap_map = bytes;
-        }
+        FCW_TRY(e->grow(e->hsrc_d, e->hcap_src, m));
+        FCW_TRY(e->grow(e->hout_d, e->hcap_out, m * stride));
+        FCW_TRY(e->grow(e->hmap_d, e->hcap_map_d, bytes));
+        FCW_TRY(e->grow_host(e->hmap_h, e->hcap_map_h, bytes));
         // health (2m doubles), maps, sample rows, counts, flags
         auto at = [&](unsigned char* base, int part) {
             const int64_t off[] = {0, 16 * m, 16 * m + 4 * cols * m, 16 * m + 4 * (cols + cap) * m,
