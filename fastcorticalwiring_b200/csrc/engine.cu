@@ -1034,11 +1034,12 @@ void sweep(fcw_engine* e, fcw::SweepArgs<T> a, const T* fwd, const T* bwd, const
     a.tasks = e->fwd_tasks;
     a.panel = fwd;
     for (int32_t l = 0; l < f.nlevels; ++l) {
-        const bool wide = l >= f.first_wide;
+        const bool wide = l >= f.first_wide, overlap = l > 0 || !a.reach;
         a.gathers = l > 0;
-        if (wide) fcw::launch_assemble<T>(a, f.asm_ptr[l], f.asm_ptr[l + 1] - f.asm_ptr[l], st);
+        if (wide) fcw::launch_assemble<T>(a, f.asm_ptr[l], f.asm_ptr[l + 1] - f.asm_ptr[l], overlap, st);
         if (l == 0 && !wide && fcw::launch_leaves<T>(a, false, f.fwd_ptr[1], f.fwd_rows[0], leaf_f, 0, st)) continue;
-        fcw::launch_fwd_level<T>(a, f.fwd_ptr[l], f.fwd_ptr[l + 1] - f.fwd_ptr[l], f.fwd_rows[l], wide, st);
+        fcw::launch_fwd_level<T>(a, f.fwd_ptr[l], f.fwd_ptr[l + 1] - f.fwd_ptr[l], f.fwd_rows[l], wide, wide || overlap,
+                                 st);
     }
     a.delta_src = nullptr;
     mark(e, st, stage_bwd);

@@ -115,10 +115,13 @@ cudaError_t configure_solve_kernels();
 int32_t max_front_rows();  // the backward sweep holds a front's row list in shared memory
 // One level of the forward sweep: tasks [t0, t0 + ntasks) of `rows` rows; wide: the level's
 // right-hand sides have been assembled (launch_assemble, rows [r0, r0 + nrows) of asm_rows).
+// overlap: the kernel may start before the stream's previous one is complete. Not for the first kernel
+// after launch_reach: later ones read the reach flags before they wait.
 template <typename T>
-void launch_fwd_level(const SweepArgs<T>& a, int32_t t0, int32_t ntasks, int32_t rows, bool wide, cudaStream_t st);
+void launch_fwd_level(const SweepArgs<T>& a, int32_t t0, int32_t ntasks, int32_t rows, bool wide, bool overlap,
+                      cudaStream_t st);
 template <typename T>
-void launch_assemble(const SweepArgs<T>& a, int32_t r0, int32_t nrows, cudaStream_t st);
+void launch_assemble(const SweepArgs<T>& a, int32_t r0, int32_t nrows, bool overlap, cudaStream_t st);
 // One level of the backward sweep; max_depth: the most front rows a task multiplies.
 template <typename T>
 void launch_bwd_level(const SweepArgs<T>& a, int32_t t0, int32_t ntasks, int32_t rows, int32_t max_depth,

@@ -30,11 +30,15 @@
 // the triangles of inv(L_ss) are cut at 16.
 //
 // Launches overlap: a level's CTAs read their task, request their panels and load their gather lists
-// while the previous level finishes (programmatic dependent launch), then wait for it.
+// while the previous level finishes (programmatic dependent launch), then wait for it. Every sweep
+// kernel lets its dependents start before its own wait, so a chain of them may have started while the
+// first still waits: what a kernel reads before its wait has to be complete before the chain begins.
 //
 // Heat right-hand sides are columns of the identity: the forward sweep builds them from the source
 // list, and only fronts on a source's path to the root (`reach`, per front and 64-column tile) are
-// solved; the others' forward results are zero and are not read.
+// solved; the others' forward results are zero and are not read. The backward sweep reads `reach` before
+// its wait (which rows of the panel to request follows from it), so the chain's first kernel is launched
+// in order after k_reach, without overlap; it would wait for `reach` before all else anyway.
 #include <algorithm>
 #include <type_traits>
 
@@ -505,7 +509,7 @@ __global__ void __launch_bounds__(NT, 3) k_bwd(SweepArgs<T> a, int32_t t0) {
     const int tid = threadIdx.x, tile = blockIdx.y, k0 = tile * KT;
     const SweepTask t = a.tasks[t0 + blockIdx.x];
     const int own = t.ns - t.r0;  // depth rows [0, own): y_s; then the structure rows
-    // y_s = 0 off the sources' paths (reach was written launches ago: the forward sweep has read it)
+    // y_s = 0 off the sources' paths (reach is complete before the chain of overlapped launches begins)
     const int d0 = (a.reach && !reached(a, t.front, tile)) ? own : 0;
     const int ld = panel_stride<T>(t.h);
     const T* panel = a.panel + (sizeof(T) == 8 ? t.off64 : t.off32);
@@ -823,10 +827,10 @@ constexpr int64_t kLeafCtas = 2368;               // eight waves of them
 constexpr int64_t kLeafRounds = 1184, kLeafRoundsReach = 5920;
 constexpr size_t kSmemMax = 227 * 1024 - 4096;  // static shared memory is kept apart
 
-// A launch that may start while the stream's previous kernel finishes; its reads of that kernel's
+// overlap: the launch may start while the stream's previous kernel finishes; its reads of that kernel's
 // results come after griddepcontrol.wait.
 template <typename Kern, typename... Args>
-void launch_overlapped(Kern kern, dim3 grid, size_t smem, cudaStream_t st, Args... args) {
+void launch_sweep(Kern kern, dim3 grid, size_t smem, bool overlap, cudaStream_t st, Args... args) {
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = grid;
     cfg.blockDim = dim3(NT);
@@ -836,7 +840,7 @@ void launch_overlapped(Kern kern, dim3 grid, size_t smem, cudaStream_t st, Args.
     at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
     at[0].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = at;
-    cfg.numAttrs = 1;
+    cfg.numAttrs = overlap ? 1 : 0;
     cudaLaunchKernelEx(&cfg, kern, args...);
 }
 
@@ -859,18 +863,18 @@ cudaError_t set_smem() {
 }
 
 template <typename T, int KT>
-void fwd_tile(const SweepArgs<T>& a, int32_t t0, int32_t n, int32_t rows, bool wide, cudaStream_t st) {
+void fwd_tile(const SweepArgs<T>& a, int32_t t0, int32_t n, int32_t rows, bool wide, bool overlap, cudaStream_t st) {
     const dim3 grid(n, a.K / KT);
-    if (!wide && rows == 128) launch_overlapped(k_fwd<T, KT, 128, false>, grid, fwd_smem<T, KT, 128>(), st, a, t0);
-    else if (!wide) launch_overlapped(k_fwd<T, KT, 64, false>, grid, fwd_smem<T, KT, 64>(), st, a, t0);
-    else if (rows == 64) launch_overlapped(k_fwd<T, KT, 64, true>, grid, fwd_smem<T, KT, 64>(), st, a, t0);
-    else launch_overlapped(k_fwd<T, KT, 32, true>, grid, fwd_smem<T, KT, 32>(), st, a, t0);
+    if (!wide && rows == 128) launch_sweep(k_fwd<T, KT, 128, false>, grid, fwd_smem<T, KT, 128>(), overlap, st, a, t0);
+    else if (!wide) launch_sweep(k_fwd<T, KT, 64, false>, grid, fwd_smem<T, KT, 64>(), overlap, st, a, t0);
+    else if (rows == 64) launch_sweep(k_fwd<T, KT, 64, true>, grid, fwd_smem<T, KT, 64>(), overlap, st, a, t0);
+    else launch_sweep(k_fwd<T, KT, 32, true>, grid, fwd_smem<T, KT, 32>(), overlap, st, a, t0);
 }
 template <typename T, int KT>
 void bwd_tile(const SweepArgs<T>& a, int32_t t0, int32_t n, int32_t rows, int32_t max_depth, cudaStream_t st) {
     const dim3 grid(n, a.K / KT);
-    if (rows == 64) launch_overlapped(k_bwd<T, KT, 64>, grid, bwd_smem<T, KT, 64>(max_depth), st, a, t0);
-    else launch_overlapped(k_bwd<T, KT, 32>, grid, bwd_smem<T, KT, 32>(max_depth), st, a, t0);
+    if (rows == 64) launch_sweep(k_bwd<T, KT, 64>, grid, bwd_smem<T, KT, 64>(max_depth), true, st, a, t0);
+    else launch_sweep(k_bwd<T, KT, 32>, grid, bwd_smem<T, KT, 32>(max_depth), true, st, a, t0);
 }
 // The leaf level with its panels resident, where two CTAs fit an SM; false: not taken.
 template <typename T, int M, bool BACK>
@@ -884,13 +888,13 @@ bool leaf_groups(const SweepArgs<T>& a, int32_t n, int32_t panel, int32_t max_de
     const int want = (int)std::max<int64_t>(1, std::min<int64_t>(rounds, (int64_t)n * rounds / kLeafCtas));
     const int ny = (rounds + want - 1) / want, per = W * ((rounds + ny - 1) / ny);
     const int groups = a.K / A::CW;
-    launch_overlapped(k_leaf<T, M, BACK>, dim3(n, (groups + per - 1) / per), smem, st, a, per, panel);
+    launch_sweep(k_leaf<T, M, BACK>, dim3(n, (groups + per - 1) / per), smem, true, st, a, per, panel);
     return true;
 }
 template <typename T, int KT>
-void asm_tile(const SweepArgs<T>& a, int32_t r0, int32_t n, cudaStream_t st) {
+void asm_tile(const SweepArgs<T>& a, int32_t r0, int32_t n, bool overlap, cudaStream_t st) {
     constexpr int RPP = NT / (KT / vec<T>());
-    launch_overlapped(k_assemble<T, KT>, dim3((n + RPP - 1) / RPP, a.K / KT), 0, st, a, r0, n);
+    launch_sweep(k_assemble<T, KT>, dim3((n + RPP - 1) / RPP, a.K / KT), 0, overlap, st, a, r0, n);
 }
 
 }  // namespace
@@ -905,11 +909,12 @@ cudaError_t configure_solve_kernels() {
 int32_t max_front_rows() { return (int32_t)((kSmemMax - bwd_smem<double, 64, 64>(0)) / sizeof(int32_t)); }
 
 template <typename T>
-void launch_fwd_level(const SweepArgs<T>& a, int32_t t0, int32_t ntasks, int32_t rows, bool wide, cudaStream_t st) {
+void launch_fwd_level(const SweepArgs<T>& a, int32_t t0, int32_t ntasks, int32_t rows, bool wide, bool overlap,
+                      cudaStream_t st) {
     if (ntasks <= 0 || a.K <= 0) return;
     constexpr int W = wide_tile<T>();
-    if (W != 64 && a.K % W == 0) fwd_tile<T, W>(a, t0, ntasks, rows, wide, st);
-    else fwd_tile<T, 64>(a, t0, ntasks, rows, wide, st);
+    if (W != 64 && a.K % W == 0) fwd_tile<T, W>(a, t0, ntasks, rows, wide, overlap, st);
+    else fwd_tile<T, 64>(a, t0, ntasks, rows, wide, overlap, st);
 }
 template <typename T>
 bool launch_leaves(const SweepArgs<T>& a, bool back, int32_t ntasks, int32_t rows, int32_t panel, int32_t max_depth,
@@ -920,11 +925,11 @@ bool launch_leaves(const SweepArgs<T>& a, bool back, int32_t ntasks, int32_t row
     return false;
 }
 template <typename T>
-void launch_assemble(const SweepArgs<T>& a, int32_t r0, int32_t nrows, cudaStream_t st) {
+void launch_assemble(const SweepArgs<T>& a, int32_t r0, int32_t nrows, bool overlap, cudaStream_t st) {
     if (nrows <= 0 || a.K <= 0) return;
     constexpr int W = wide_tile<T>();
-    if (W != 64 && a.K % W == 0) asm_tile<T, W>(a, r0, nrows, st);
-    else asm_tile<T, 64>(a, r0, nrows, st);
+    if (W != 64 && a.K % W == 0) asm_tile<T, W>(a, r0, nrows, overlap, st);
+    else asm_tile<T, 64>(a, r0, nrows, overlap, st);
 }
 template <typename T>
 void launch_bwd_level(const SweepArgs<T>& a, int32_t t0, int32_t ntasks, int32_t rows, int32_t max_depth,
@@ -943,8 +948,8 @@ void launch_reach(const int32_t* col_front, const int32_t* parent, int32_t nfron
 }
 
 #define FCW_SWEEPS(T)                                                                                           \
-    template void launch_fwd_level<T>(const SweepArgs<T>&, int32_t, int32_t, int32_t, bool, cudaStream_t);      \
-    template void launch_assemble<T>(const SweepArgs<T>&, int32_t, int32_t, cudaStream_t);                      \
+    template void launch_fwd_level<T>(const SweepArgs<T>&, int32_t, int32_t, int32_t, bool, bool, cudaStream_t); \
+    template void launch_assemble<T>(const SweepArgs<T>&, int32_t, int32_t, bool, cudaStream_t);                \
     template bool launch_leaves<T>(const SweepArgs<T>&, bool, int32_t, int32_t, int32_t, int32_t, cudaStream_t); \
     template void launch_bwd_level<T>(const SweepArgs<T>&, int32_t, int32_t, int32_t, int32_t, cudaStream_t);
 FCW_SWEEPS(double)
