@@ -27,3 +27,21 @@ def test_fields_after_a_larger_call(precision):
         assert np.array_equal(eng.compute_distances(other, precision=precision), a)
     finally:
         eng.close()
+
+
+@pytest.mark.parametrize("count", [2, 63, 65, 1000, 2049, 4096])
+def test_sources_sorted_in_place(count):
+    """The host-buffer call sorts its sources where they were copied to, up to the largest block: every
+    field is the one its source has alone."""
+    g = folded_icosphere(2, seed=2, jitter=0.1)
+    pm = M.prepare(g.vertices, g.faces, g.cortex_mask)
+    src = np.random.default_rng(count).integers(0, pm.n_vertices, count).astype(np.int32)
+    eng = engine.HeatEngine(pm.V, pm.F, block_k=4096, pipeline_depth=1)
+    try:
+        alone = eng.compute_distances(np.arange(pm.n_vertices, dtype=np.int32), precision="fp64")
+        d = eng.compute_distances(src, precision="fp64")
+        # a column's sums do not depend on the block it is in, but the kernels' split of a block may
+        assert np.max(np.abs(d - alone[src])) <= 1e-12 * np.max(np.abs(alone))
+        assert np.array_equal(d[np.arange(count), src], np.zeros(count))
+    finally:
+        eng.close()
