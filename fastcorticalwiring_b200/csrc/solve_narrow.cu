@@ -46,6 +46,7 @@ constexpr int kTaskDoubles = kNarrowTaskDoubles;  // panel data of one task (88 
 constexpr int kMaxRows = 192, kSplitTo = 64;      // rows of a whole-front task; of a split front's
 constexpr int kMaxCols = 64, kSplitDepth = 256;   // columns of a strip; fronts deeper than this are split
 constexpr uint64_t kWaitNs = 1000000000ull;
+constexpr int kSmemMax = 227 * 1024 - 16;         // dynamic shared memory of a CTA; 16 bytes are static
 
 constexpr long long kPending = -1;  // bit pattern of an entry not yet written
 
@@ -396,13 +397,13 @@ cudaError_t configure_narrow_kernels(int max_ns, int max_m, int num_sms, NarrowL
     L->fwd_smem = fwd_bytes(max_ns);
     L->bwd_smem = bwd_bytes(max_m);
     L->strip = strip_doubles(max_m);
-    if (L->fwd_smem > 227 * 1024 || L->bwd_smem > 227 * 1024) return cudaErrorInvalidValue;
-    cudaError_t e = cudaFuncSetAttribute(k_fwd_tasks<true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                         (int)L->fwd_smem);
+    if (L->fwd_smem > kSmemMax || L->bwd_smem > kSmemMax) return cudaErrorInvalidValue;
+    // the same allowance for every engine: it belongs to the kernel, and engines of other sizes launch it too
+    cudaError_t e = cudaFuncSetAttribute(k_fwd_tasks<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemMax);
     if (e == cudaSuccess)
-        e = cudaFuncSetAttribute(k_fwd_tasks<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)L->fwd_smem);
+        e = cudaFuncSetAttribute(k_fwd_tasks<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemMax);
     if (e == cudaSuccess)
-        e = cudaFuncSetAttribute(k_bwd_tasks, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)L->bwd_smem);
+        e = cudaFuncSetAttribute(k_bwd_tasks, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemMax);
     int per_sm = 0;
     if (e == cudaSuccess)
         e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_fwd_tasks<false>, NTN, L->fwd_smem);
