@@ -19,6 +19,7 @@ include/fcw_b200.h), in the order of the job's sources.
 
 from __future__ import annotations
 
+import math
 import threading
 import time
 from collections import deque
@@ -93,16 +94,20 @@ def _stride(nt, nb):
 
 
 def estimate_device_bytes(n_vertices: int, n_faces: int, block_k: int, pipeline_depth: int, n_sources: int,
-                          stride: int) -> int:
+                          stride: int, tc_sweeps: int = 0, refine: int = 0, leaf_size: int = 64) -> int:
     """Upper estimate of a job's device memory before it is factored.
 
-    Per workspace and right-hand side about 100 bytes per vertex (four FP64 n x K
-    arrays, the near-vertex lists, the update rows at ~2.65 n, and the per-source
-    face band of 20 bytes per face), plus factors and mesh arrays (~3 KB per
-    vertex at these fills) and the job's source list and result records.
+    Per workspace and right-hand side about 87 bytes per vertex (four FP64 n x K arrays, the near-vertex
+    lists, 1.1 to 1.4 n update and assembled rows, more with narrow supernodes, and the per-source face
+    band of 20 bytes per face), 60 + 20 per face allowed. Factors and mesh arrays take 7.1 KB per vertex
+    at 2.3k vertices, 8.7 KB at 147k and 9.1 KB at 590k: each factor's blocks and its forward and
+    backward panels, two factors in FP64 and one in FP32. The tensor-core sweeps add their core arrays
+    and per-supernode update rows. Then the job's source list and result records.
     """
-    ws = int(block_k) * (n_vertices * 60 + n_faces * 20 + int(2.65 * n_vertices * 8) + stride * 8)
-    return pipeline_depth * ws + 3000 * n_vertices + n_sources * (4 + stride * 8) + (64 << 20)
+    ws = int(block_k) * (n_vertices * (75 if tc_sweeps else 60) + n_faces * 20 + stride * 8)
+    factors = (4000 + 300 * math.log2(max(int(n_vertices), 2))) * (1.25 if leaf_size > 64 else 1.0)
+    factors += (2800 if tc_sweeps else 0) + (100 if refine else 0)
+    return pipeline_depth * ws + int(factors * n_vertices) + n_sources * (4 + stride * 8) + (64 << 20)
 
 
 class Server:
@@ -256,8 +261,9 @@ class Server:
             job = p.job
             nv = int(np.count_nonzero(job.cortex_mask))
             nsrc = nv if job.sources is None else int(np.asarray(job.sources).size)
+            opts = {k: self.params[k] for k in ("tc_sweeps", "refine", "leaf_size") if k in self.params}
             p.estimate = estimate_device_bytes(nv, 2 * nv, self.params["block_k"], self.params["pipeline_depth"],
-                                               nsrc, _stride(len(job.scales), job.n_between))
+                                               nsrc, _stride(len(job.scales), job.n_between), **opts)
         return p.estimate
 
     def _pick(self):
