@@ -65,4 +65,27 @@ struct Fronts {
 
 int build_fronts(const Symbolic& S, Fronts& f, std::string& err);
 
+// The leaf level with resident panels (k_leaf, solve.cu): a CTA's warps, a warp's ring of right-hand
+// sides (chunks, depth rows per chunk), the columns of a warp's groups, and the shared memory of a CTA,
+// of which two fit an SM.
+constexpr int kLeafWarps = 8, kLeafStages = 3, kLeafChunk = 16;
+constexpr size_t kLeafSmem = 113 * 1024 - 1024;
+constexpr int leaf_columns(bool fp64, bool back) { return !fp64 ? 32 : (back ? 16 : 8); }
+// panel: entries of the largest task's panel; index_rows: rows whose indices a backward CTA holds
+inline size_t leaf_smem(int64_t panel, int columns, size_t entry, int32_t index_rows) {
+    return ((size_t)panel + (size_t)kLeafWarps * kLeafStages * kLeafChunk * columns) * entry +
+           (size_t)index_rows * sizeof(int32_t);
+}
+// Least tasks times column rounds (a warp's groups) for which k_leaf is the faster: with fewer, its
+// CTAs, each with all of a panel to fetch first, do not fill the chip. 147k vertices FP64, backward:
+// 2066 rounds (128 columns) 0.324 against 0.334 ms, 16528 (1024) 1.36 against 1.48; 37k vertices: 1038
+// rounds equal, 2076 0.241 against 0.245; 9k vertices, forward: 2096 0.160 against 0.163, 131 0.069
+// against 0.064. With reach flags rounds differ in length, so more are needed: 147k vertices 16528
+// 1.04 against 1.11 ms, 8264 0.612 against 0.633, 4132 0.403 against 0.400; 37k vertices 4152 0.306
+// against 0.297.
+constexpr int64_t kLeafRounds = 1184, kLeafRoundsReach = 5920;
+inline bool leaves_resident(int64_t tasks, int rounds, size_t smem, bool reach) {
+    return smem <= kLeafSmem && tasks * rounds >= (reach ? kLeafRoundsReach : kLeafRounds);
+}
+
 }  // namespace fcw

@@ -581,7 +581,8 @@ __global__ void __launch_bounds__(NT, 3) k_bwd(SweepArgs<T> a, int32_t t0) {
 // slot). Bound by issue around the matrix instructions (tensor pipe 60-66% busy). Poisson forward 2.12 to 1.96 ms and
 // backward 1.48 to 1.36, heat backward 1.11 to 1.04; FP32 backward 1.12 to 1.08. FP32 forward takes the
 // general kernel: more shared-memory reads per product here, 1.54 against 1.44 ms.
-constexpr int kLeafStages = 3, LD = 16;  // a warp's ring: chunks, depth rows per chunk
+constexpr int LD = kLeafChunk;  // depth rows per chunk of a warp's ring
+static_assert(kLeafWarps == NT / 32, "the plan's warps are the kernel's");
 
 // Products of one warp: C (h rows x CW columns) += P V, P k-major in the CTA's panel, V the warp's own
 // [depth][CW] rows. Row tiles are numbered so that the ones a depth reaches are the last: forward, the
@@ -815,16 +816,7 @@ template <typename T, int KT, int M>
 size_t bwd_smem(int max_depth) {
     return (size_t)kBwdStages * (panel_stage<T, M>() + DC * ld_rhs<T, KT>()) * sizeof(T) + (size_t)max_depth * sizeof(int32_t);
 }
-constexpr size_t kLeafSmem = 113 * 1024 - 1024;  // of two CTAs per SM
-constexpr int64_t kLeafCtas = 2368;               // eight waves of them
-// Least tasks times column rounds (a warp's groups) for which k_leaf is the faster: with fewer, its
-// CTAs, each with all of a panel to fetch first, do not fill the chip. 147k vertices FP64, backward:
-// 2066 rounds (128 columns) 0.324 against 0.334 ms, 16528 (1024) 1.36 against 1.48; 37k vertices: 1038
-// rounds equal, 2076 0.241 against 0.245; 9k vertices, forward: 2096 0.160 against 0.163, 131 0.069
-// against 0.064. With reach flags rounds differ in length, so more are needed: 147k vertices 16528
-// 1.04 against 1.11 ms, 8264 0.612 against 0.633, 4132 0.403 against 0.400; 37k vertices 4152 0.306
-// against 0.297.
-constexpr int64_t kLeafRounds = 1184, kLeafRoundsReach = 5920;
+constexpr int64_t kLeafCtas = 2368;               // eight waves of two CTAs per SM
 constexpr size_t kSmemMax = 227 * 1024 - 4096;  // static shared memory is kept apart
 
 // overlap: the launch may start while the stream's previous kernel finishes; its reads of that kernel's
@@ -880,11 +872,11 @@ void bwd_tile(const SweepArgs<T>& a, int32_t t0, int32_t n, int32_t rows, int32_
 template <typename T, int M, bool BACK>
 bool leaf_groups(const SweepArgs<T>& a, int32_t n, int32_t panel, int32_t max_depth, cudaStream_t st) {
     using A = WarpAcc<T, M, BACK>;
-    constexpr int W = NT / 32;
-    const size_t smem = ((size_t)panel + W * kLeafStages * LD * A::CW) * sizeof(T) +
-                        (BACK ? (size_t)max_depth * sizeof(int32_t) : 0);
+    constexpr int W = kLeafWarps;
+    static_assert(A::CW == leaf_columns(sizeof(T) == 8, BACK), "the plan's column groups are the kernel's");
+    const size_t smem = leaf_smem(panel, A::CW, sizeof(T), BACK ? max_depth : 0);
     const int rounds = a.K / A::CW / W;  // column groups per warp, were a CTA to take them all
-    if (smem > kLeafSmem || (int64_t)n * rounds < (a.reach ? kLeafRoundsReach : kLeafRounds)) return false;
+    if (!leaves_resident(n, rounds, smem, a.reach != nullptr)) return false;
     const int want = (int)std::max<int64_t>(1, std::min<int64_t>(rounds, (int64_t)n * rounds / kLeafCtas));
     const int ny = (rounds + want - 1) / want, per = W * ((rounds + ny - 1) / ny);
     const int groups = a.K / A::CW;
