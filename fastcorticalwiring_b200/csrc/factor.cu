@@ -26,11 +26,6 @@ __global__ void k_scatter_a(int64_t nnz, const int64_t* __restrict__ dst, const 
         val[dst[e]] = aval[e];
 }
 
-__global__ void k_to_float(int64_t n, const double* __restrict__ s, float* __restrict__ d) {
-    for (int64_t e = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; e < n; e += (int64_t)gridDim.x * blockDim.x)
-        d[e] = (float)s[e];
-}
-
 __global__ void __launch_bounds__(256) k_factor_front(DevPlan p, int32_t l0, double* __restrict__ val,
                                                       double* __restrict__ inv, double* __restrict__ upd,
                                                       int* __restrict__ err) {
@@ -220,13 +215,6 @@ void launch_scatter_a(int64_t nnz, const int64_t* dst, const double* aval, doubl
     int blocks = (int)((nnz + 255) / 256);
     if (blocks > 148 * 16) blocks = 148 * 16;
     k_scatter_a<<<blocks, 256, 0, st>>>(nnz, dst, aval, val);
-}
-
-void launch_to_float(int64_t n, const double* src, float* dst, cudaStream_t st) {
-    if (n <= 0) return;
-    int blocks = (int)((n + 255) / 256);
-    if (blocks > 148 * 16) blocks = 148 * 16;
-    k_to_float<<<blocks, 256, 0, st>>>(n, src, dst);
 }
 
 void launch_factor_front(const DevPlan& p, int32_t l0, int32_t count, double* val, double* inv, double* upd,

@@ -22,7 +22,6 @@ enum : int {
 };
 
 constexpr int kMaxWidth = 64;      // widest supernode the dense kernels accept
-constexpr int kSlice = 32;         // right-hand sides per CTA column slice (one per lane)
 constexpr int kMaxBins = 2048;     // distance bins per source held in shared memory
 constexpr int kMaxTargets = 32;
 constexpr int kMaxBetween = 8;
@@ -58,7 +57,6 @@ void launch_factor_front(const DevPlan& p, int32_t l0, int32_t count, double* va
 // one level: update matrices U -= L21 L21^T
 void launch_factor_update(const DevPlan& p, int32_t l0, int32_t count, int32_t max_tiles, const double* val,
                           double* upd, cudaStream_t st);
-void launch_to_float(int64_t n, const double* src, float* dst, cudaStream_t st);
 // after every level: each panel's L21 becomes Q = L21 L11^{-1} (what the solves read)
 void launch_panel_inverse(const DevPlan& p, double* val, const double* inv, cudaStream_t st);
 

@@ -76,7 +76,7 @@ __device__ __forceinline__ void gather_sub_swz(unsigned char* Tt, const float* S
     }
 }
 
-// gather_finish of solve.cu on the swizzled own-row tile (subtracting).
+// gather_finish of sweep_rows.cuh on the swizzled own-row tile (subtracting).
 __device__ __forceinline__ void gather_finish_swz(const SolveArgs<float>& a, const GatherRange& g, int k0,
                                                   unsigned char* Tt, int nrows, float* St,
                                                   const int* grs) {
