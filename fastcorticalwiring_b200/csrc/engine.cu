@@ -1943,7 +1943,7 @@ int fcw_assemble_samples(fcw_engine* e, const double* records, int64_t n, int32_
     return FCW_OK;
 }
 
-// The maps of up to kMapChunk sources at a time pass through page-locked staging (8.4 MB at 12 scales
+// The maps of up to kMapChunk sources at a time pass through page-locked staging (8.0 MB at 12 scales
 // and 3 samples between): records never leave the device, and the host only scatters float32 values.
 int fcw_compute_wiring(fcw_engine* e, const int32_t* sources, int64_t n, int32_t precision, const double* targets,
                        int32_t nt, int32_t nb, double eps, double boundary_cap, const int32_t* vertices, int64_t n_full,

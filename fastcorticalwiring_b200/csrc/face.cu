@@ -9,7 +9,7 @@
 // needs, so a first pass forms the scales (a warp takes four faces) and a second gathers them (a warp
 // per vertex, its faces in ascending order): 2.1x less FP64 work than evaluating each face at each of
 // its corners, for one 8-byte value per face and column through memory. 147k vertices,
-// 1024 columns: 4.76 to 3.26 ms, bound by the gathers' latency (FP64 pipe 40% busy).
+// 1024 columns: 4.76 to 3.26 ms, bound by the gathers' latency (FP64 pipe 45% busy).
 //
 // Mixed form: X = -grad u / |grad u| is invariant to scaling u's differences, so FP64 differences
 // scaled by a power of two (exact) are rounded to FP32 and the rest runs in FP32 in the intrinsic

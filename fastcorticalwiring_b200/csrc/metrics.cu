@@ -97,7 +97,7 @@ __device__ __forceinline__ Thresholds<T> thresholds(const MetricArgs& a) {
         return {-a.health_h, a.eps, a.near_radius};
 }
 
-// The shift + transpose of one kStatVTile-vertex x 32-source tile, fused with the per-vertex
+// The shift + transpose of one tile of a.vtile vertices (stat_tile) x 32 sources, fused with the per-vertex
 // work of the health screen and MSD (lean_geometry.py:343-357, core_analysis.py:1573-1581):
 // counts of d < -h and of d < 0.9 |x - x_s| - h, the valid-distance sums and the maximum.
 // The chord test runs in FP32 first: with E = a.chord_slack bounding the error of the FP32 straight
