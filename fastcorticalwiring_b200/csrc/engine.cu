@@ -18,6 +18,7 @@
 #include <string>
 #include <system_error>
 #include <type_traits>
+#include <utility>
 #include <vector>
 
 #include "fcw_b200.h"
@@ -554,6 +555,18 @@ struct MeshTables {
     fcw::PatchArrays patches;
 };
 
+// f on a thread of its own, or at once (an invalid future) when there is none to be had. The future
+// waits for its thread when it goes out of scope.
+template <class F>
+std::future<void> on_thread(F&& f) {
+    try {
+        return std::async(std::launch::async, std::forward<F>(f));
+    } catch (const std::system_error&) {
+        f();
+        return {};
+    }
+}
+
 void mesh_tables(const fcw::MeshPrep& m, const fcw::Symbolic& S, MeshTables& t) {
     const int64_t n = S.n, nf = m.nf;
     t.coords.resize(3 * n);
@@ -593,27 +606,31 @@ void mesh_tables(const fcw::MeshPrep& m, const fcw::Symbolic& S, MeshTables& t) 
     t.farea_fx.resize(nf);
     for (int64_t f = 0; f < nf; ++f) t.farea_fx[f] = std::llround(m.lean_area[f] * area_scale);
     t.area_unscale = 1.0 / area_scale;
-    fcw::face_fans(m, fv, inc_ptr, inc_face, inc_corner, t.fan_ptr, t.fan_steps, t.fan_walk);
     // FP64 divergence: faces in the order of their lowest vertices, with their corners and geometry
-    std::vector<int32_t> place(nf), start(n + 1, 0);
-    t.corners.resize(nf);
-    t.div_rec.resize(3 * nf);
-    t.geo.assign(8 * nf, 0.0);
-    for (int64_t f = 0; f < nf; ++f) start[std::min({fv[3 * f], fv[3 * f + 1], fv[3 * f + 2]}) + 1]++;
-    for (int64_t j = 0; j < n; ++j) start[j + 1] += start[j];
-    for (int64_t f = 0; f < nf; ++f) {
-        const int32_t p = start[std::min({fv[3 * f], fv[3 * f + 1], fv[3 * f + 2]})]++;
-        place[f] = p;
-        t.corners[p] = make_int4(fv[3 * f], fv[3 * f + 1], fv[3 * f + 2], 0);
-        for (int x = 0; x < 6; ++x) t.geo[8 * (int64_t)p + x] = m.gb[9 * f + 3 + x];
-        t.geo[8 * (int64_t)p + 6] = m.grad_area[f];
-    }
-    for (int64_t q = 0; q < 3 * nf; ++q) {
-        const int32_t f = inc_face[q];
-        t.div_rec[q] = make_int4(fv[3 * f], fv[3 * f + 1], fv[3 * f + 2],
-                                 place[f] | ((int32_t)inc_corner[q] << fcw::kIncCornerShift));
-    }
+    auto face_records = [&] {
+        std::vector<int32_t> place(nf), start(n + 1, 0);
+        t.corners.resize(nf);
+        t.div_rec.resize(3 * nf);
+        t.geo.assign(8 * nf, 0.0);
+        for (int64_t f = 0; f < nf; ++f) start[std::min({fv[3 * f], fv[3 * f + 1], fv[3 * f + 2]}) + 1]++;
+        for (int64_t j = 0; j < n; ++j) start[j + 1] += start[j];
+        for (int64_t f = 0; f < nf; ++f) {
+            const int32_t p = start[std::min({fv[3 * f], fv[3 * f + 1], fv[3 * f + 2]})]++;
+            place[f] = p;
+            t.corners[p] = make_int4(fv[3 * f], fv[3 * f + 1], fv[3 * f + 2], 0);
+            for (int x = 0; x < 6; ++x) t.geo[8 * (int64_t)p + x] = m.gb[9 * f + 3 + x];
+            t.geo[8 * (int64_t)p + 6] = m.grad_area[f];
+        }
+        for (int64_t q = 0; q < 3 * nf; ++q) {
+            const int32_t f = inc_face[q];
+            t.div_rec[q] = make_int4(fv[3 * f], fv[3 * f + 1], fv[3 * f + 2],
+                                     place[f] | ((int32_t)inc_corner[q] << fcw::kIncCornerShift));
+        }
+    };
+    std::future<void> records = on_thread(face_records);
+    fcw::face_fans(m, fv, inc_ptr, inc_face, inc_corner, t.fan_ptr, t.fan_steps, t.fan_walk);
     fcw::face_patches(t.fan_ptr, t.fan_steps, t.patches);
+    if (records.valid()) records.get();
 }
 
 // e's device arrays of the mesh
@@ -685,16 +702,10 @@ int build_engine(fcw_engine* e, const double* V, int64_t nv, const int32_t* F, i
     const auto& m = e->mesh;
     if (S.max_ns > fcw::kMaxWidth) return fail(FCW_E_INVALID, "supernode wider than the kernels support");
     if (nf > fcw::kIncFace) return fail(FCW_E_INVALID, "mesh has too many faces");
-    // The mesh tables are formed on a thread of their own while this one plans the sweeps and waits for
-    // the device's factorisations: 122 ms against 100 at 147k vertices, 4.9 against 5.5 at 9k. One after
-    // the other, a build at 147k vertices took 460 ms instead of 375.
+    // The mesh tables are formed on threads of their own while this one plans the sweeps. A build at 147k
+    // vertices (64 columns, one block in flight) took 480 ms with all of it one after the other, 375 now.
     MeshTables tables;
-    std::future<void> tables_done;  // waits for its thread when the build fails
-    try {
-        tables_done = std::async(std::launch::async, [&] { mesh_tables(m, S, tables); });
-    } catch (const std::system_error&) {  // no thread to be had
-        mesh_tables(m, S, tables);
-    }
+    std::future<void> tables_done = on_thread([&] { mesh_tables(m, S, tables); });
     {
         // each connected component grounded at its last eliminated vertex: L is singular once
         // per component
@@ -885,6 +896,11 @@ int build_engine(fcw_engine* e, const double* V, int64_t nv, const int32_t* F, i
         FCW_TRY(e->upload(&e->gm_src_d, gsrc));
     }
 
+    // uploaded before the factors are allocated: where an engine's arrays lie shows in the single-source
+    // sweeps (26k vertices: 110 us a call, 117 with the tables uploaded after the factors)
+    if (tables_done.valid()) tables_done.get();
+    FCW_TRY(upload_mesh(e, tables));
+
     // numeric factorisations
     t0 = now_ms();
     double *upd, *aval_d;
@@ -990,8 +1006,7 @@ int build_engine(fcw_engine* e, const double* V, int64_t nv, const int32_t* F, i
     e->release(upd);
     e->release(aval_d);
     e->factor_ms = now_ms() - t0;
-    if (tables_done.valid()) tables_done.get();
-    return upload_mesh(e, tables);
+    return FCW_OK;
 }
 
 // Statistics records that any block of at most K columns writes.

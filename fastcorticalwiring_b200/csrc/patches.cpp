@@ -1,23 +1,28 @@
 // The divergence's view of the mesh (face.cu): each vertex's faces as fans, and patches of vertices.
 #include "patches.h"
 
+#include <algorithm>
+#include <future>
+#include <system_error>
+#include <thread>
+
 namespace fcw {
+
+namespace {
 
 // Each vertex's incident faces as fans for the mixed divergence (FaceData): walks from face to face
 // over the neighbour they share, first from the neighbours with one face (boundary ends), then around
 // the closed fans. A neighbour with more than two faces at the vertex (a non-manifold edge) ends fans.
-void face_fans(const MeshPrep& m, const std::vector<int32_t>& fv, const std::vector<int32_t>& inc_ptr,
-               const std::vector<int32_t>& inc_face, const std::vector<int8_t>& inc_corner,
-               std::vector<int32_t>& ptr, std::vector<FanStep>& steps, std::vector<int32_t>& walked) {
-    const int64_t n = (int64_t)inc_ptr.size() - 1;
-    ptr.assign(n + 1, 0);
-    steps.clear();
-    steps.reserve(inc_face.size() + n);
-    walked.clear();
-    walked.reserve(2 * (inc_face.size() + n));
+// Vertices [v0, v1): ptr[v + 1] = the steps of the range up to and with v.
+void fans_of(const MeshPrep& m, const std::vector<int32_t>& fv, const std::vector<int32_t>& inc_ptr,
+             const std::vector<int32_t>& inc_face, const std::vector<int8_t>& inc_corner, int64_t v0, int64_t v1,
+             std::vector<int32_t>& ptr, std::vector<FanStep>& steps, std::vector<int32_t>& walked) {
+    const int64_t n = (int64_t)inc_ptr.size() - 1, most = inc_ptr[v1] - inc_ptr[v0] + (v1 - v0);
+    steps.reserve(most);
+    walked.reserve(2 * most);
     std::vector<int32_t> at(n, -1);                   // neighbour -> its slot at the current vertex
     std::vector<int32_t> slot_face, slot_count, slot_of, done;  // two faces per slot; the faces' two slots
-    for (int64_t v = 0; v < n; ++v) {
+    for (int64_t v = v0; v < v1; ++v) {
         const int32_t q0 = inc_ptr[v], deg = inc_ptr[v + 1] - q0;
         slot_face.clear();
         slot_count.clear();
@@ -69,6 +74,53 @@ void face_fans(const MeshPrep& m, const std::vector<int32_t>& fv, const std::vec
         for (int32_t i = 0; i < deg; ++i)
             for (int k = 0; k < 2; ++k) at[other(i, k)] = -1;
         ptr[v + 1] = (int32_t)steps.size();
+    }
+}
+
+}  // namespace
+
+// The vertices in equal ranges, one per thread, joined in order: the same arrays for any number of them.
+// 147k vertices on eight cores: 74 ms with one thread, 35 with eight; 9k vertices 2.8 and 2.0 (three).
+void face_fans(const MeshPrep& m, const std::vector<int32_t>& fv, const std::vector<int32_t>& inc_ptr,
+               const std::vector<int32_t>& inc_face, const std::vector<int8_t>& inc_corner,
+               std::vector<int32_t>& ptr, std::vector<FanStep>& steps, std::vector<int32_t>& walked, int threads) {
+    const int64_t n = (int64_t)inc_ptr.size() - 1;
+    ptr.assign(n + 1, 0);
+    steps.clear();
+    walked.clear();
+    const int most = std::max(1, (int)std::min<int64_t>(8, std::thread::hardware_concurrency()));
+    const int parts = threads > 0 ? threads : (int)std::min<int64_t>(most, n / kFanRange + 1);
+    auto first = [&](int r) { return n * r / parts; };
+    struct Range {
+        std::vector<FanStep> steps;
+        std::vector<int32_t> walked;
+        std::future<void> done;  // waits for its thread when another range fails
+    };
+    std::vector<Range> ranges(parts - 1);
+    auto form = [&](int r, std::vector<FanStep>& st, std::vector<int32_t>& wk) {
+        fans_of(m, fv, inc_ptr, inc_face, inc_corner, first(r), first(r + 1), ptr, st, wk);
+    };
+    for (int r = 1; r < parts; ++r) {
+        Range& g = ranges[r - 1];
+        try {
+            g.done = std::async(std::launch::async, [&form, &g, r] { form(r, g.steps, g.walked); });
+        } catch (const std::system_error&) {  // no thread to be had
+            form(r, g.steps, g.walked);
+        }
+    }
+    form(0, steps, walked);
+    size_t total = steps.size();
+    for (Range& g : ranges) {
+        if (g.done.valid()) g.done.get();
+        total += g.steps.size();
+    }
+    steps.reserve(total);
+    walked.reserve(2 * total);
+    for (int r = 1; r < parts; ++r) {
+        Range& g = ranges[r - 1];
+        for (int64_t v = first(r); v < first(r + 1); ++v) ptr[v + 1] += (int32_t)steps.size();
+        steps.insert(steps.end(), g.steps.begin(), g.steps.end());
+        walked.insert(walked.end(), g.walked.begin(), g.walked.end());
     }
 }
 

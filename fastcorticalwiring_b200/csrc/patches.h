@@ -32,10 +32,13 @@ struct PatchArrays {
 };
 
 // fv: faces (elimination order), inc_*: each vertex's incident faces in ascending face order. walk: per
-// step, its neighbour and the face it closes (-1 in a fan's first step).
+// step, its neighbour and the face it closes (-1 in a fan's first step). threads: 0 takes one per
+// kFanRange vertices, at most 8 and at most the host's.
+constexpr int64_t kFanRange = 4096;
 void face_fans(const MeshPrep& m, const std::vector<int32_t>& fv, const std::vector<int32_t>& inc_ptr,
                const std::vector<int32_t>& inc_face, const std::vector<int8_t>& inc_corner,
-               std::vector<int32_t>& ptr, std::vector<FanStep>& steps, std::vector<int32_t>& walk);
+               std::vector<int32_t>& ptr, std::vector<FanStep>& steps, std::vector<int32_t>& walk,
+               int threads = 0);
 // fv: faces (elimination order). Rewrites the steps' neighbours as patch rows (big vertices keep theirs).
 void face_patches(const std::vector<int32_t>& fan_ptr, std::vector<FanStep>& steps, PatchArrays& pa);
 
