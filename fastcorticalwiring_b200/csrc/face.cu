@@ -24,7 +24,8 @@
 // with a scale of its own. A CTA takes a patch of consecutive vertices in elimination order (mostly
 // part of one dissection leaf, so a compact piece of the surface) and brings its rows and their
 // neighbours' into shared memory once; gathered through L1, rows came back from L2 three to four
-// times. 147k vertices, 1024 columns: 1.73 to 1.33 ms, bound by issue and the conversions' latency.
+// times. 147k vertices, 1024 columns: 1.73 to 1.33 ms; issue 52%, shared memory 49% and the conversion pipe 36%
+// busy: warps wait about equally for fixed latencies, for conversions and shared memory, and for rows.
 // Vertices with too many neighbours for a patch are gathered from memory, a warp each.
 #include "kernels.cuh"
 
