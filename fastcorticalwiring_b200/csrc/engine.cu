@@ -552,6 +552,7 @@ struct MeshTables {
     std::vector<fcw::FanStep> fan_steps;
     std::vector<int4> corners, div_rec;
     std::vector<double> geo;
+    fcw::SharpFans sharp;
     fcw::PatchArrays patches;
 };
 
@@ -629,7 +630,10 @@ void mesh_tables(const fcw::MeshPrep& m, const fcw::Symbolic& S, MeshTables& t) 
     };
     std::future<void> records = on_thread(face_records);
     fcw::face_fans(m, fv, inc_ptr, inc_face, inc_corner, t.fan_ptr, t.fan_steps, t.fan_walk);
+    std::future<void> sharp =
+        on_thread([&] { fcw::sharp_fans(m, fv, t.fan_ptr, t.fan_steps, t.fan_walk, t.sharp); });
     fcw::face_patches(t.fan_ptr, t.fan_steps, t.patches);
+    if (sharp.valid()) sharp.get();
     if (records.valid()) records.get();
 }
 
@@ -685,6 +689,15 @@ int upload_mesh(fcw_engine* e, const MeshTables& t) {
         FCW_TRY(e->upload(&e->clevel.area, e->carea_h));
     }
     FCW_TRY(e->upload(&e->perm_d, S.perm));
+    if (!t.sharp.vertices.empty()) {
+        int32_t *sharp_d, *sharp_ptr_d;
+        fcw::FanStep* sharp_fans_d;
+        FCW_TRY(e->upload(&sharp_d, t.sharp.vertices));
+        FCW_TRY(e->upload(&sharp_ptr_d, t.sharp.ptr));
+        FCW_TRY(e->upload(&sharp_fans_d, t.sharp.steps));
+        e->fd.nsharp = (int32_t)t.sharp.vertices.size();
+        e->fd.sharp = sharp_d; e->fd.sharp_ptr = sharp_ptr_d; e->fd.sharp_fans = sharp_fans_d;
+    }
     return FCW_OK;
 }
 

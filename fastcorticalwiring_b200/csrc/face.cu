@@ -27,6 +27,14 @@
 // times. 147k vertices, 1024 columns: 1.73 to 1.33 ms; issue 52%, shared memory 49% and the conversion pipe 36%
 // busy: warps wait about equally for fixed latencies, for conversions and shared memory, and for rows.
 // Vertices with too many neighbours for a patch are gathered from memory, a warp each.
+//
+// At a sharp corner (under 6 degrees: needle triangles) the two edges are nearly parallel and |g|^2 cancels
+// in FP32, at that corner but not at the face's other two, so the face's three terms no longer cancel in the
+// sum over the mesh. Vertices with such corners are evaluated once more, a warp each: the sharp faces with
+// the difference along the short edge, formed in FP64, in place of the second long one,
+//   a = d1 c_vv + e c_vb,  b = d1 c_vb + e c_bb,  |g|^2 = d1 a + e b,  g . gb_vertex = -a.
+// A fan of 500 needles: fields 7.3e-5 of their maximum off without this. Meshes without such corners (every
+// folded icosphere up to jitter 0.2) launch nothing.
 #include "kernels.cuh"
 
 namespace fcw {
@@ -182,14 +190,15 @@ __device__ __forceinline__ double unit_scale(double x) {
     return __longlong_as_double((2046 - e) << 52);
 }
 // One face's term at its vertex from the FP64 differences, with a scale of its own; c holds the
-// coefficients times the squared area.
+// coefficients times the squared area. SHARP: those of a sharp corner (SharpFans).
+template <bool SHARP>
 __device__ __noinline__ float face_alone(double d1, double d2, float c11, float c12, float c22) {
     const double mx = fmax(fabs(d1), fabs(d2));
     if (!(mx >= 2.2250738585072014e-308)) return 0.0f;  // zero (or subnormal) gradient
     const double sc = unit_scale(mx);
     const float x1 = (float)(d1 * sc), x2 = (float)(d2 * sc);
     const float a = x1 * c11 + x2 * c12, b = x1 * c12 + x2 * c22, q = x1 * a + x2 * b;
-    return q > 0.0f ? (a + b) * rsqrtf(q) : 0.0f;
+    return q > 0.0f ? (SHARP ? a : a + b) * rsqrtf(q) : 0.0f;
 }
 
 // Pairs of FP32 values in one register pair (packed FMA pipe).
@@ -259,9 +268,9 @@ __device__ __forceinline__ f32x2 fan_sum(double2 uv, int e0, int e1, Steps&& fan
                 float2 r = unpack2(acc);
                 const float2 n2 = unpack2(ab);
                 r.x = in0 ? fmaf(n2.x, rsqrt_approx(q.x), r.x)
-                          : r.x + face_alone(up.x - uv.x, un.x - uv.x, c.c11[0], c.c12[0], c.c22[0]);
+                          : r.x + face_alone<false>(up.x - uv.x, un.x - uv.x, c.c11[0], c.c12[0], c.c22[0]);
                 r.y = in1 ? fmaf(n2.y, rsqrt_approx(q.y), r.y)
-                          : r.y + face_alone(up.y - uv.y, un.y - uv.y, c.c11[0], c.c12[0], c.c22[0]);
+                          : r.y + face_alone<false>(up.y - uv.y, un.y - uv.y, c.c11[0], c.c12[0], c.c22[0]);
                 acc = pack2(r.x, r.y);
             }
             xp = x;
@@ -322,6 +331,32 @@ __global__ void __launch_bounds__(256) k_div_mixed_big(FaceData fd, const double
     *reinterpret_cast<float2*>(div + (int64_t)v * K + (int64_t)blockIdx.y * kColsMixed + 2 * lane) = unpack2(acc);
 }
 
+__global__ void __launch_bounds__(256) k_div_mixed_sharp(FaceData fd, const double* __restrict__ u,
+                                                         float* __restrict__ div, int32_t K,
+                                                         const uint8_t* __restrict__ grounded) {
+    const int lane = threadIdx.x & 31, i = blockIdx.x * 8 + (threadIdx.x >> 5);
+    if (i >= fd.nsharp || grounded[fd.sharp[i]]) return;
+    const int v = fd.sharp[i];
+    const int64_t c0 = (int64_t)blockIdx.y * kColsMixed + 2 * lane;
+    auto row = [&](int w) { return *reinterpret_cast<const double2*>(u + (int64_t)w * K + c0); };
+    const double2 uv = row(v);
+    double2 up = uv;
+    float2 acc = make_float2(0.0f, 0.0f);
+    for (int e = fd.sharp_ptr[i]; e < fd.sharp_ptr[i + 1]; ++e) {
+        const FanStep c = fd.sharp_fans[e];
+        const double2 un = row(c.neighbour);
+        if (c.faces == -2) {
+            acc.x += face_alone<true>(up.x - uv.x, un.x - up.x, c.c11[0], c.c12[0], c.c22[0]);
+            acc.y += face_alone<true>(up.y - uv.y, un.y - up.y, c.c11[0], c.c12[0], c.c22[0]);
+        } else if (c.faces < 0) {
+            acc.x += face_alone<false>(up.x - uv.x, un.x - uv.x, c.c11[0], c.c12[0], c.c22[0]);
+            acc.y += face_alone<false>(up.y - uv.y, un.y - uv.y, c.c11[0], c.c12[0], c.c22[0]);
+        }
+        up = un;
+    }
+    *reinterpret_cast<float2*>(div + (int64_t)v * K + c0) = acc;
+}
+
 constexpr size_t kSmemMixed = (size_t)kPatchRows * kColsMixed * 8 + (size_t)kPatchSteps * sizeof(FanStep);
 
 }  // namespace
@@ -355,6 +390,8 @@ void launch_divergence_mixed(const FaceData& fd, const double* u, float* div, in
         k_div_mixed<<<dim3(fd.npatches, K / kColsMixed), 256, kSmemMixed, st>>>(fd, u, div, K, grounded);
     if (fd.nbig > 0)
         k_div_mixed_big<<<dim3((fd.nbig + 7) / 8, K / kColsMixed), 256, 0, st>>>(fd, u, div, K, grounded);
+    if (fd.nsharp > 0)
+        k_div_mixed_sharp<<<dim3((fd.nsharp + 7) / 8, K / kColsMixed), 256, 0, st>>>(fd, u, div, K, grounded);
 }
 
 }  // namespace fcw

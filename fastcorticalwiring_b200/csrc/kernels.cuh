@@ -279,6 +279,11 @@ struct FaceData {
     const int32_t* patch_rows = nullptr;  // the vertices of a patch's rows, its own first
     const int32_t* fan_ptr = nullptr;     // nv+1
     const FanStep* fans = nullptr;
+    // mixed form: the vertices with sharp corners (SharpFans, patches.h), evaluated once more
+    int32_t nsharp = 0;
+    const int32_t* sharp = nullptr;
+    const int32_t* sharp_ptr = nullptr;   // nsharp + 1
+    const FanStep* sharp_fans = nullptr;
 };
 cudaError_t configure_divergence_kernels();
 // scale: nf * K doubles of scratch

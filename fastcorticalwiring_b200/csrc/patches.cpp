@@ -124,6 +124,41 @@ void face_fans(const MeshPrep& m, const std::vector<int32_t>& fv, const std::vec
     }
 }
 
+void sharp_fans(const MeshPrep& m, const std::vector<int32_t>& fv, const std::vector<int32_t>& fan_ptr,
+                const std::vector<FanStep>& steps, const std::vector<int32_t>& walk, SharpFans& sf) {
+    const int32_t n = (int32_t)fan_ptr.size() - 1;
+    auto sharp = [](const FanStep& s) {  // an acute corner; a fan's first step has no coefficients
+        const double a = s.c11[0], b = s.c12[0], c = s.c22[0];
+        return b < 0.0 && a * c - b * b < kSharp * a * c;
+    };
+    sf.ptr.assign(1, 0);
+    for (int32_t v = 0; v < n; ++v) {
+        bool any = false;
+        for (int32_t e = fan_ptr[v]; e < fan_ptr[v + 1] && !any; ++e) any = sharp(steps[e]);
+        if (!any) continue;
+        sf.vertices.push_back(v);
+        for (int32_t e = fan_ptr[v]; e < fan_ptr[v + 1]; ++e) {
+            const FanStep& x = steps[e];
+            FanStep s{{x.c11[0], x.c11[1]}, {x.c12[0], x.c12[1]}, {x.c22[0], x.c22[1]}, walk[2 * (int64_t)e], x.faces};
+            if (sharp(x)) {
+                const int64_t f = walk[2 * (int64_t)e + 1];
+                auto gradient = [&](int32_t w) {
+                    int c = 0;
+                    while (c < 2 && fv[3 * f + c] != w) ++c;
+                    return &m.gb[9 * f + 3 * c];
+                };
+                const double *gv = gradient(v), *gn = gradient(s.neighbour), aa = m.grad_area[f] * m.grad_area[f];
+                auto dot = [](const double* x, const double* y) { return x[0] * y[0] + x[1] * y[1] + x[2] * y[2]; };
+                s.c11[0] = s.c11[1] = (float)(aa * dot(gv, gv));
+                s.c12[0] = s.c12[1] = (float)(-aa * dot(gv, gn));
+                s.faces = -2;
+            }
+            sf.steps.push_back(s);
+        }
+        sf.ptr.push_back((int32_t)sf.steps.size());
+    }
+}
+
 // Consecutive vertices join a patch while its rows and fan steps fit. A vertex's rows are itself and
 // the neighbours its steps name.
 void face_patches(const std::vector<int32_t>& fan_ptr, std::vector<FanStep>& steps, PatchArrays& pa) {

@@ -22,7 +22,7 @@ struct Patch {
 // each, as packed operands.
 struct FanStep {
     float c11[2], c12[2], c22[2];
-    int32_t neighbour, faces;  // faces: of the fan, in its first step; -1 in the others
+    int32_t neighbour, faces;  // faces: of the fan, in its first step; negative in the others
 };
 
 struct PatchArrays {
@@ -39,6 +39,18 @@ void face_fans(const MeshPrep& m, const std::vector<int32_t>& fv, const std::vec
                const std::vector<int32_t>& inc_face, const std::vector<int8_t>& inc_corner,
                std::vector<int32_t>& ptr, std::vector<FanStep>& steps, std::vector<int32_t>& walk,
                int threads = 0);
+// The vertices with a sharp corner (sine squared below kSharp): their fans with the neighbours as vertices,
+// and for the sharp faces (faces = -2) other coefficients: gb_v . gb_v, -gb_v . gb_b, gb_b . gb_b times the
+// squared area, gb_v the gradient of the vertex itself, for the differences along the step before's edge
+// and from its neighbour to this one's.
+constexpr double kSharp = 0.01;
+struct SharpFans {
+    std::vector<int32_t> vertices, ptr;  // ptr: their steps
+    std::vector<FanStep> steps;
+};
+// walk, steps: of face_fans. Does not read the steps' neighbours, which face_patches rewrites.
+void sharp_fans(const MeshPrep& m, const std::vector<int32_t>& fv, const std::vector<int32_t>& fan_ptr,
+                const std::vector<FanStep>& steps, const std::vector<int32_t>& walk, SharpFans& sf);
 // fv: faces (elimination order). Rewrites the steps' neighbours as patch rows (big vertices keep theirs).
 void face_patches(const std::vector<int32_t>& fan_ptr, std::vector<FanStep>& steps, PatchArrays& pa);
 

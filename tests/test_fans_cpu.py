@@ -1,6 +1,6 @@
 """The fans are the same arrays for any number of threads (no GPU): fans_check.cpp forms them in one
 range of vertices, in the number the engine would take, and in 2 to 64, also more than the mesh has
-vertices."""
+vertices. And the fans of vertices with sharp corners: which they are, and their coefficients."""
 import os
 import subprocess
 
@@ -29,14 +29,17 @@ def _icosphere(level):
     return pm.V, pm.F
 
 
-@pytest.mark.parametrize("mesh", [
-    lambda: _icosphere(6),  # 36,866 vertices: eight ranges by the engine's own rule
-    lambda: _icosphere(4), lambda: book(5), lambda: hub(300),
-    lambda: (np.array([[0.0, 0, 0], [1, 0, 0], [0, 1, 0]]), np.array([[0, 1, 2]], np.int32)),
-], ids=["L6", "L4", "book", "hub", "triangle"])
-def test_fans_do_not_depend_on_the_threads(checker, tmp_path, mesh):
+@pytest.mark.parametrize("mesh,sharp", [
+    (lambda: _icosphere(6), 0),  # 36,866 vertices: eight ranges by the engine's own rule
+    (lambda: _icosphere(4), 0), (lambda: book(5), 0),
+    (lambda: hub(60), 0), (lambda: hub(64), 1),    # the hub, from 5.7 degrees on
+    (lambda: hub(500), 1001),                      # there the rings' triangles are needles too
+    (lambda: (np.array([[0.0, 0, 0], [1, 0, 0], [0, 1, 0]]), np.array([[0, 1, 2]], np.int32)), 0),
+], ids=["L6", "L4", "book", "hub60", "hub64", "hub500", "triangle"])
+def test_fans_do_not_depend_on_the_threads(checker, tmp_path, mesh, sharp):
     V, F = mesh()
     path = str(tmp_path / "mesh.bin")
     _write(path, V, F)
     out = subprocess.check_output([checker, path], text=True).split()
     assert out[0] == "ok" and int(out[1]) > 3 * len(F)
+    assert int(out[2]) == sharp
